@@ -582,6 +582,7 @@ struct Batch {
     cudaStream_t st = nullptr;
     cudaStream_t side = nullptr;       // concurrent branch (small-island PGS)
     cudaEvent_t fork = nullptr, join = nullptr;
+    int max_world = 0;                 // bodies of the largest world
     int dv_cap = 64;                   // island bodies whose Δv fits in shared memory
     int pgs_blocks = 0;                // k_pgs_big grid: one resident chain per block
     int isl_smem = 0;                  // k_islands dynamic shared memory
@@ -645,7 +646,7 @@ struct Batch {
             launch_springs(x, L);                          // impulses before the rows read the velocities
             launch_rows(x, s == 0, s == substeps - 1, L);
             launch_joint_rows(x, s == 0, L);               mark(6 + 3 * s);
-            launch_pgs(x, dv_cap, pgs_blocks, side, fork, join, L);
+            launch_pgs(x, dv_cap, max_world, pgs_blocks, side, fork, join, L);
             launch_pgs_joint(x, s == 0, L);                mark(7 + 3 * s);
             launch_integrate(x, s == substeps - 1, L);     mark(8 + 3 * s);
         }
@@ -658,7 +659,8 @@ struct Batch {
     // (+2 per substep and 1 factorisation with joints)
     int launches_per_step() const {
         return 1 + 6 + 2 + (prims ? 1 : 0) + ((meshes || unions) ? 1 : 0) + (6 + 9) + (2 + 3) + 3 + 5 * substeps + 1 + (joints ? 2 * substeps : 0) +
-               (systems ? 1 : 0) + (audit ? 1 : 0) + (springs ? substeps : 0) + (tiles ? 3 : 0);
+               (systems ? 1 : 0) + (audit ? 1 : 0) + (springs ? substeps : 0) + (tiles ? 3 : 0) +
+               (max_world > dv_cap ? substeps : 0);
     }
 
     // solver schedule: chain workers per SM of k_pgs_big (0 = as many as fit)
@@ -1004,7 +1006,7 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
     }
     B->tiles = !tile_task.empty();
     {
-        int max_world = 0;
+        int& max_world = B->max_world;
         for (size_t k = 0; k + 1 < wstart.size(); k++) max_world = std::max(max_world, wstart[k + 1] - wstart[k]);
         // islands of more bodies keep their Δv in global memory (the same
         // arithmetic); CPGPU_PGS_DV_CAP lowers the cap, so that a batch of a

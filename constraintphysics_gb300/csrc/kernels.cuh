@@ -55,7 +55,9 @@ void launch_pgs_schedule(const Dev& d, const Launch& L);
 void prepare_pgs(int dv_cap);
 int pgs_big_smem_bytes(int dv_cap);
 int pgs_big_blocks_per_sm(int dv_cap);
-void launch_pgs(const Dev& d, int dv_cap, int big_blocks, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, const Launch& L);
+// `max_world`: bodies of the batch's largest world
+void launch_pgs(const Dev& d, int dv_cap, int max_world, int big_blocks, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join,
+                const Launch& L);
 void launch_integrate(const Dev& d, int last, const Launch& L);
 // joints: rows every substep, the holonomic systems' factorisation on the
 // first; islands with joint rows solved by their own kernel

@@ -152,11 +152,16 @@ struct EdgeStore {
 
 // Solver row block of one contact (normal row + 2-dof friction row), built each
 // substep in island order (ConstraintSolver.cpp:240-343).  384 bytes, 16-byte
-// aligned.  After a 96-byte header come twelve 6-vectors (linear xyz, angular
-// xyz), 24 bytes apart from byte 96, so that every (x, y), (z, ax), (ay, az)
-// component pair sits in one half of a 16-byte word: the solver loads the
-// row with 16-byte loads and computes on the pairs with packed FP32
-// instructions (fma.rn.f32x2).
+// aligned: a 96-byte header, then per body of the contact one RowSide of six
+// 6-vectors (linear xyz, angular xyz), 24 bytes apart, so that every (x, y),
+// (z, ax), (ay, az) component pair sits in one half of a 16-byte word: a
+// solver lane that owns one of the two bodies reads its 144 bytes with nine
+// 16-byte loads and computes on the pairs with packed FP32 instructions
+// (fma.rn.f32x2).
+struct RowSide {
+    float nj[6], fj0[6], fj1[6];      // J of the normal row and of the friction rows (u, w)
+    float nit[6], fit0[6], fit1[6];   // M^-1 J^T of the same
+};
 struct alignas(16) RowBlock {
     float4 imp;          // accumulated impulses: normal, pseudo normal, friction u, w
     int sa, sb;          // island body slots (-1 = body with infinite mass)
@@ -169,12 +174,11 @@ struct alignas(16) RowBlock {
     float nminv, nptarget;
     float kd0, kd1;      // friction impulse change per unit normal impulse: Fm^-1 (J_f M^-1 J_n^T)
     float fmc[4];        // the friction rows' 2x2 effective-mass inverse Fm^-1 by columns: (m00, m10), (m01, m11)
-    float nja[6], njb[6], nita[6], nitb[6];          // normal row J and M^-1 J^T (bodies a, b)
-    float fja0[6], fjb0[6], fja1[6], fjb1[6];        // friction rows (u, w)
-    float fita0[6], fitb0[6], fita1[6], fitb1[6];    // friction M^-1 J^T columns (u, w)
+    RowSide a, b;
 };
+static_assert(sizeof(RowSide) == 144, "row side size");
 static_assert(sizeof(RowBlock) == 384, "row block size");
-static_assert(offsetof(RowBlock, nja) == 96, "row vectors start at byte 96");
+static_assert(offsetof(RowBlock, tgt_n) == 48 && offsetof(RowBlock, a) == 96, "row sides start at byte 96");
 
 // Velocity deltas of an island body (the solver's accumulator): 12 floats in
 // kDvF4 float4s, v xyz, w xyz, pv xyz, pw xyz (pseudo velocities for the

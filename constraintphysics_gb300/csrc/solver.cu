@@ -105,7 +105,7 @@ __global__ void k_rows(Dev d, int first, int last) {
             it_of(ima, Ia, ja, ia);
             it_of(imb, Ib, jb, ib);
             float itv = dot6(ja, ia) + dot6(jb, ib);
-            for (int k = 0; k < 6; k++) { R.nja[k] = ja[k]; R.njb[k] = jb[k]; R.nita[k] = ia[k]; R.nitb[k] = ib[k]; }
+            for (int k = 0; k < 6; k++) { R.a.nj[k] = ja[k]; R.b.nj[k] = jb[k]; R.a.nit[k] = ia[k]; R.b.nit[k] = ib[k]; }
             R.nminv = 1.0f / (itv * (1.0f + P.cfm));
             R.nptarget = fmaxf(0.0f, depth - 0.05f) * pcc;
             // friction rows in the tangent basis of n, warm impulse re-projected
@@ -145,8 +145,8 @@ __global__ void k_rows(Dev d, int first, int last) {
             R.kd0 = m00 * kf0 + m01 * kf1;
             R.kd1 = m10 * kf0 + m11 * kf1;
             for (int k = 0; k < 6; k++) {
-                R.fja0[k] = fja[k]; R.fjb0[k] = fjb[k]; R.fja1[k] = fja[6 + k]; R.fjb1[k] = fjb[6 + k];
-                R.fita0[k] = fia[2 * k]; R.fitb0[k] = fib[2 * k]; R.fita1[k] = fia[2 * k + 1]; R.fitb1[k] = fib[2 * k + 1];
+                R.a.fj0[k] = fja[k]; R.b.fj0[k] = fjb[k]; R.a.fj1[k] = fja[6 + k]; R.b.fj1[k] = fjb[6 + k];
+                R.a.fit0[k] = fia[2 * k]; R.b.fit0[k] = fib[2 * k]; R.a.fit1[k] = fia[2 * k + 1]; R.b.fit1[k] = fib[2 * k + 1];
             }
             // velocity targets from the bodies' velocities at the start of the
             // solve (ContactConstraint::findTargetConstraintValue,
@@ -221,8 +221,7 @@ __device__ __forceinline__ void paxpy(P3& v, const P3& x, float2 s) {
 
 // Δv of island body `slot`: which 0 = (v, w), 1 = (pv, pw); slot < 0 is a
 // body of infinite mass (always zero)
-__device__ __forceinline__ P3 dv_get(const float4* dv, int slot, int which) {
-    if (slot < 0) return P3{make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+__device__ __forceinline__ P3 dv_get_z(const float4* dv, int slot, int which) {   // dv has an entry at -1
     const float4* s = dv + kDvF4 * slot;
     if (which == 0) {
         const float4 A = s[0];
@@ -233,8 +232,11 @@ __device__ __forceinline__ P3 dv_get(const float4* dv, int slot, int which) {
     const float4 C = s[2];
     return P3{A, make_float2(C.x, C.y), make_float2(C.z, C.w)};
 }
-__device__ __forceinline__ void dv_put(float4* dv, int slot, int which, const P3& v) {
-    if (slot < 0) return;
+__device__ __forceinline__ P3 dv_get(const float4* dv, int slot, int which) {
+    if (slot < 0) return P3{make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    return dv_get_z(dv, slot, which);
+}
+__device__ __forceinline__ void dv_put_z(float4* dv, int slot, int which, const P3& v) {
     float4* s = dv + kDvF4 * slot;
     if (which == 0) {
         s[0] = make_float4(v.a.x, v.a.y, v.b.x, v.b.y);
@@ -245,6 +247,10 @@ __device__ __forceinline__ void dv_put(float4* dv, int slot, int which, const P3
     }
 }
 
+__device__ __forceinline__ void dv_put(float4* dv, int slot, int which, const P3& v) {
+    if (slot >= 0) dv_put_z(dv, slot, which, v);
+}
+
 // ---- one row of each PGS pass (PGS_solve, ConstraintSolver.cpp:120-161) ----------
 // warm start: apply the stored impulses when they are non-zero
 // (DegreedConstraint::constraintWarmStarted / applyWarmStartVelocityChange)
@@ -253,14 +259,14 @@ __device__ __forceinline__ void row_warm(const RowBlock& R, const float4 imp, fl
     if (!wn && !wf) return;
     P3 va = dv_get(dv, R.sa, 0), vb = dv_get(dv, R.sb, 0);
     if (wn) {
-        paxpy(va, p3(R.nita), bc2(imp.x));
-        paxpy(vb, p3(R.nitb), bc2(imp.x));
+        paxpy(va, p3(R.a.nit), bc2(imp.x));
+        paxpy(vb, p3(R.b.nit), bc2(imp.x));
     }
     if (wf) {
-        paxpy(va, p3(R.fita0), bc2(imp.z));
-        paxpy(va, p3(R.fita1), bc2(imp.w));
-        paxpy(vb, p3(R.fitb0), bc2(imp.z));
-        paxpy(vb, p3(R.fitb1), bc2(imp.w));
+        paxpy(va, p3(R.a.fit0), bc2(imp.z));
+        paxpy(va, p3(R.a.fit1), bc2(imp.w));
+        paxpy(vb, p3(R.b.fit0), bc2(imp.z));
+        paxpy(vb, p3(R.b.fit1), bc2(imp.w));
     }
     dv_put(dv, R.sa, 0, va);
     dv_put(dv, R.sb, 0, vb);
@@ -278,8 +284,8 @@ __device__ __forceinline__ void row_warm(const RowBlock& R, const float4 imp, fl
 // friction rows are evaluated.  The disc projection compares squared
 // magnitudes and scales by rsqrt.  `va`, `vb` are the two bodies' Δv.
 __device__ __forceinline__ void row_vel_r(const RowBlock& R, float4& imp, int& stat, P3& va, P3& vb) {
-    const float cur = pdot(p3(R.nja), va, p3(R.njb), vb);
-    const float b0 = pdot(p3(R.fja0), va, p3(R.fjb0), vb), b1 = pdot(p3(R.fja1), va, p3(R.fjb1), vb);
+    const float cur = pdot(p3(R.a.nj), va, p3(R.b.nj), vb);
+    const float b0 = pdot(p3(R.a.fj0), va, p3(R.b.fj0), vb), b1 = pdot(p3(R.a.fj1), va, p3(R.b.fj1), vb);
     // friction impulses for the incoming velocities: imp.zw + Fm^-1 (tgt_f - b)
     const float2 g = psub(make_float2(R.tgt_f0, R.tgt_f1), make_float2(b0, b1));
     const float2 A = __fadd2_rn(make_float2(imp.z, imp.w),
@@ -290,8 +296,8 @@ __device__ __forceinline__ void row_vel_r(const RowBlock& R, float4& imp, int& s
     if (!(fabsf(diff) > kZero)) diff = 0.f;
     const float ix = __fadd_rn(imp.x, diff);
     const float2 sd = bc2(diff);
-    paxpy(va, p3(R.nita), sd);
-    paxpy(vb, p3(R.nitb), sd);
+    paxpy(va, p3(R.a.nit), sd);
+    paxpy(vb, p3(R.b.nit), sd);
     float2 nf = __ffma2_rn(bc2(-diff), make_float2(R.kd0, R.kd1), A);
     const float mx = __fmul_rn(R.fcoeff, ix);
     const float s2 = __fmaf_rn(nf.x, nf.x, __fmul_rn(nf.y, nf.y));
@@ -300,10 +306,10 @@ __device__ __forceinline__ void row_vel_r(const RowBlock& R, float4& imp, int& s
     float2 e = psub(nf, make_float2(imp.z, imp.w));
     if (!(fabsf(e.x) > kZero || fabsf(e.y) > kZero)) e = make_float2(0.f, 0.f);
     const float2 s0 = bc2(e.x), s1 = bc2(e.y);
-    paxpy(va, p3(R.fita0), s0);
-    paxpy(vb, p3(R.fitb0), s0);
-    paxpy(va, p3(R.fita1), s1);
-    paxpy(vb, p3(R.fitb1), s1);
+    paxpy(va, p3(R.a.fit0), s0);
+    paxpy(vb, p3(R.b.fit0), s0);
+    paxpy(va, p3(R.a.fit1), s1);
+    paxpy(vb, p3(R.b.fit1), s1);
     imp.x = ix;
     imp.z = __fadd_rn(imp.z, e.x);
     imp.w = __fadd_rn(imp.w, e.y);
@@ -320,12 +326,12 @@ __device__ __forceinline__ void row_vel(const RowBlock& R, float4& imp, int& sta
 // pseudo-velocity (position correction) pass of the normal row
 __device__ __forceinline__ void row_pos(const RowBlock& R, float4& imp, float4* dv) {
     P3 va = dv_get(dv, R.sa, 1), vb = dv_get(dv, R.sb, 1);
-    const float cur = pdot(p3(R.nja), va, p3(R.njb), vb);
+    const float cur = pdot(p3(R.a.nj), va, p3(R.b.nj), vb);
     const float nw = __fmaf_rn(R.nminv, __fsub_rn(R.nptarget, cur), imp.y);
     const float diff = __fsub_rn(fmaxf(nw, 0.0f), imp.y);
     if (fabsf(diff) > kZero) {
-        paxpy(va, p3(R.nita), bc2(diff));
-        paxpy(vb, p3(R.nitb), bc2(diff));
+        paxpy(va, p3(R.a.nit), bc2(diff));
+        paxpy(vb, p3(R.b.nit), bc2(diff));
         imp.y = __fadd_rn(imp.y, diff);
         dv_put(dv, R.sa, 1, va);
         dv_put(dv, R.sb, 1, vb);
@@ -454,8 +460,10 @@ __global__ void k_pgs_small(Dev d) {
 }
 
 // ---- large islands: one warp per island, rows streamed through shared memory
-constexpr int kRingSlots = 6;
-constexpr int kChunkRows = 16;
+// 36 KB of rows per chain; chunks of 32 rows measured 279 cycles per row-step on
+// a 2,000-row chain, of 16 rows 297 (the work at a chunk's edge)
+constexpr int kRingSlots = 3;
+constexpr int kChunkRows = 32;
 
 __device__ __forceinline__ uint32_t saddr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
@@ -482,166 +490,410 @@ __device__ __forceinline__ bool ring_wait(uint64_t* bar, uint32_t parity, long l
     return false;
 }
 
-// The serial Gauss-Seidel chain of one island on one thread: 1 warm-start pass,
-// pgs_vel velocity passes and pgs_pos position passes over the island's rows,
-// in order.  The first position pass is fused into the warm-start pass: the
-// position rows read and write only the pseudo velocities and the pseudo
-// impulse, which no other pass touches and which start at zero, so running
-// position row j right after warm-start row j gives the same result as a
-// separate pass, one pass sooner (the two rows' arithmetic interleaves).  Rows stream through the shared ring (look-ahead up to one pass,
-// since a pass must see the impulses the previous pass wrote back); each row
-// is copied to registers with 16-byte loads before it is used.
-__device__ __forceinline__ bool big_chain(const Dev& d, RowBlock* ring, uint64_t* bars, uint32_t& phase, float4* dv, int rs,
-                                       int rc, const WorldParams& P) {
-    const int nch = (rc + kChunkRows - 1) / kChunkRows;
-    const int n_vel = P.pgs_vel;   // read once: the row stores below could alias P for the compiler
-    const int n_pos = P.pgs_pos;
-    const bool fused = n_pos > 0;
-    const int passes = 1 + n_vel + (fused ? n_pos - 1 : 0);
-    const int total = passes * nch;
-    const int ahead = nch < kRingSlots ? nch : kRingSlots;
-    // A proxy fence covers every impulse write issued before it.  Chunk c of
-    // sequence t was last written at sequence t - nch (every pass writes when
-    // the position rows are fused into the warm-start pass, the others from
-    // the first velocity pass on); a fence is needed only if none was issued
-    // since: about once per pass on a large island, every chunk on a small one.
-    int fenced = -1;
-    // body pair whose Δv the velocity passes hold in registers (-1: none)
-    int cur_a = -1, cur_b = -1;
-    P3 ca{}, cb{};
-    auto issue = [&](int t, int now) {
-        int c = t % nch, slot = t % kRingSlots;
-        int n = min(kChunkRows, rc - c * kChunkRows);
-        const int tw = t - nch;
-        const bool fence = tw >= (fused ? 0 : nch) && tw > fenced;
+// ---- the chain of one island on two lanes -------------------------------------
+// Gauss-Seidel is serial, so a large island costs its row-steps one after the
+// other.  On one lane a row-step issues ~150 instructions (~460 cycles; its
+// dependency chain is ~130), so two lanes share it, one body of the contact
+// each: a lane reads its body's half of the row (144 of 288 bytes), forms its
+// three partial dot products, meets the other lane's by shuffle (the sum is
+// the same either way round, so both get the bits of the one-lane row),
+// evaluates the row's scalars alongside and updates its own body's Δv.  That
+// halves the loads, dot products and updates, and leaves the registers to
+// load the next row while the current one is solved.  A lane keeps its body
+// while consecutive rows share it, whichever side of the row it is on; the Δv
+// of a body that changes is read one row ahead.  A row's code has no branch (a
+// branch costs a lone warp ~40 cycles), and the whole warp runs it, even lanes
+// as lane 0 and odd lanes as lane 1 (same addresses, same values): two lanes
+// inside a branch would check for divergence at every shuffle (404 cycles per
+// row-step against 307).  Measured on a chain of 2,000 rows: 459 -> 274 cycles
+// per row-step; of 90 rows (held in shared memory): 523 -> 265.
+
+struct HalfRow {
+    float2 j[9];     // J of the normal and friction rows (u, w) for the lane's body, three component pairs each
+    float2 m[9];     // M^-1 J^T of the same
+    float4 imp;      // impulses: normal, pseudo normal, friction u, w
+    float4 tgt;      // targets n, u, w; friction coefficient
+    float4 nrm;      // nminv, nptarget, kd0, kd1
+    float4 fm;       // Fm^-1 by columns
+};
+__device__ __forceinline__ void half_load(const RowBlock* R, int side, HalfRow& h) {
+    const float4* q = reinterpret_cast<const float4*>(R);
+    h.imp = q[0];
+    h.tgt = q[3];
+    h.nrm = q[4];
+    h.fm = q[5];
+    const float4* s = q + 6 + 9 * side;
+    float2 f[18];
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        const float4 x = s[k];
+        f[2 * k] = make_float2(x.x, x.y);
+        f[2 * k + 1] = make_float2(x.z, x.w);
+    }
+#pragma unroll
+    for (int k = 0; k < 9; k++) { h.j[k] = f[k]; h.m[k] = f[9 + k]; }
+}
+// one body's part of pdot
+__device__ __forceinline__ float2 half_dot(const float2* j, const P3& v) {
+    float2 s = __fmul2_rn(j[0], v.a);
+    s = __ffma2_rn(j[1], v.b, s);
+    return __ffma2_rn(j[2], v.c, s);
+}
+// ... and its sum with the other lane's part
+__device__ __forceinline__ float2 half_other(float2 s) {
+    return make_float2(__shfl_xor_sync(0xffffffffu, s.x, 1), __shfl_xor_sync(0xffffffffu, s.y, 1));
+}
+__device__ __forceinline__ float half_sum(float2 s, float2 o) {
+    const float2 u = __fadd2_rn(s, o);
+    return __fadd_rn(u.x, u.y);
+}
+__device__ __forceinline__ void half_axpy(P3& v, const float2* m, float s) {
+    const float2 b = bc2(s);
+    v.a = __ffma2_rn(m[0], b, v.a);
+    v.b = __ffma2_rn(m[1], b, v.b);
+    v.c = __ffma2_rn(m[2], b, v.c);
+}
+__device__ __forceinline__ P3 psel(bool first, const P3& x, const P3& y) {
+    return P3{make_float2(first ? x.a.x : y.a.x, first ? x.a.y : y.a.y),
+              make_float2(first ? x.b.x : y.b.x, first ? x.b.y : y.b.y),
+              make_float2(first ? x.c.x : y.c.x, first ? x.c.y : y.c.y)};
+}
+template <bool SH>
+__device__ __forceinline__ P3 dv_load(const float4* dv, int slot, int which) {
+    return SH ? dv_get_z(dv, slot, which) : dv_get(dv, slot, which);
+}
+template <bool SH>
+__device__ __forceinline__ void dv_store(float4* dv, int slot, int which, const P3& v) {
+    if (SH) dv_put_z(dv, slot, which, v);
+    else dv_put(dv, slot, which, v);
+}
+// the same by scalar FMAs: no broadcast of s into a register pair, which the
+// chain would wait for
+__device__ __forceinline__ void half_axpy1(P3& v, const float2* m, float s) {
+    v.a = make_float2(__fmaf_rn(m[0].x, s, v.a.x), __fmaf_rn(m[0].y, s, v.a.y));
+    v.b = make_float2(__fmaf_rn(m[1].x, s, v.b.x), __fmaf_rn(m[1].y, s, v.b.y));
+    v.c = make_float2(__fmaf_rn(m[2].x, s, v.c.x), __fmaf_rn(m[2].y, s, v.c.y));
+}
+// row_warm for the lane's body
+__device__ __forceinline__ void half_warm(const HalfRow& h, P3& v) {
+    if (fabsf(h.imp.x) > kZero) half_axpy(v, h.m, h.imp.x);
+    if (fabsf(h.imp.z) > kZero || fabsf(h.imp.w) > kZero) {
+        half_axpy(v, h.m + 3, h.imp.z);
+        half_axpy(v, h.m + 6, h.imp.w);
+    }
+}
+// row_pos for the lane's body (pseudo velocities p)
+__device__ __forceinline__ void half_pos(HalfRow& h, P3& p) {
+    const float2 s = half_dot(h.j, p);
+    const float cur = half_sum(s, half_other(s));
+    const float nw = __fmaf_rn(h.nrm.x, __fsub_rn(h.nrm.y, cur), h.imp.y);
+    const float diff = __fsub_rn(fmaxf(nw, 0.0f), h.imp.y);
+    if (fabsf(diff) > kZero) {
+        half_axpy(p, h.m, diff);
+        h.imp.y = __fadd_rn(h.imp.y, diff);
+    }
+}
+// row_vel_r for the lane's body
+__device__ __forceinline__ void half_vel(HalfRow& h, P3& v, int& stat) {
+    const float2 sn = half_dot(h.j, v), s0 = half_dot(h.j + 3, v), s1 = half_dot(h.j + 6, v);
+    const float2 on = half_other(sn), o0 = half_other(s0), o1 = half_other(s1);
+    const float cur = half_sum(sn, on), b0 = half_sum(s0, o0), b1 = half_sum(s1, o1);
+    const float nw = __fmaf_rn(h.nrm.x, __fsub_rn(h.tgt.x, cur), h.imp.x);
+    const float2 g = psub(make_float2(h.tgt.y, h.tgt.z), make_float2(b0, b1));
+    const float2 A = __fadd2_rn(make_float2(h.imp.z, h.imp.w),
+                                __ffma2_rn(make_float2(h.fm.z, h.fm.w), bc2(g.y),
+                                           __fmul2_rn(make_float2(h.fm.x, h.fm.y), bc2(g.x))));
+    float diff = __fsub_rn(fmaxf(nw, 0.0f), h.imp.x);
+    if (!(fabsf(diff) > kZero)) diff = 0.f;
+    const float ix = __fadd_rn(h.imp.x, diff);
+    half_axpy(v, h.m, diff);
+    float2 nf = __ffma2_rn(bc2(-diff), make_float2(h.nrm.z, h.nrm.w), A);
+    const float mx = __fmul_rn(h.tgt.w, ix);
+    const float s2 = __fmaf_rn(nf.x, nf.x, __fmul_rn(nf.y, nf.y));
+    // selected, not branched over: a branch costs a single warp more than the
+    // rsqrt it would save
+    const bool slide = s2 > __fmul_rn(mx, mx);
+    const float2 cl = __fmul2_rn(nf, bc2(__fmul_rn(mx, rsqrtf(s2))));
+    nf = make_float2(slide ? cl.x : nf.x, slide ? cl.y : nf.y);
+    stat = slide ? 0 : 1;
+    float2 e = psub(nf, make_float2(h.imp.z, h.imp.w));
+    if (!(fabsf(e.x) > kZero || fabsf(e.y) > kZero)) e = make_float2(0.f, 0.f);
+    half_axpy1(v, h.m + 3, e.x);
+    half_axpy1(v, h.m + 6, e.y);
+    h.imp.x = ix;
+    h.imp.z = __fadd_rn(h.imp.z, e.x);
+    h.imp.w = __fadd_rn(h.imp.w, e.y);
+}
+
+// A chain's rows in shared memory.  An island of at most kRingSlots chunks is
+// resident: every chunk is copied in once and the passes run over it in
+// place, impulses included.  A larger one streams through the ring, chunk c
+// of a pass at sequence t = pass * chunks + c, looked ahead by at most one
+// pass (a pass must see the impulses the previous pass wrote back).
+struct RowFeed {
+    RowBlock* ring;
+    uint64_t* bars;
+    RowBlock* rows;        // the island's rows in global memory
+    uint32_t phase;        // bit k: parity of slot k
+    int rc, nch, total, ahead;
+    int t, slot;           // the chunk being read: sequence, ring slot
+    int issued, islot, ic; // the next chunk to copy: sequence, ring slot, chunk index
+    int fenced;            // sequence of the last proxy fence
+    int first_write;       // sequence from which passes write impulses back
+    bool lead;
+    long long limit;
+
+    // Copies the next chunk; the rows up to sequence `now` have been written
+    // back.  A proxy fence covers every impulse write issued before it; the
+    // chunk was last written at sequence issued - nch, so a fence is needed
+    // only if none was issued since: about once per pass on a large island.
+    __device__ __forceinline__ void issue(int now) {
+        const int tw = issued - nch;
+        const bool fence = tw >= first_write && tw > fenced;
         if (fence) fenced = now;
-        ring_load(ring + slot * kChunkRows, d.rows + rs + c * kChunkRows, n, &bars[slot], fence);
-    };
-    for (int t = 0; t < ahead && t < total; t++) issue(t, -1);
-    for (int t = 0; t < total; t++) {
-        const int slot = t % kRingSlots, pass = t / nch, c = t % nch;
-        if (!ring_wait(&bars[slot], (phase >> slot) & 1u, d.wait_limit)) {
-            // gave up on chunk t: let the copies already issued (chunks t to
-            // t + ahead - 1) land before the ring is abandoned (bounded)
-            for (int u = t; u < t + ahead && u < total; u++) {
-                const int su = u % kRingSlots;
-                ring_wait(&bars[su], (phase >> su) & 1u, kDefaultWaitLimit);
+        if (lead)
+            ring_load(ring + islot * kChunkRows, rows + ic * kChunkRows, min(kChunkRows, rc - ic * kChunkRows), &bars[islot], fence);
+        issued++;
+        if (++islot == kRingSlots) islot = 0;
+        if (++ic == nch) ic = 0;
+    }
+    // the rows of the chunk at sequence t are in shared memory
+    __device__ __forceinline__ bool arrive() {
+        if (!ring_wait(&bars[slot], (phase >> slot) & 1u, limit)) {
+            // gave up on chunk t: let the copies in flight land before the
+            // ring is abandoned (bounded)
+            for (int u = t; u < issued; u++) {
+                ring_wait(&bars[slot], (phase >> slot) & 1u, kDefaultWaitLimit);
+                if (++slot == kRingSlots) slot = 0;
             }
             return false;
         }
         phase ^= 1u << slot;
-        const int n = min(kChunkRows, rc - c * kChunkRows);
-        const float4* rb = reinterpret_cast<const float4*>(ring + slot * kChunkRows);
-        RowBlock* g = d.rows + rs + c * kChunkRows;
-        auto load = [&](int j, RowBlock& R) {
-            float4* dst = reinterpret_cast<float4*>(&R);
-#pragma unroll
-            for (int k = 0; k < (int)(sizeof(RowBlock) / 16); k++) dst[k] = rb[j * (sizeof(RowBlock) / 16) + k];
-        };
-        // one loop per pass kind (the pass is fixed within a chunk); the
-        // friction state is read only after the last velocity pass, so only
-        // that pass stores it
-        if (pass == 0) {
-            for (int j = 0; j < n; j++) {
-                RowBlock R;
-                load(j, R);
-                float4 imp = R.imp;
-                row_warm(R, imp, dv);
-                if (fused) {
-                    row_pos(R, imp, dv);
-                    g[j].imp = imp;
-                }
-            }
-        } else if (pass <= n_vel) {
-            // consecutive rows of one body pair (the points of a manifold)
-            // keep the pair's Δv in registers: the array is read when the
-            // pair changes and written back when it changes again (at the
-            // latest at the end of the pass), so the chain skips the
-            // shared-memory round trip between such rows
-            const bool last_vel = pass == n_vel;
-            for (int j = 0; j < n; j++) {
-                RowBlock R;
-                load(j, R);
-                if (R.sa != cur_a || R.sb != cur_b) {
-                    dv_put(dv, cur_a, 0, ca);
-                    dv_put(dv, cur_b, 0, cb);
-                    cur_a = R.sa;
-                    cur_b = R.sb;
-                    ca = dv_get(dv, cur_a, 0);
-                    cb = dv_get(dv, cur_b, 0);
-                }
-                float4 imp = R.imp;
-                int st = R.stat;
-                row_vel_r(R, imp, st, ca, cb);
-                g[j].imp = imp;
-                if (last_vel) g[j].stat = st;
-            }
-            if (c == nch - 1) {
-                dv_put(dv, cur_a, 0, ca);
-                dv_put(dv, cur_b, 0, cb);
-                cur_a = cur_b = -1;
-            }
+        return true;
+    }
+    __device__ __forceinline__ void advance() {
+        t++;
+        if (++slot == kRingSlots) slot = 0;
+    }
+    __device__ __forceinline__ RowBlock* rows_at() const { return ring + slot * kChunkRows; }
+    // the rows of the chunks up to sequence t - 1 have been read and their
+    // impulses written: refill their slots
+    __device__ __forceinline__ void refill() {
+        while (issued < total && issued < t + ahead) issue(t - 1);
+    }
+};
+
+// A run of n consecutive rows at `row` (shared memory), in order; KIND 0: warm
+// start, with the first position pass fused in when there is one (the position
+// rows read and write only the pseudo velocities and the pseudo impulse, which
+// no other pass touches and which start at zero, so position row j right after
+// warm-start row j gives the same result as a separate pass, one pass sooner);
+// 1: a velocity pass; 3: the last one (the friction state is stored too); 2: a
+// position pass.  The first row is already in `A`; each row's successor (`then`
+// after the last one) is loaded while the row is solved, without a branch in a
+// row's code.  Impulses go to `out`; `fin`: also there (KIND 3).
+// SH: `dv` is in shared memory with a zero entry at index -1 for the bodies of
+// infinite mass (their M^-1 J^T is zero, so it stays zero).
+struct ChainState {
+    P3 v, p;       // Δv and pseudo Δv of the lane's body
+    int own;       // its slot
+    int side;      // the side of the row it is on
+    int sa, sb;    // the row's slots
+};
+template <int KIND, bool SH, bool FUSED>
+__device__ __forceinline__ void chain_run(const RowBlock* row, int n, const RowBlock* then, RowBlock* out, RowBlock* fin, float4* dv,
+                                          ChainState& c, HalfRow& A) {
+    constexpr bool kV = KIND != 2, kP = KIND == 2 || (KIND == 0 && FUSED);
+    int left = n;
+    auto step = [&](HalfRow& cur, HalfRow& nxt) {
+        left--;
+        const RowBlock* next = left == 0 ? then : row + 1;
+        const int na = next->sa, nb = next->sb;
+        // a body that changes sides stays with its lane
+        const int nside = c.side ^ (int)((na == c.sb) | (nb == c.sa));
+        const int nown = nside ? nb : na;
+        half_load(next, nside, nxt);
+        P3 nv{}, np{};
+        if (kV) nv = dv_load<SH>(dv, nown, 0);
+        if (kP) np = dv_load<SH>(dv, nown, 1);
+        int stat = 0;
+        if (KIND == 0) {
+            half_warm(cur, c.v);
+            if (FUSED) half_pos(cur, c.p);
+        } else if (KIND == 2) {
+            half_pos(cur, c.p);
         } else {
-            for (int j = 0; j < n; j++) {
-                RowBlock R;
-                load(j, R);
-                float4 imp = R.imp;
-                row_pos(R, imp, dv);
-                g[j].imp = imp;
-            }
+            half_vel(cur, c.v, stat);
         }
-        if (t + ahead < total) issue(t + ahead, t);
+        if (KIND != 0 || FUSED) {   // both lanes, the same value
+            out->imp = cur.imp;
+            if (KIND == 3) {
+                fin->imp = cur.imp;
+                fin->stat = stat;
+                fin++;
+            }
+            out++;
+        }
+        if (kV) dv_store<SH>(dv, c.own, 0, c.v);
+        if (kP) dv_store<SH>(dv, c.own, 1, c.p);
+        __syncwarp(0xffffffffu);   // the other lane may read this body next
+        const bool keep = nown == c.own;
+        if (kV) c.v = psel(keep, c.v, nv);
+        if (kP) c.p = psel(keep, c.p, np);
+        c.own = nown;
+        c.side = nside;
+        c.sa = na;
+        c.sb = nb;
+        row = next;
+    };
+    HalfRow B;
+    while (left > 1) {
+        step(A, B);
+        step(B, A);
+    }
+    if (left) step(A, B);
+}
+
+// One pass over the island's rows.  RES: the rows are resident (one run in
+// place, impulses included); otherwise a run per chunk, the next chunk's
+// arrival waited for before the run that looks ahead to it.
+template <int KIND, bool SH, bool RES, bool FUSED>
+__device__ __forceinline__ bool chain_pass(RowFeed& x, float4* dv, int lane) {
+    constexpr bool kV = KIND != 2, kP = KIND == 2 || (KIND == 0 && FUSED);
+    if (!RES) {
+        x.refill();
+        if (!x.arrive()) return false;
+    }
+    RowBlock* row = RES ? x.ring : x.rows_at();
+    ChainState c{};
+    c.sa = row->sa;
+    c.sb = row->sb;
+    c.side = lane;
+    c.own = lane ? c.sb : c.sa;
+    if (kV) c.v = dv_load<SH>(dv, c.own, 0);
+    if (kP) c.p = dv_load<SH>(dv, c.own, 1);
+    HalfRow A;
+    half_load(row, lane, A);
+    if (RES) {
+        chain_run<KIND, SH, FUSED>(row, x.rc, row, row, x.rows, dv, c, A);
+    } else {
+        RowBlock* out = x.rows;
+        for (int k = 0; k < x.nch; k++) {
+            const int n = min(kChunkRows, x.rc - k * kChunkRows);
+            RowBlock* then = row;
+            x.refill();
+            x.advance();
+            if (k + 1 < x.nch) {
+                if (!x.arrive()) return false;
+                then = x.rows_at();
+            }
+            chain_run<KIND, SH, FUSED>(row, n, then, out, out, dv, c, A);
+            row = then;
+            out += n;
+        }
     }
     return true;
 }
 
-// One warp's solver-chain worker: takes big-island list entries q0, q0+1, ...
-// (below q1) through `counter` and runs each island's chain.  `sm`: the
-// warp's own shared area (mbarriers, row ring, Δv of up to `dv_cap` bodies).
-// False when a bounded wait gave up (the status is set).
-__device__ bool big_worker(const Dev& d, int dv_cap, uint8_t* sm, int* counter, int q0, int q1) {
+// the chain of one island: 1 warm-start pass, pgs_vel velocity passes and
+// pgs_pos position passes over its rows
+template <bool SH, bool RES>
+__device__ __forceinline__ bool chain_passes(RowFeed& x, float4* dv, int lane, int n_vel, int n_pos) {
+    if (RES)
+        while (x.t < x.total) {
+            if (!x.arrive()) return false;
+            x.advance();
+        }
+    bool ok = n_pos > 0 ? chain_pass<0, SH, RES, true>(x, dv, lane & 1) : chain_pass<0, SH, RES, false>(x, dv, lane & 1);
+    for (int k = 1; ok && k < n_vel; k++) ok = chain_pass<1, SH, RES, false>(x, dv, lane & 1);
+    if (ok && n_vel > 0) ok = chain_pass<3, SH, RES, false>(x, dv, lane & 1);
+    for (int k = 1; ok && k < n_pos; k++) ok = chain_pass<2, SH, RES, false>(x, dv, lane & 1);
+    return ok;
+}
+template <bool SH>
+__device__ __forceinline__ bool big_chain(const Dev& d, RowBlock* ring, uint64_t* bars, uint32_t& phase, float4* dv, int rs,
+                                       int rc, const WorldParams& P, int lane) {
+    const int n_vel = P.pgs_vel;   // read once: the row stores could alias P for the compiler
+    const int n_pos = P.pgs_pos;
+    const bool fused = n_pos > 0;
+    const int passes = 1 + n_vel + (fused ? n_pos - 1 : 0);
+    RowFeed x;
+    x.ring = ring;
+    x.bars = bars;
+    x.rows = d.rows + rs;
+    x.phase = phase;
+    x.rc = rc;
+    x.nch = (rc + kChunkRows - 1) / kChunkRows;
+    const bool resident = x.nch <= kRingSlots;
+    x.total = resident ? x.nch : passes * x.nch;
+    x.ahead = x.nch < kRingSlots ? x.nch : kRingSlots;
+    x.t = x.slot = x.issued = x.islot = x.ic = 0;
+    x.fenced = -1;
+    x.first_write = fused ? 0 : x.nch;
+    x.lead = lane == 0;
+    x.limit = d.wait_limit;
+    // the previous island may have written the ring in place
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp(0xffffffffu);
+    x.refill();
+    const bool ok = resident ? chain_passes<SH, true>(x, dv, lane, n_vel, n_pos) : chain_passes<SH, false>(x, dv, lane, n_vel, n_pos);
+    phase = x.phase;
+    return ok;
+}
+
+// One warp's solver-chain worker: takes the big-island list's entries through
+// `counter` and runs the chains of its islands -- SH: those of at most `dv_cap`
+// bodies, whose Δv stays in shared memory; otherwise the larger ones, Δv in
+// global memory.  `sm`: the warp's own shared area (mbarriers, row ring, the
+// zero entry of the bodies of infinite mass, Δv).  A bounded wait that gives
+// up ends the worker (the status is set).
+template <bool SH>
+__device__ void big_worker(const Dev& d, int dv_cap, uint8_t* sm, int* counter, int n) {
     uint64_t* bars = reinterpret_cast<uint64_t*>(sm);
     RowBlock* ring = reinterpret_cast<RowBlock*>(sm + 64);
-    float4* sdv = reinterpret_cast<float4*>(sm + 64 + kRingSlots * kChunkRows * sizeof(RowBlock));
+    float4* sdv = reinterpret_cast<float4*>(sm + 64 + kRingSlots * kChunkRows * sizeof(RowBlock)) + kDvF4;
     const int lane = threadIdx.x & 31;
     if (lane == 0)
         for (int k = 0; k < kRingSlots; k++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(&bars[k])), "r"(1) : "memory");
         }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (SH && lane < kDvF4) sdv[lane - kDvF4] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncwarp();
     uint32_t phase = 0;   // bit k: parity of slot k
     while (true) {
         int q = 0;
-        if (lane == 0) q = q0 + atomicAdd(counter, 1);
+        if (lane == 0) q = atomicAdd(counter, 1);
         q = __shfl_sync(0xffffffffu, q, 0);
-        if (q >= q1) break;
+        if (q >= n) break;
         const int i = d.big_list[q];
-        const int rs = d.g_isl_row_start[i], rc = d.g_isl_row_count[i];
         const int bs = d.g_isl_body_start[i], bc = d.g_isl_body_count[i];
+        if (SH != (bc <= dv_cap)) continue;
+        const int rs = d.g_isl_row_start[i], rc = d.g_isl_row_count[i];
         const WorldParams& P = d.wparams[d.g_isl_world[i]];
-        float4* dv = (bc <= dv_cap) ? sdv : d.dv + kDvF4 * (size_t)bs;
+        float4* dv = SH ? sdv : d.dv + kDvF4 * (size_t)bs;
         for (int k = lane; k < kDvF4 * bc; k += 32) dv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         __syncwarp();
-        bool ok = true;
-        if (lane == 0) {
-            ok = (bc <= dv_cap) ? big_chain(d, ring, bars, phase, sdv, rs, rc, P)
-                                : big_chain(d, ring, bars, phase, d.dv + kDvF4 * (size_t)bs, rs, rc, P);
-            if (!ok) atomicOr(d.status, ST_TIMEOUT);
+        bool ok = big_chain<SH>(d, ring, bars, phase, dv, rs, rc, P, lane);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) {
+            if (lane == 0) atomicOr(d.status, ST_TIMEOUT);
+            return;
         }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (!ok) return false;
         __syncwarp();
         island_finish(d, rs, rc, bs, bc, dv, lane, 32);
         __syncwarp();
     }
-    return true;
 }
 
+// sched[kBigNext + (SH ? 0 : 1)]: the next list entry
+constexpr int kBigNext = 8;
+
 // blockDim.x == 32; `dv_cap` island bodies fit in the shared Δv area
+template <bool SH>
 __global__ void __launch_bounds__(32) k_pgs_big(Dev d, int dv_cap) {
     extern __shared__ __align__(16) uint8_t sm[];
-    big_worker(d, dv_cap, sm, &d.sched[2], 0, d.sched[0]);
+    big_worker<SH>(d, dv_cap, sm, &d.sched[kBigNext + (SH ? 0 : 1)], d.sched[0]);
 }
 
 // HolonomicSystem::computeAndApplyImpulses (HolonomicBlockSolver.cpp:319-378)
@@ -898,13 +1150,13 @@ void launch_rows(const Dev& d, int first, int last, const Launch& L) {
 }
 
 int pgs_big_smem_bytes(int dv_cap) {
-    return 64 + kRingSlots * kChunkRows * (int)sizeof(RowBlock) + dv_cap * 16 * kDvF4;
+    return 64 + kRingSlots * kChunkRows * (int)sizeof(RowBlock) + (dv_cap + 1) * 16 * kDvF4;
 }
 
 // blocks of k_pgs_big resident per SM for this Δv capacity (one chain each)
 int pgs_big_blocks_per_sm(int dv_cap) {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_pgs_big, 32, pgs_big_smem_bytes(dv_cap)) != cudaSuccess || n < 1) n = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_pgs_big<true>, 32, pgs_big_smem_bytes(dv_cap)) != cudaSuccess || n < 1) n = 1;
     return n;
 }
 
@@ -913,7 +1165,7 @@ int pgs_big_blocks_per_sm(int dv_cap) {
 // a smaller one does not lower the limit under an earlier batch's launches
 void prepare_pgs(int dv_cap) {
     (void)dv_cap;
-    cudaFuncSetAttribute(k_pgs_big, cudaFuncAttributeMaxDynamicSharedMemorySize, pgs_big_smem_bytes(kPgsDvCapMax));
+    cudaFuncSetAttribute(k_pgs_big<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, pgs_big_smem_bytes(kPgsDvCapMax));
 }
 
 void launch_pgs_schedule(const Dev& d, const Launch& L) {
@@ -927,14 +1179,18 @@ void launch_pgs_joint(const Dev& d, bool first, const Launch& L) {
     k_pgs_joint<<<L.n_sms * 8, 32, 0, L.st>>>(d, first ? 1 : 0);
 }
 
-void launch_pgs(const Dev& d, int dv_cap, int big_blocks, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, const Launch& L) {
-    // large islands on the main stream, small ones concurrently on a side branch
-    cudaMemsetAsync(d.sched + 2, 0, sizeof(int), L.st);
+void launch_pgs(const Dev& d, int dv_cap, int max_world, int big_blocks, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join,
+                const Launch& L) {
+    // large islands on the main stream, small ones (and islands whose Δv does
+    // not fit in shared memory, where a world is large enough to hold one)
+    // concurrently on a side branch
+    cudaMemsetAsync(d.sched + kBigNext, 0, 2 * sizeof(int), L.st);
     cudaEventRecord(fork, L.st);
     cudaStreamWaitEvent(side, fork, 0);
+    if (max_world > dv_cap) k_pgs_big<false><<<L.n_sms, 32, pgs_big_smem_bytes(0), side>>>(d, dv_cap);
     k_pgs_small<<<L.n_sms * 4, 64, 0, side>>>(d);
     cudaEventRecord(join, side);
-    k_pgs_big<<<big_blocks, 32, pgs_big_smem_bytes(dv_cap), L.st>>>(d, dv_cap);
+    k_pgs_big<true><<<big_blocks, 32, pgs_big_smem_bytes(dv_cap), L.st>>>(d, dv_cap);
     cudaStreamWaitEvent(L.st, join, 0);
 }
 
