@@ -5,25 +5,25 @@
 // every pair of bodies of the same world whose true AABBs overlap under the
 // inclusive test of AABB::intersects (ConstraintPhysics/src/AABB.h:10-14; the
 // tree query AABB_Tree.h:153-224 visits every overlapping leaf pair once).
-// Pairs are emitted as (lower id, higher id) sorted by (a, b): one thread per
-// body counts its overlaps with the later bodies of its world, an exclusive
-// scan gives each body its output offset, and a second pass writes.  Worlds
-// above kTileWorld bodies (where one thread per body would loop over up to
-// the whole world) run the same test over kTile x kTile blocks instead.
+// Pairs are emitted as (lower id, higher id) sorted by (a, b): a warp counts the
+// overlaps of kPairGroup consecutive bodies with the later bodies of their
+// world, 32 of those at a time, an exclusive scan gives each body its output
+// offset, and a second pass writes.  Bound by the tests' FP32 issue in large
+// worlds and by latency in small ones; a thread per body (each walking the
+// rest of its world alone) took 117 us a pass on one world of 1,000 bodies
+// where this takes 6.  The bodies of worlds above kTileWorld bodies go into a
+// hashed grid instead (pairs.cuh).
 #include <algorithm>
 
 #include "kernels.cuh"
 #include "devmath.cuh"
+#include "pairs.cuh"
 #include "shapes.cuh"
 
 namespace cpgpu {
 
 namespace {
 constexpr int kScanBlock = 1024;
-
-__device__ __forceinline__ bool overlap(float4 alo, float4 ahi, float4 blo, float4 bhi) {
-    return !(ahi.x < blo.x || alo.x > bhi.x || ahi.y < blo.y || alo.y > bhi.y || ahi.z < blo.z || alo.z > bhi.z);
-}
 
 // inclusive block scan of one value per thread (blockDim.x == kScanBlock)
 __device__ int block_scan_incl(int v, int* warp_sums) {
@@ -97,83 +97,101 @@ __global__ void k_gravity(Dev d) {
     }
 }
 
-__global__ void k_pairs(Dev d, int write) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < d.n_bodies; i += gridDim.x * blockDim.x) {
-        if (d.n_tile_tasks > 0 && d.tile_base[d.world[i]] >= 0) continue;   // a large world: k_pairs_tile
-        const int end = d.world_start[d.world[i] + 1];
-        const float4 lo = d.aabb_lo[i], hi = d.aabb_hi[i];
+struct BodyBox {
+    const float4 *lo, *hi;
+    __device__ __forceinline__ PairBox operator()(int j) const {
+        const float4 l = lo[j], h = hi[j];
+        return PairBox{l.x, l.y, l.z, h.x, h.y, h.z};
+    }
+};
+__global__ void __launch_bounds__(256) k_pairs(Dev d, int write) {
+    const int nw = gridDim.x * (blockDim.x >> 5);
+    const bool big = d.grid_buckets > 0;   // the batch holds worlds of the grid
+    const BodyBox load{d.aabb_lo, d.aabb_hi};
+    auto end = [&](int i) {
+        const int w = d.world[i], e = d.world_start[w + 1];
+        return big && e - d.world_start[w] > kTileWorld ? 0 : e;
+    };
+    for (int i0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kPairGroup; i0 < d.n_bodies; i0 += nw * kPairGroup) {
+        int c[kPairGroup];
         if (!write) {
-            int c = 0;
-            for (int j = i + 1; j < end; j++) c += overlap(lo, hi, d.aabb_lo[j], d.aabb_hi[j]);
-            d.pair_count[i] = c;
+            pairs_of_group<kPairGroup>(i0, d.n_bodies, load, end, [](int, int, int) {}, c);
+            if ((threadIdx.x & 31) == 0)
+#pragma unroll
+                for (int g = 0; g < kPairGroup; g++)
+                    if (i0 + g < d.n_bodies && !(big && end(i0 + g) == 0)) d.pair_count[i0 + g] = c[g];
         } else {
-            int o = d.pair_count[i];
-            for (int j = i + 1; j < end; j++) {
-                if (overlap(lo, hi, d.aabb_lo[j], d.aabb_hi[j])) {
-                    if (o < d.cap_pairs) { d.pair_a[o] = i; d.pair_b[o] = j; }
-                    o++;
-                }
-            }
+            int o[kPairGroup];
+#pragma unroll
+            for (int g = 0; g < kPairGroup; g++) o[g] = i0 + g < d.n_bodies ? d.pair_count[i0 + g] : 0;
+            pairs_of_group<kPairGroup>(i0, d.n_bodies, load, end, [&](int g, int j, int k) {
+                int at = o[0];
+#pragma unroll
+                for (int q = 1; q < kPairGroup; q++) at = g == q ? o[q] : at;
+                at += k;
+                if (at < d.cap_pairs) { d.pair_a[at] = i0 + g; d.pair_b[at] = j; }
+            }, c);
         }
     }
 }
 
-// Large worlds: a block per (i tile, j tile >= i tile) of the world's bodies;
-// the j tile's AABBs are staged in shared memory and each thread tests its
-// body i against them (j > i).  The count pass stores, per body and j tile,
-// the pairs found there; k_pairs_tile_rows turns a body's cells into their
-// prefix and its total; the write pass writes each body's pairs of a tile at
-// its offset plus the tile's prefix, in increasing j -- the same sorted
-// (a, b) list as the per-body loop, with every thread doing kTile tests.
-__global__ void __launch_bounds__(kTile) k_pairs_tile(Dev d, int write) {
-    __shared__ float4 slo[kTile], shi[kTile];
-    for (int q = blockIdx.x; q < d.n_tile_tasks; q += gridDim.x) {
-        const int4 t = d.tile_task[q];
-        const int s = d.world_start[t.x], e = d.world_start[t.x + 1];
-        const int j0 = s + t.z * kTile, jn = min(kTile, e - j0);
-        __syncthreads();   // the previous task's tile is no longer read
-        if ((int)threadIdx.x < jn) {
-            slo[threadIdx.x] = d.aabb_lo[j0 + threadIdx.x];
-            shi[threadIdx.x] = d.aabb_hi[j0 + threadIdx.x];
+// Large worlds: their bodies go into one hashed grid (keyed by the world too),
+// and a warp tests a body against those of its 27 cells.
+struct GridWorld {
+    const Dev& d;
+    __device__ __forceinline__ int operator()(int i) const { return d.world[i]; }
+};
+__device__ __forceinline__ PairGrid<int> dev_grid(const Dev& d) {
+    return PairGrid<int>{d.grid_bucket, d.grid_ids, d.grid_far, d.grid_n_far, d.grid_inv, d.grid_buckets};
+}
+__device__ __forceinline__ bool in_grid_world(const Dev& d, int i) {
+    const int w = d.world[i];
+    return d.world_start[w + 1] - d.world_start[w] > kTileWorld;
+}
+__global__ void __launch_bounds__(1024) k_grid_begin(Dev d) {
+    grid_begin(dev_grid(d), d.n_bodies, BodyBox{d.aabb_lo, d.aabb_hi}, [&](int i) { return in_grid_world(d, i); });
+}
+__global__ void __launch_bounds__(256) k_grid_put(Dev d, int pass) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < d.n_bodies; i += gridDim.x * blockDim.x)
+        if (in_grid_world(d, i)) grid_put(dev_grid(d), i, d.world[i], BodyBox{d.aabb_lo, d.aabb_hi}, pass);
+}
+__global__ void __launch_bounds__(1024) k_grid_buckets(Dev d) { block_prefix_1024(d.grid_bucket, d.grid_buckets); }
+__global__ void __launch_bounds__(256) k_grid_count(Dev d) {
+    const BodyBox load{d.aabb_lo, d.aabb_hi};
+    for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < d.n_bodies; i += gridDim.x * 8) {
+        if (!in_grid_world(d, i)) continue;
+        const int w = d.world[i];
+        int c = grid_near(dev_grid(d), i, w, load, GridWorld{d}, [](int) {});
+        if (c == -2) continue;   // k_grid_far's
+        if (c < 0) {
+            int one[1];
+            pairs_of_group<1>(i, d.n_bodies, load, [&](int) { return d.world_start[w + 1]; }, [](int, int, int) {}, one);
+            c = one[0];
         }
-        __syncthreads();
-        const int i = s + t.y * kTile + (int)threadIdx.x;
-        if (i >= e) continue;
-        const float4 lo = d.aabb_lo[i], hi = d.aabb_hi[i];
-        int* cell = d.tile_cnt + d.tile_base[t.x] + (size_t)(i - s) * t.w + t.z;
-        const int first = max(0, i + 1 - j0);   // j > i
-        if (!write) {
-            int c = 0;
-            for (int k = first; k < jn; k++) c += overlap(lo, hi, slo[k], shi[k]);
-            *cell = c;
-        } else {
-            int o = d.pair_count[i] + *cell;
-            for (int k = first; k < jn; k++) {
-                if (overlap(lo, hi, slo[k], shi[k])) {
-                    if (o < d.cap_pairs) { d.pair_a[o] = i; d.pair_b[o] = j0 + k; }
-                    o++;
-                }
-            }
-        }
+        if ((threadIdx.x & 31) == 0) d.pair_count[i] = c;
     }
 }
-
-// per large-world body: the prefix of its j-tile cells (from its own tile on)
-// and its pair count
-__global__ void k_pairs_tile_rows(Dev d) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < d.n_bodies; i += gridDim.x * blockDim.x) {
-        const int w = d.world[i], base = d.tile_base[w];
-        if (base < 0) continue;
-        const int s = d.world_start[w], e = d.world_start[w + 1];
-        const int T = (e - s + kTile - 1) / kTile;
-        int* row = d.tile_cnt + base + (size_t)(i - s) * T;
-        int acc = 0;
-        for (int jt = (i - s) / kTile; jt < T; jt++) {
-            const int c = row[jt];
-            row[jt] = acc;
-            acc += c;
-        }
-        d.pair_count[i] = acc;
+__global__ void __launch_bounds__(1024) k_grid_far(Dev d, int write) {
+    const int m = *d.grid_n_far;
+    for (int k = blockIdx.x; k < m; k += gridDim.x) {
+        const int i = d.grid_far[k], o = write ? d.pair_count[i] : 0;
+        const int c = grid_far(i, d.world_start[d.world[i] + 1], BodyBox{d.aabb_lo, d.aabb_hi}, write != 0, [&](int r, int j) {
+            if (o + r < d.cap_pairs) { d.pair_a[o + r] = i; d.pair_b[o + r] = j; }
+        });
+        if (!write && threadIdx.x == 0) d.pair_count[i] = c;
+    }
+}
+__global__ void __launch_bounds__(256) k_grid_write(Dev d) {
+    __shared__ int near[8][kGridNear], n_near[8];
+    const int wid = threadIdx.x >> 5;
+    const BodyBox load{d.aabb_lo, d.aabb_hi};
+    for (int i = blockIdx.x * 8 + wid; i < d.n_bodies; i += gridDim.x * 8) {
+        if (!in_grid_world(d, i)) continue;
+        const int o = d.pair_count[i], m = (i + 1 < d.n_bodies ? d.pair_count[i + 1] : *d.n_pairs) - o;
+        if (m == 0 || o >= d.cap_pairs) continue;
+        const int e = d.world_start[d.world[i] + 1];
+        grid_write(dev_grid(d), i, d.n_bodies, m, load, GridWorld{d}, [&](int) { return e; }, near[wid], &n_near[wid],
+                   [&](int k, int j) { if (o + k < d.cap_pairs) { d.pair_a[o + k] = i; d.pair_b[o + k] = j; } });
     }
 }
 
@@ -241,16 +259,23 @@ void launch_gravity(const Dev& d, const Launch& L) {
 }
 
 void launch_pairs(const Dev& d, const Launch& L) {
-    int g = grid_for(d.n_bodies, 128, L.n_sms);
-    const int gt = std::min(d.n_tile_tasks, L.n_sms * 16);
-    k_pairs<<<g, 128, 0, L.st>>>(d, 0);
-    if (d.n_tile_tasks > 0) {
-        k_pairs_tile<<<gt, kTile, 0, L.st>>>(d, 0);
-        k_pairs_tile_rows<<<g, 128, 0, L.st>>>(d);
+    const int g = grid_for(d.n_bodies, 8 * kPairGroup, L.n_sms), gw = grid_for(d.n_bodies, 8, 2 * L.n_sms);
+    const bool grid = d.grid_buckets > 0;
+    if (grid) {
+        k_grid_begin<<<17, 1024, 0, L.st>>>(d);
+        k_grid_put<<<grid_for(d.n_bodies, 256, L.n_sms), 256, 0, L.st>>>(d, 0);
+        k_grid_buckets<<<1, 1024, 0, L.st>>>(d);
+        k_grid_put<<<grid_for(d.n_bodies, 256, L.n_sms), 256, 0, L.st>>>(d, 1);
+        k_grid_count<<<gw, 256, 0, L.st>>>(d);
+        k_grid_far<<<64, 1024, 0, L.st>>>(d, 0);
     }
+    if (!d.all_grid) k_pairs<<<g, 256, 0, L.st>>>(d, 0);
     scan_exclusive(d.pair_count, d.pair_count, nullptr, d.n_bodies, d.n_bodies, d.n_pairs, d.scan_tmp, L);
-    k_pairs<<<g, 128, 0, L.st>>>(d, 1);
-    if (d.n_tile_tasks > 0) k_pairs_tile<<<gt, kTile, 0, L.st>>>(d, 1);
+    if (grid) {
+        k_grid_far<<<64, 1024, 0, L.st>>>(d, 1);
+        k_grid_write<<<gw, 256, 0, L.st>>>(d);
+    }
+    if (!d.all_grid) k_pairs<<<g, 256, 0, L.st>>>(d, 1);
     k_clamp_pairs<<<1, 1, 0, L.st>>>(d);
 }
 

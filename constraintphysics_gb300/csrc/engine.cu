@@ -577,7 +577,8 @@ struct Batch {
     bool unions = false;               // the batch holds bodies of several primitives
     bool joints = false;               // the batch holds joints (or springs: joint edges)
     bool springs = false;              // the batch holds springs
-    bool tiles = false;                // the batch holds worlds above kTileWorld bodies (tiled pair pass)
+    bool tiles = false;                // the batch holds worlds above kTileWorld bodies (pair grid)
+    bool all_tiles = false;            // ... and no others
     bool systems = false;              // ... and holonomic systems
     cudaStream_t st = nullptr;
     cudaStream_t side = nullptr;       // concurrent branch (small-island PGS)
@@ -659,7 +660,7 @@ struct Batch {
     // (+2 per substep and 1 factorisation with joints)
     int launches_per_step() const {
         return 1 + 6 + 2 + (prims ? 1 : 0) + ((meshes || unions) ? 1 : 0) + (6 + 9) + (2 + 3) + 3 + 5 * substeps + 1 + (joints ? 2 * substeps : 0) +
-               (systems ? 1 : 0) + (audit ? 1 : 0) + (springs ? substeps : 0) + (tiles ? 3 : 0) +
+               (systems ? 1 : 0) + (audit ? 1 : 0) + (springs ? substeps : 0) + (tiles ? (all_tiles ? 6 : 8) : 0) +
                (max_world > dv_cap ? substeps : 0);
     }
 
@@ -991,20 +992,17 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
     }
     B->n_bodies = N;
     B->world_start = wstart;
-    // large worlds' pair pass: tasks over (i tile, j tile >= i tile) blocks
-    std::vector<int4> tile_task;
-    std::vector<int> tile_base(worlds.size(), -1);
-    size_t tile_cells = 0;
+    // the bodies of large worlds go into the pair grid: about two a bucket
+    int64_t grid_bodies = 0;
     for (size_t k = 0; k < worlds.size(); k++) {
         const int n = wstart[k + 1] - wstart[k];
-        if (n <= kTileWorld) continue;
-        const int T = (n + kTile - 1) / kTile;
-        tile_base[k] = (int)tile_cells;
-        tile_cells += (size_t)n * T;
-        for (int it = 0; it < T; it++)
-            for (int jt = it; jt < T; jt++) tile_task.push_back(make_int4((int)k, it, jt, T));
+        if (n > kTileWorld) grid_bodies += n;
     }
-    B->tiles = !tile_task.empty();
+    int grid_buckets = 0;
+    if (grid_bodies > 0)
+        for (grid_buckets = 1024; grid_buckets < grid_bodies / 2 && grid_buckets < (1 << 17);) grid_buckets *= 2;
+    B->tiles = grid_bodies > 0;
+    B->all_tiles = grid_bodies == N;
     {
         int& max_world = B->max_world;
         for (size_t k = 0; k + 1 < wstart.size(); k++) max_world = std::max(max_world, wstart[k + 1] - wstart[k]);
@@ -1353,13 +1351,16 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
         d_pool = A.take<uint8_t>(pool.size());
         x.shapes = d_pool;
         x.pair_count = A.take<int>(N);
-        x.n_tile_tasks = (int)tile_task.size();
-        x.tile_task = A.take<int4>(tile_task.size());
-        x.tile_base = A.take<int>(worlds.size());
-        x.tile_cnt = A.take<int>(tile_cells);
+        x.grid_buckets = grid_buckets;
+        x.all_grid = B->all_tiles ? 1 : 0;
+        if (grid_buckets > 0) {
+            x.grid_bucket = A.take<int>(grid_buckets);
+            x.grid_ids = A.take<int>(N); x.grid_far = A.take<int>(N); x.grid_n_far = A.take<int>(1);
+            x.grid_inv = A.take<float>(1);
+        }
         // CPGPU_ISLANDS_SERIAL=1: large worlds take the serial search too (a
         // test compares the two)
-        if (!tile_task.empty() && !env_int("CPGPU_ISLANDS_SERIAL", 0)) {
+        if (grid_buckets > 0 && !env_int("CPGPU_ISLANDS_SERIAL", 0)) {
             x.comp = A.take<int>((size_t)kCompArrays * N);
             x.sys_mark = A.take<int>(std::max<size_t>(hs_degree.size(), 1));
         }
@@ -1496,13 +1497,11 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
     up(d_mov, movement.data(), N); up(d_mat, mat.data(), N * sizeof(float4));
     up(d_pool, pool.data(), pool.size());
     up(x.moved, fresh.data(), N * 4);   // the first geometry pass renormalises these orientations
-    up((void*)x.tile_task, tile_task.data(), tile_task.size() * sizeof(int4));
     if (B->unions) {
         up((void*)x.prim_start, prim_start.data(), N * 4); up((void*)x.prim_count, prim_count.data(), N * 4);
         up((void*)x.prim_shape, prim_shape.data(), prim_shape.size() * 4);
         up((void*)x.prim_mat, prim_mat.data(), prim_mat.size() * 16);
     }
-    up((void*)x.tile_base, tile_base.data(), tile_base.size() * 4);
     if (has_sleep) {
         up(x.asleep, s_asleep.data(), N * 4); up(x.waking, s_waking.data(), N * 4); up(x.ready_cnt, s_ready.data(), N * 4);
         up(x.non_sleepy, s_nons.data(), N * 4); up(x.hist_n, s_hn.data(), N * 4);

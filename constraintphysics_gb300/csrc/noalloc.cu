@@ -8,18 +8,23 @@
 // plugins that are handed pre-allocated input/output buffers and nothing
 // else.  cpgpu_pairs_noalloc serves them: the caller passes the AABBs and the
 // output buffers (device memory it already owns) and the call allocates
-// nothing.  Its only scratch (per-body overlap counts and the scan's chunk
-// sums) is a file-scope __device__ array of fixed size, so the maximum body
-// count per call is kNoAllocMaxBodies.
+// nothing.  Its only scratch (per-body overlap counts, and a grid's buckets) is
+// a file-scope __device__ array of fixed size, so the maximum body count per
+// call is kNoAllocMaxBodies.
 //
 // Same result as the batch path's pair generation (broadphase.cu): every pair
 // (i, j), i < j, whose AABBs overlap under the inclusive test, in (i, j)
 // order, ids 1-based.
+//
+// Up to kNoAllocBrute boxes a warp tests each box against all later ones, 32 at
+// a time (n^2 / 2 tests).  Above, the boxes go into a hashed grid and a warp
+// tests a box against those of its 27 cells.
 #include <cstdio>
 #include <mutex>
 #include <vector>
 
 #include "kernels.cuh"
+#include "pairs.cuh"
 
 extern "C" {
 #include "../../include/cpgpu.h"
@@ -28,72 +33,149 @@ extern "C" {
 namespace cpgpu {
 
 constexpr int kNoAllocMaxBodies = 1 << 16;
-constexpr int kNoAllocChunk = 1024;
-constexpr int kNoAllocChunks = kNoAllocMaxBodies / kNoAllocChunk;
+// the pass over all later boxes up to here, the grid above: 40 us against 51 at
+// 4,096 boxes, 91 against 67 at 8,192 (4.7 ms against 0.2 at 65,536)
+constexpr int kNoAllocBrute = 5120;
+constexpr int kNoAllocBuckets = 1 << 15;
 
 // Scratch of every call on a device: per-body overlap counts (turned into
-// output offsets in place) followed by the chunk sums.  Every GPU that loads
-// the library holds it (about 260 KB) until the process exits.
-static __device__ __align__(256) int g_noalloc_scratch[kNoAllocMaxBodies + kNoAllocChunks + 32];
+// output offsets in place), bucket starts, the boxes by bucket, the boxes that
+// do not go into the grid, and the grid's numbers.  Every GPU that loads the
+// library holds it (about 650 KB) until the process exits.
+struct NoAllocScratch {
+    int count[kNoAllocMaxBodies];
+    int bucket[kNoAllocBuckets];
+    int chunk[kNoAllocMaxBodies / 1024];  // overlaps per 1,024 boxes
+    uint16_t ids[kNoAllocMaxBodies];
+    uint16_t far_ids[kNoAllocMaxBodies];
+    int n_far, total;
+    float inv;
+};
+static __device__ __align__(256) NoAllocScratch g_noalloc_scratch;
 
 namespace {
 
-__device__ __forceinline__ bool overlap6(const float* a, const float* b) {
-    return !(a[3] < b[0] || a[0] > b[3] || a[4] < b[1] || a[1] > b[4] || a[5] < b[2] || a[2] > b[5]);
+struct NaLoad {
+    const float2* b;   // boxes of 6 floats, 8-byte aligned at the least
+    const float* f;
+    bool vec;
+    __device__ __forceinline__ explicit NaLoad(const float* aabbs)
+        : b(reinterpret_cast<const float2*>(aabbs)), f(aabbs), vec((reinterpret_cast<uintptr_t>(aabbs) & 7) == 0) {}
+    __device__ __forceinline__ PairBox operator()(int j) const {
+        if (vec) {
+            const float2 x = b[3 * j], y = b[3 * j + 1], z = b[3 * j + 2];
+            return PairBox{x.x, x.y, y.x, y.y, z.x, z.y};
+        }
+        const float* p = f + 6 * j;
+        return PairBox{p[0], p[1], p[2], p[3], p[4], p[5]};
+    }
+};
+struct NaEnd {
+    int n;
+    __device__ __forceinline__ int operator()(int) const { return n; }
+};
+__device__ __forceinline__ void na_put(uint32_t* pairs, int cap, int o, int i, int j) {
+    if (o < cap) { pairs[2 * (size_t)o] = (uint32_t)i + 1; pairs[2 * (size_t)o + 1] = (uint32_t)j + 1; }
 }
 
-__global__ void k_na_count(const float* aabbs, int n, int* scratch) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float* a = aabbs + 6 * i;
-        int c = 0;
-        for (int j = i + 1; j < n; j++) c += overlap6(a, aabbs + 6 * j);
-        scratch[i] = c;
+__global__ void __launch_bounds__(256) k_na_count(const float* aabbs, int n, NoAllocScratch* s) {
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (i >= n) return;
+    int c[1];
+    pairs_of_group<1>(i, n, NaLoad(aabbs), NaEnd{n}, [](int, int, int) {}, c);
+    if ((threadIdx.x & 31) == 0) s->count[i] = c[0];
+}
+__global__ void __launch_bounds__(1024) k_na_scan(int n, NoAllocScratch* s, int* count) {
+    const int total = block_prefix_1024(s->count, n);
+    if (threadIdx.x == 0) { *count = total; s->total = total; }
+}
+__global__ void __launch_bounds__(256) k_na_write(const float* aabbs, int n, const NoAllocScratch* s, uint32_t* pairs, int cap) {
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (i >= n) return;
+    const int o = s->count[i];
+    int c[1];
+    pairs_of_group<1>(i, n, NaLoad(aabbs), NaEnd{n}, [&](int, int j, int k) { na_put(pairs, cap, o + k, i, j); }, c);
+}
+
+// ---- the grid ------------------------------------------------------------------------
+__device__ __forceinline__ PairGrid<uint16_t> na_grid(NoAllocScratch* s) {
+    return PairGrid<uint16_t>{s->bucket, s->ids, s->far_ids, &s->n_far, &s->inv, kNoAllocBuckets};
+}
+struct NaWorld {   // one world
+    __device__ __forceinline__ int operator()(int) const { return 0; }
+};
+__global__ void __launch_bounds__(1024) k_na_begin(const float* aabbs, int n, NoAllocScratch* s) {
+    if (blockIdx.x == 0 && threadIdx.x < kNoAllocMaxBodies / 1024) s->chunk[threadIdx.x] = 0;
+    grid_begin(na_grid(s), n, NaLoad(aabbs), [](int) { return true; });
+}
+__global__ void __launch_bounds__(256) k_na_put(const float* aabbs, int n, NoAllocScratch* s, int pass) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) grid_put(na_grid(s), i, 0, NaLoad(aabbs), pass);
+}
+__global__ void __launch_bounds__(1024) k_na_buckets(NoAllocScratch* s) { block_prefix_1024(s->bucket, kNoAllocBuckets); }
+__global__ void __launch_bounds__(256) k_na_grid_count(const float* aabbs, int n, NoAllocScratch* s) {
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (i >= n) return;
+    const NaLoad load(aabbs);
+    int c = grid_near(na_grid(s), i, 0, load, NaWorld{}, [](int) {});
+    if (c == -2) return;   // k_na_far's
+    if (c < 0) {
+        int one[1];
+        pairs_of_group<1>(i, n, load, NaEnd{n}, [](int, int, int) {}, one);
+        c = one[0];
+    }
+    if ((threadIdx.x & 31) == 0) {
+        s->count[i] = c;
+        if (c > 0) atomicAdd(&s->chunk[i >> 10], c);
     }
 }
-
-// exclusive scan of scratch[0..n) in place, one chunk of 1024 per block; the
-// chunk totals go to scratch[kNoAllocMaxBodies + chunk]
-__global__ void k_na_scan_chunks(int n, int* scratch) {
-    __shared__ int ws[32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int i = blockIdx.x * kNoAllocChunk + threadIdx.x;
-    int v = (i < n) ? scratch[i] : 0, x = v;
-    for (int o = 1; o < 32; o <<= 1) { int t = __shfl_up_sync(0xffffffffu, x, o); if (lane >= o) x += t; }
+__global__ void __launch_bounds__(1024) k_na_far(const float* aabbs, int n, NoAllocScratch* s, uint32_t* pairs, int cap, int write) {
+    const int m = s->n_far;
+    for (int k = blockIdx.x; k < m; k += gridDim.x) {
+        const int i = s->far_ids[k], o = write ? s->count[i] : 0;
+        const int c = grid_far(i, n, NaLoad(aabbs), write != 0, [&](int r, int j) { na_put(pairs, cap, o + r, i, j); });
+        if (!write && threadIdx.x == 0) {
+            s->count[i] = c;
+            if (c > 0) atomicAdd(&s->chunk[i >> 10], c);
+        }
+    }
+}
+// counts to offsets, a block per 1,024 boxes: every block sums the chunks
+// before its own (at most 64)
+__global__ void __launch_bounds__(1024) k_na_offsets(int n, NoAllocScratch* s, int* count) {
+    __shared__ int ws[32], before;
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5, i = blockIdx.x * 1024 + t;
+    if (wid == 0) {
+        int x = 0, all = 0;
+        for (int k = lane; k < (int)gridDim.x; k += 32) { all += s->chunk[k]; if (k < (int)blockIdx.x) x += s->chunk[k]; }
+        x = __reduce_add_sync(0xffffffffu, x);
+        all = __reduce_add_sync(0xffffffffu, all);
+        if (lane == 0) {
+            before = x;
+            if (blockIdx.x == 0) { *count = all; s->total = all; }
+        }
+    }
+    const int v = i < n ? s->count[i] : 0;
+    int x = v;
+    for (int o = 1; o < 32; o <<= 1) { const int q = __shfl_up_sync(0xffffffffu, x, o); if (lane >= o) x += q; }
     if (lane == 31) ws[wid] = x;
     __syncthreads();
     if (wid == 0) {
         int y = ws[lane];
-        for (int o = 1; o < 32; o <<= 1) { int t = __shfl_up_sync(0xffffffffu, y, o); if (lane >= o) y += t; }
+        for (int o = 1; o < 32; o <<= 1) { const int q = __shfl_up_sync(0xffffffffu, y, o); if (lane >= o) y += q; }
         ws[lane] = y;
     }
     __syncthreads();
-    int incl = x + (wid > 0 ? ws[wid - 1] : 0);
-    if (i < n) scratch[i] = incl - v;
-    if (threadIdx.x == kNoAllocChunk - 1) scratch[kNoAllocMaxBodies + blockIdx.x] = incl;
+    if (i < n) s->count[i] = before + x - v + (wid > 0 ? ws[wid - 1] : 0);
 }
-
-// chunk offsets (one thread, at most 64 chunks) and the total pair count
-__global__ void k_na_scan_top(int n_chunks, int* scratch, int* count) {
-    int run = 0;
-    for (int c = 0; c < n_chunks; c++) {
-        int t = scratch[kNoAllocMaxBodies + c];
-        scratch[kNoAllocMaxBodies + c] = run;
-        run += t;
-    }
-    *count = run;
-}
-
-__global__ void k_na_write(const float* aabbs, int n, const int* scratch, uint32_t* pairs, int cap) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float* a = aabbs + 6 * i;
-        int o = scratch[i] + scratch[kNoAllocMaxBodies + i / kNoAllocChunk];
-        for (int j = i + 1; j < n; j++) {
-            if (overlap6(a, aabbs + 6 * j)) {
-                if (o < cap) { pairs[2 * (size_t)o] = (uint32_t)i + 1; pairs[2 * (size_t)o + 1] = (uint32_t)j + 1; }
-                o++;
-            }
-        }
-    }
+__global__ void __launch_bounds__(256) k_na_grid_write(const float* aabbs, int n, NoAllocScratch* s, uint32_t* pairs, int cap) {
+    __shared__ int near[8][kGridNear], n_near[8];
+    const int wid = threadIdx.x >> 5, i = blockIdx.x * 8 + wid;
+    if (i >= n) return;
+    const int o = s->count[i], m = (i + 1 < n ? s->count[i + 1] : s->total) - o;
+    if (m == 0 || o >= cap) return;
+    grid_write(na_grid(s), i, n, m, NaLoad(aabbs), NaWorld{}, NaEnd{n}, near[wid], &n_near[wid],
+               [&](int k, int j) { na_put(pairs, cap, o + k, i, j); });
 }
 
 // Device address of the scratch array, looked up with the device current
@@ -105,7 +187,7 @@ __global__ void k_na_write(const float* aabbs, int n, const int* scratch, uint32
 // on every call.
 typedef int (*CtxGetCurrentFn)(void**);
 typedef int (*CtxGetIdFn)(void*, unsigned long long*);
-struct NaCache { unsigned long long ctx_id; int* ptr; };
+struct NaCache { unsigned long long ctx_id; NoAllocScratch* ptr; };
 std::mutex g_na_mutex;
 std::vector<NaCache> g_na_cache;
 CtxGetCurrentFn g_ctx_current = nullptr;
@@ -130,7 +212,7 @@ bool current_context_id(unsigned long long* id) {
     return g_ctx_id(ctx, id) == 0;
 }
 
-int scratch_for_current_device(int** out) {
+int scratch_for_current_device(NoAllocScratch** out) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return CPGPU_ERR_NO_DEVICE;
     std::lock_guard<std::mutex> lock(g_na_mutex);
@@ -141,8 +223,8 @@ int scratch_for_current_device(int** out) {
     void* p = nullptr;
     if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess) return CPGPU_ERR_CUDA;
     // the lookup made the device's primary context current if it was not
-    if (current_context_id(&id)) g_na_cache.push_back({id, static_cast<int*>(p)});
-    *out = static_cast<int*>(p);
+    if (current_context_id(&id)) g_na_cache.push_back({id, static_cast<NoAllocScratch*>(p)});
+    *out = static_cast<NoAllocScratch*>(p);
     return CPGPU_OK;
 }
 
@@ -169,21 +251,30 @@ extern "C" int cpgpu_pairs_noalloc(const float* aabbs, int n_bodies, uint32_t* p
         set_last_error(msg);
         return CPGPU_ERR_CUDA;
     }
-    int* scratch = nullptr;
+    NoAllocScratch* scratch = nullptr;
     int rc = scratch_for_current_device(&scratch);
     if (rc != CPGPU_OK) {
         set_last_error("cpgpu_pairs_noalloc: no usable CUDA device or scratch symbol lookup failed");
         return rc;
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int n_chunks = (n_bodies + kNoAllocChunk - 1) / kNoAllocChunk;
-    const int grid = n_bodies > 0 ? (n_bodies + 127) / 128 : 1;
-    if (n_bodies > 0) {
-        k_na_count<<<grid, 128, 0, st>>>(aabbs, n_bodies, scratch);
-        k_na_scan_chunks<<<n_chunks, kNoAllocChunk, 0, st>>>(n_bodies, scratch);
+    const int warps = (n_bodies + 7) / 8;
+    if (n_bodies <= kNoAllocBrute) {
+        if (n_bodies > 0) k_na_count<<<warps, 256, 0, st>>>(aabbs, n_bodies, scratch);
+        k_na_scan<<<1, 1024, 0, st>>>(n_bodies, scratch, count);
+        if (n_bodies > 0) k_na_write<<<warps, 256, 0, st>>>(aabbs, n_bodies, scratch, pairs, cap);
+    } else {
+        const int per = (n_bodies + 255) / 256;
+        k_na_begin<<<17, 1024, 0, st>>>(aabbs, n_bodies, scratch);
+        k_na_put<<<per, 256, 0, st>>>(aabbs, n_bodies, scratch, 0);
+        k_na_buckets<<<1, 1024, 0, st>>>(scratch);
+        k_na_put<<<per, 256, 0, st>>>(aabbs, n_bodies, scratch, 1);
+        k_na_grid_count<<<warps, 256, 0, st>>>(aabbs, n_bodies, scratch);
+        k_na_far<<<64, 1024, 0, st>>>(aabbs, n_bodies, scratch, pairs, cap, 0);
+        k_na_offsets<<<(n_bodies + 1023) / 1024, 1024, 0, st>>>(n_bodies, scratch, count);
+        k_na_far<<<64, 1024, 0, st>>>(aabbs, n_bodies, scratch, pairs, cap, 1);
+        k_na_grid_write<<<warps, 256, 0, st>>>(aabbs, n_bodies, scratch, pairs, cap);
     }
-    k_na_scan_top<<<1, 1, 0, st>>>(n_chunks, scratch, count);
-    if (n_bodies > 0) k_na_write<<<grid, 128, 0, st>>>(aabbs, n_bodies, scratch, pairs, cap);
     if (cudaGetLastError() != cudaSuccess) {
         set_last_error("cpgpu_pairs_noalloc: kernel launch failed");
         return CPGPU_ERR_CUDA;

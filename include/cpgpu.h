@@ -433,7 +433,7 @@ int cpgpu_batch_read_audit(cpgpu_batch* b, double* out);               /* 10 per
  * plugins handed only pre-allocated buffers -- this computes the same
  * candidate pairs as the device path's pair generation for one set of AABBs
  * and allocates nothing: every buffer is the caller's device memory, and the
- * only scratch is a fixed file-scope device array (about 260 KB, held by
+ * only scratch is a fixed file-scope device array (about 650 KB, held by
  * every GPU that loads the library until the process exits).
  *   aabbs   device, n_bodies x 6 floats (min xyz, max xyz)
  *   pairs   device, cap x 2 uint32: (i, j) with 1-based ids, i < j, sorted
