@@ -11,7 +11,7 @@
 // offset, and a second pass writes.  Bound by the tests' FP32 issue in large
 // worlds and by latency in small ones; a thread per body (each walking the
 // rest of its world alone) took 117 us a pass on one world of 1,000 bodies
-// where this takes 6.  The bodies of worlds above kTileWorld bodies go into a
+// where this takes 12.  The bodies of worlds above kTileWorld bodies go into a
 // hashed grid instead (pairs.cuh).
 #include <algorithm>
 

@@ -1358,9 +1358,10 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
             x.grid_ids = A.take<int>(N); x.grid_far = A.take<int>(N); x.grid_n_far = A.take<int>(1);
             x.grid_inv = A.take<float>(1);
         }
-        // CPGPU_ISLANDS_SERIAL=1: large worlds take the serial search too (a
-        // test compares the two)
-        if (grid_buckets > 0 && !env_int("CPGPU_ISLANDS_SERIAL", 0)) {
+        // CPGPU_ISLANDS_SERIAL=1: every world takes the one-thread search (a
+        // test compares the searches)
+        x.isl_serial = env_int("CPGPU_ISLANDS_SERIAL", 0);
+        if (grid_buckets > 0 && !x.isl_serial) {
             x.comp = A.take<int>((size_t)kCompArrays * N);
             x.sys_mark = A.take<int>(std::max<size_t>(hs_degree.size(), 1));
         }

@@ -339,6 +339,7 @@ struct Dev {
     float* grid_inv;
     // islands of worlds above kTileWorld bodies: one DFS per connected
     // component, the components in parallel (kCompArrays ints per body)
+    int isl_serial;                // every world takes the one-thread search (a test compares)
     int* comp;
     int* sys_mark;                 // per holonomic system: the component that counted it
     // narrowphase output per pair
