@@ -10,12 +10,6 @@ namespace cpgpu {
 
 constexpr float kJZero = 0.00000001f;   // NVec::isZero cutoff (Math/src/NVec.h:4)
 
-__device__ __forceinline__ bool jzero(const float* x, int n) {
-    for (int i = 0; i < n; i++)
-        if (fabsf(x[i]) > kJZero) return false;
-    return true;
-}
-
 // Δv slots of one island: kDvF4 float4 per island body, 12 floats v xyz,
 // w xyz, pv xyz, pw xyz; `which` 0 = (v, w), 1 = (pv, pw)
 __device__ __forceinline__ void jload(const float4* dv, int slot, int which, float* out) {
@@ -23,12 +17,6 @@ __device__ __forceinline__ void jload(const float4* dv, int slot, int which, flo
     const float* f = reinterpret_cast<const float*>(dv + kDvF4 * slot) + 6 * which;
     for (int k = 0; k < 6; k++) out[k] = f[k];
 }
-__device__ __forceinline__ void jadd(float4* dv, int slot, int which, const float* x) {
-    if (slot < 0) return;
-    float* f = reinterpret_cast<float*>(dv + kDvF4 * slot) + 6 * which;
-    for (int k = 0; k < 6; k++) f[k] += x[k];
-}
-
 // J_a v_a + J_b v_b
 __device__ __forceinline__ void jvalue(const JointRow& R, const float* va, const float* vb, float* out) {
     for (int i = 0; i < R.n; i++) {
@@ -39,103 +27,102 @@ __device__ __forceinline__ void jvalue(const JointRow& R, const float* va, const
     }
 }
 
-// impulse_to_velocity * imp added to both bodies' slots (`which` 0 = velocity,
-// 1 = pseudo velocity)
-__device__ __forceinline__ void japply(const JointRow& R, const float* imp, float4* dv, int which) {
-    float xa[6], xb[6];
-    for (int k = 0; k < 6; k++) {
-        float x = 0.f, y = 0.f;
-        for (int i = 0; i < R.n; i++) { x += imp[i] * R.ita[kJMax * k + i]; y += imp[i] * R.itb[kJMax * k + i]; }
-        xa[k] = x;
-        xb[k] = y;
-    }
-    jadd(dv, R.sa, which, xa);
-    jadd(dv, R.sb, which, xb);
+// ---- one joint row by a warp ----------------------------------------------------
+// A row's work is spread over lanes so that a row-step is a few short chains
+// instead of a few hundred instructions on one lane: lane i < 6 has dof i (its
+// two Jacobian rows and its row of the effective mass inverse), lane c < 12
+// component c of M^-1 J^T and of the two bodies' Δv (a's six, then b's); lanes
+// meet by shuffles.  Every sum runs in the order of the one-thread form with
+// FMAs from zero, so the results are the same bits; dofs beyond the row's are
+// zeros.  Loaded one row ahead of its use.
+struct JointLane {
+    float ja[6], jb[6], minv[6];   // dof lane
+    float it[6];                   // component lane
+    float target, ptarget, acc, pacc, lim;
+    int n, sa, sb, proj, pos;
+};
+__device__ __forceinline__ void jl_row6(const float* p, float* o) {   // 8-byte aligned
+    const float2* q = reinterpret_cast<const float2*>(p);
+    const float2 x = q[0], y = q[1], z = q[2];
+    o[0] = x.x; o[1] = x.y; o[2] = y.x; o[3] = y.y; o[4] = z.x; o[5] = z.y;
 }
-
-// The same steps for a row of N dofs known at compile time (1: distance and
-// limits, 3: ball-socket, 4: sliding hinge, 5: hinge and slider, 6: weld):
-// every loop unrolls, so the row's entries are loaded once into registers
-// instead of through loops over a run-time count (identical sums)
-template <int N>
-__device__ __forceinline__ void japply_n(const JointRow& R, const float* imp, float4* dv, int which) {
-    float xa[6], xb[6];
-#pragma unroll
-    for (int k = 0; k < 6; k++) {
-        float x = 0.f, y = 0.f;
-#pragma unroll
-        for (int i = 0; i < N; i++) { x += imp[i] * R.ita[kJMax * k + i]; y += imp[i] * R.itb[kJMax * k + i]; }
-        xa[k] = x;
-        xb[k] = y;
-    }
-    jadd(dv, R.sa, which, xa);
-    jadd(dv, R.sb, which, xb);
+__device__ __forceinline__ void jl_load(const JointRow& R, int lane, JointLane& L) {
+    const int i = min(lane, 5), c = min(lane, 11);
+    L.n = R.n; L.sa = R.sa; L.sb = R.sb; L.proj = R.proj; L.pos = R.pos; L.lim = R.lim;
+    jl_row6(R.ja + 6 * i, L.ja);
+    jl_row6(R.jb + 6 * i, L.jb);
+    jl_row6(R.minv + kJMax * i, L.minv);
+    jl_row6(c < 6 ? R.ita + kJMax * c : R.itb + kJMax * (c - 6), L.it);
+    L.target = R.target[i];
+    L.ptarget = R.ptarget[i];
+    L.acc = R.impulse[i];
+    L.pacc = R.pimpulse[i];
 }
-
+// Δv of a body for `which`, zeros for infinite mass
+__device__ __forceinline__ void jl_dv(const float4* dv, int slot, int which, float* o) {
+    if (slot < 0) {
+#pragma unroll
+        for (int k = 0; k < 6; k++) o[k] = 0.f;
+        return;
+    }
+    jl_row6(reinterpret_cast<const float*>(dv + kDvF4 * slot) + 6 * which, o);
+}
+// component lane: sum of imp_i M^-1 J^T added to its component of Δv, where
+// lane i holds imp_i (zero beyond the row's dofs)
+__device__ __forceinline__ void jl_apply(const JointLane& L, float imp, float4* dv, int which, int lane) {
+    const int slot = lane < 6 ? L.sa : L.sb;
+    float x = 0.f;
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+        const float v = __shfl_sync(0xffffffffu, imp, i);
+        if (i < L.n) x = __fmaf_rn(v, L.it[i], x);
+    }
+    if (lane < 12 && slot >= 0) {
+        float* f = reinterpret_cast<float*>(dv + kDvF4 * slot) + 6 * which + (lane < 6 ? lane : lane - 6);
+        *f = __fadd_rn(*f, x);
+    }
+    __syncwarp();
+}
+// warm start (DegreedConstraint::applyWarmStartVelocityChange)
+__device__ __forceinline__ void jl_warm(const JointLane& L, float4* dv, int lane) {
+    if (__any_sync(0xffffffffu, lane < L.n && fabsf(L.acc) > kJZero)) jl_apply(L, L.acc, dv, 0, lane);
+}
 // PGSConstraintStep<n> (ConstraintSolver.cpp:12-40): the accumulated impulse
 // plus the row's correction, projected (ConeLimitConstraint /
 // TwistLimitConstraint::projectValidImpulse, ConstraintSolver.cpp:434-436,
-// 463-465: one-sided limits), applied when the change is not zero
-template <int N>
-__device__ __forceinline__ void jstep_n(JointRow& R, float4* dv, bool pseudo) {
+// 463-465: one-sided limits; MotorConstraint / PistonConstraint, :591-606,
+// 728-731), applied when the change is not zero
+__device__ __forceinline__ void jl_step(const JointLane& L, JointRow& R, float4* dv, bool pseudo, int lane) {
     const int which = pseudo ? 1 : 0;
-    float va[6], vb[6], delta[N], diff[N], acc[N];
-    jload(dv, R.sa, which, va);
-    jload(dv, R.sb, which, vb);
-    float* accp = pseudo ? R.pimpulse : R.impulse;
-    const float* tgt = pseudo ? R.ptarget : R.target;
+    float va[6], vb[6];
+    jl_dv(dv, L.sa, which, va);
+    jl_dv(dv, L.sb, which, vb);
+    float x = 0.f, y = 0.f;
 #pragma unroll
-    for (int i = 0; i < N; i++) {
-        float x = 0.f, y = 0.f;
-#pragma unroll
-        for (int k = 0; k < 6; k++) x += va[k] * R.ja[6 * i + k];
-#pragma unroll
-        for (int k = 0; k < 6; k++) y += vb[k] * R.jb[6 * i + k];
-        delta[i] = tgt[i] - (x + y);
-        acc[i] = accp[i];
+    for (int k = 0; k < 6; k++) {
+        x = __fmaf_rn(va[k], L.ja[k], x);
+        y = __fmaf_rn(vb[k], L.jb[k], y);
     }
-    bool zero = true;
+    const float delta = __fsub_rn(pseudo ? L.ptarget : L.target, __fadd_rn(x, y));
+    const float acc = pseudo ? L.pacc : L.acc;
+    float s = 0.f;
 #pragma unroll
-    for (int i = 0; i < N; i++) {
-        float x = 0.f;
-#pragma unroll
-        for (int k = 0; k < N; k++) x += delta[k] * R.minv[kJMax * i + k];
-        float nw = acc[i] + x;
-        if (N == 1 && R.proj == 1) nw = fmaxf(nw, 0.f);
-        else if (N == 1 && R.proj == 2) nw = fminf(nw, 0.f);
-        // MotorConstraint / PistonConstraint::projectValidImpulse
-        // (ConstraintSolver.cpp:591-606, 728-731)
-        else if (N == 1 && R.proj == 3) nw = nw > 0.f ? fminf(nw, R.lim) : fmaxf(nw, -R.lim);
-        diff[i] = nw - acc[i];
-        zero = zero && !(fabsf(diff[i]) > kJZero);
+    for (int k = 0; k < 6; k++) {
+        const float v = __shfl_sync(0xffffffffu, delta, k);
+        if (k < L.n) s = __fmaf_rn(v, L.minv[k], s);
     }
-    if (!zero) {
-        japply_n<N>(R, diff, dv, which);
-#pragma unroll
-        for (int i = 0; i < N; i++) accp[i] = acc[i] + diff[i];
+    float nw = __fadd_rn(acc, s);
+    if (L.n == 1 && L.proj != 0) {
+        if (L.proj == 1) nw = fmaxf(nw, 0.f);
+        else if (L.proj == 2) nw = fminf(nw, 0.f);
+        else nw = nw > 0.f ? fminf(nw, L.lim) : fmaxf(nw, -L.lim);
     }
-}
-
-// warm start (DegreedConstraint::applyWarmStartVelocityChange)
-__device__ __forceinline__ void jwarm(const JointRow& R, float4* dv) {
-    if (jzero(R.impulse, R.n)) return;
-    switch (R.n) {
-        case 1: japply_n<1>(R, R.impulse, dv, 0); break;
-        case 3: japply_n<3>(R, R.impulse, dv, 0); break;
-        case 4: japply_n<4>(R, R.impulse, dv, 0); break;
-        case 5: japply_n<5>(R, R.impulse, dv, 0); break;
-        default: japply_n<6>(R, R.impulse, dv, 0); break;
-    }
-}
-
-// one Gauss-Seidel step of a joint row
-__device__ __forceinline__ void jstep(JointRow& R, float4* dv, bool pseudo) {
-    switch (R.n) {
-        case 1: jstep_n<1>(R, dv, pseudo); break;
-        case 3: jstep_n<3>(R, dv, pseudo); break;
-        case 4: jstep_n<4>(R, dv, pseudo); break;
-        case 5: jstep_n<5>(R, dv, pseudo); break;
-        default: jstep_n<6>(R, dv, pseudo); break;
+    const float diff = __fsub_rn(nw, acc);
+    if (__any_sync(0xffffffffu, lane < L.n && fabsf(diff) > kJZero)) {
+        jl_apply(L, diff, dv, which, lane);
+        if (lane < L.n) (pseudo ? R.pimpulse : R.impulse)[lane] = __fadd_rn(acc, diff);
+    } else {
+        __syncwarp();
     }
 }
 
@@ -144,55 +131,55 @@ __device__ __forceinline__ int holo_loc(const int* table, int n, int row, int co
     return table[row - col + ((2 * n + 1) * col - col * col) / 2];
 }
 
-// multInverseWithVector (HolonomicBlockSolver.cpp:251-317): v <- L^-T D^-1 L^-1 v.
-// `eff` holds `degree` scratch values.
+// multInverseWithVector (HolonomicBlockSolver.cpp:251-317): v <- L^-T D^-1 L^-1 v
+// by one warp, a lane per entry of the blocks of a column (each entry summed in
+// the order of the one-thread form).
 template <class T>
-__device__ void holo_solve(const HoloStore& hs, int s, const JointRow* rows, const T* B, T* v, T* eff) {
+__device__ void holo_solve(const HoloStore& hs, int s, const JointRow* rows, const T* B, T* v, int lane) {
     const int c0 = hs.cstart[s], n = hs.cstart[s + 1] - c0;
     const int* cons = hs.cons + c0;
     const int* vp = hs.vpos + c0;
     const int* table = hs.table + hs.tstart[s];
     const int* ls = hs.lstart + hs.lbase[s];   // column col's blocks below the diagonal
+    const int r8 = lane >> 3, i8 = lane & 7;   // four blocks at a time, eight lanes each
     for (int col = 0; col + 1 < n; col++) {
         const int bw = rows[cons[col]].n;
-        for (int q = ls[col]; q < ls[col + 1]; q++) {
-            const int row = hs.lrow[q], l = hs.lloc[q];
-            const int bh = rows[cons[row]].n;
-            for (int i = 0; i < bh; i++) {
-                T x = 0;
-                for (int k = 0; k < bw; k++) x += B[l + i * bw + k] * v[vp[col] + k];
-                eff[vp[row] + i] = x;
+        for (int q0 = ls[col]; q0 < ls[col + 1]; q0 += 4) {
+            const int q = q0 + r8;
+            if (q < ls[col + 1]) {
+                const int row = hs.lrow[q], l = hs.lloc[q];
+                if (i8 < rows[cons[row]].n) {
+                    T x = 0;
+                    for (int k = 0; k < bw; k++) x += B[l + i8 * bw + k] * v[vp[col] + k];
+                    v[vp[row] + i8] -= x;
+                }
             }
         }
-        // only rows below `col` were written this pass: subtract and clear them
-        for (int q = ls[col]; q < ls[col + 1]; q++) {
-            const int row = hs.lrow[q];
-            for (int i = 0; i < rows[cons[row]].n; i++) { v[vp[row] + i] -= eff[vp[row] + i]; eff[vp[row] + i] = 0; }
-        }
+        __syncwarp();
     }
-    for (int col = 0; col < n; col++) {
+    for (int col = r8; col < n; col += 4) {
         const int w = rows[cons[col]].n, l = holo_loc(table, n, col, col);
-        T tmp[kJMax];
-        for (int i = 0; i < w; i++) {
-            T x = 0;
-            for (int k = 0; k < w; k++) x += B[l + i * w + k] * v[vp[col] + k];
-            tmp[i] = x;
-        }
-        for (int i = 0; i < w; i++) v[vp[col] + i] = tmp[i];
+        T x = 0;
+        if (i8 < w)
+            for (int k = 0; k < w; k++) x += B[l + i8 * w + k] * v[vp[col] + k];
+        __syncwarp(0xffu << (lane & 24));   // the eight lanes of the block
+        if (i8 < w) v[vp[col] + i8] = x;
     }
+    __syncwarp();
     for (int col = n - 2; col >= 0; col--) {
         const int bw = rows[cons[col]].n;
-        T e6[kJMax] = {};
-        for (int q = ls[col]; q < ls[col + 1]; q++) {
-            const int row = hs.lrow[q], l = hs.lloc[q];
-            const int bh = rows[cons[row]].n;
-            for (int i = 0; i < bw; i++) {
+        if (lane < bw) {
+            T e = 0;
+            for (int q = ls[col]; q < ls[col + 1]; q++) {
+                const int row = hs.lrow[q], l = hs.lloc[q];
+                const int bh = rows[cons[row]].n;
                 T dp = 0;
-                for (int j = 0; j < bh; j++) dp += v[vp[row] + j] * B[l + i + bw * j];
-                e6[i] += dp;
+                for (int j = 0; j < bh; j++) dp += v[vp[row] + j] * B[l + lane + bw * j];
+                e += dp;
             }
+            v[vp[col] + lane] -= e;
         }
-        for (int i = 0; i < bw; i++) v[vp[col] + i] -= e6[i];
+        __syncwarp();
     }
 }
 

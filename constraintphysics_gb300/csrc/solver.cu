@@ -897,63 +897,80 @@ __global__ void __launch_bounds__(32) k_pgs_big(Dev d, int dv_cap) {
 }
 
 // HolonomicSystem::computeAndApplyImpulses (HolonomicBlockSolver.cpp:319-378)
-// for system s: solve A d = t - J dv with the factorisation, then (with a
-// threshold) discard a pseudo solution whose angular velocity change exceeds
-// it anywhere, else apply d.  Runs on one thread.
+// for system s by one warp: solve A d = t - J dv with the factorisation, then
+// (with a threshold) discard a pseudo solution whose angular velocity change
+// exceeds it anywhere, else apply d.
 template <class T>
-__device__ void holo_apply(const Dev& d, int s, float4* dv, float4* err, bool pseudo, float thr) {
+__device__ __noinline__ void holo_apply(const Dev& d, int s, float4* dv, float4* err, bool pseudo, float thr, int lane) {
     const HoloStore& hs = d.hs;
-    const int c0 = hs.cstart[s], n = hs.cstart[s + 1] - c0, deg = hs.degree[s];
+    const int c0 = hs.cstart[s], n = hs.cstart[s + 1] - c0;
     const int* cons = hs.cons + c0;
     const int* vp = hs.vpos + c0;
     const T* B = reinterpret_cast<const T*>(hs.fp64[s] ? (const void*)(hs.pool64 + hs.bstart[s])
                                                        : (const void*)(hs.pool32 + hs.bstart[s]));
     T* v = reinterpret_cast<T*>(hs.work + hs.wstart[s]);
-    T* eff = v + deg;
     const int which = pseudo ? 1 : 0;
-    for (int i = 0; i < n; i++) {
+    for (int i = lane; i < n; i += 32) {
         const JointRow& R = d.jt.rows[cons[i]];
         float va[6], vb[6], cur[kJMax];
         jload(dv, R.sa, which, va);
         jload(dv, R.sb, which, vb);
         jvalue(R, va, vb, cur);
         const float* tgt = pseudo ? R.ptarget : R.target;
-        for (int k = 0; k < R.n; k++) { v[vp[i] + k] = (T)tgt[k] - (T)cur[k]; eff[vp[i] + k] = 0; }
+        for (int k = 0; k < R.n; k++) v[vp[i] + k] = (T)tgt[k] - (T)cur[k];
     }
-    holo_solve<T>(hs, s, d.jt.rows, B, v, eff);
-    if (thr > 0.f) {
+    __syncwarp();
+    holo_solve<T>(hs, s, d.jt.rows, B, v, lane);
+    // the solution's change of Δv, constraint by constraint in order (bodies
+    // are shared); the next constraint's row is loaded meanwhile
+    auto apply = [&](float4* to, int wh, bool store) {
+        JointLane L, N;
+        float imp = 0.f, nimp = 0.f;
+        auto load = [&](int i, JointLane& x, float& z) {
+            jl_load(d.jt.rows[cons[i]], lane, x);
+            z = lane < x.n ? (float)v[vp[i] + lane] : 0.f;
+        };
+        load(0, L, imp);
         for (int i = 0; i < n; i++) {
-            const JointRow& R = d.jt.rows[cons[i]];
-            float ic[kJMax];
-            for (int k = 0; k < R.n; k++) ic[k] = (float)v[vp[i] + k];
-            if (!jzero(ic, R.n)) japply(R, ic, err, 0);
+            if (i + 1 < n) load(i + 1, N, nimp);
+            if (__any_sync(0xffffffffu, lane < L.n && fabsf(imp) > kJZero)) {
+                jl_apply(L, imp, to, wh, lane);
+                if (store && lane < L.n) {
+                    JointRow& R = d.jt.rows[cons[i]];
+                    (pseudo ? R.pimpulse : R.holo)[lane] += imp;
+                }
+            }
+            L = N;
+            imp = nimp;
         }
-        for (int i = 0; i < n; i++) {
+        __syncwarp();
+    };
+    if (thr > 0.f) {
+        apply(err, 0, false);
+        bool over = false;
+        for (int i = lane; i < n; i += 32) {
             const JointRow& R = d.jt.rows[cons[i]];
             float ea[6], eb[6];
             jload(err, R.sa, 0, ea);
             jload(err, R.sb, 0, eb);
             float r2 = 0.f;
             for (int k = 3; k < 6; k++) r2 += ea[k] * ea[k] + eb[k] * eb[k];
-            if (r2 > thr * thr) return;
+            over = over || r2 > thr * thr;
         }
+        if (__any_sync(0xffffffffu, over)) return;
     }
-    for (int i = 0; i < n; i++) {
-        JointRow& R = d.jt.rows[cons[i]];
-        float ic[kJMax];
-        for (int k = 0; k < R.n; k++) ic[k] = (float)v[vp[i] + k];
-        if (jzero(ic, R.n)) continue;
-        japply(R, ic, dv, which);
-        float* acc = pseudo ? R.pimpulse : R.holo;
-        for (int k = 0; k < R.n; k++) acc[k] += ic[k];
-    }
+    apply(dv, which, true);
 }
 
-// islands with joint rows: one warp per island, the serial chain on lane 0
-// over contact rows and joint rows in island order, then the island's
-// holonomic systems (first substep); Δv and the linearisation probe in global
-// memory
-__global__ void __launch_bounds__(32) k_pgs_joint(Dev d, int first) {
+// Islands with joint rows: one warp per island, contact rows and joint rows in
+// island order, then the island's holonomic systems (first substep).  A joint
+// row is spread over the lanes (joints.cuh), a contact row runs on lane 0;
+// Δv in shared memory for islands of up to kJointDv bodies.  Bound by
+// the chain of row-steps: on 512 chains of 16-64 links one lane and Δv in
+// global memory took 568 us a substep.
+constexpr int kJointDv = 128;
+__global__ void __launch_bounds__(32, 4) k_pgs_joint(Dev d, int first) {
+    __shared__ float4 sdv[kDvF4 * kJointDv];
     const int lane = threadIdx.x;
     const int nj = d.sched[3];
     for (int q = blockIdx.x; q < nj; q += gridDim.x) {
@@ -961,53 +978,69 @@ __global__ void __launch_bounds__(32) k_pgs_joint(Dev d, int first) {
         const int rs = d.g_isl_row_start[i], rc = d.g_isl_row_count[i];
         const int bs = d.g_isl_body_start[i], bc = d.g_isl_body_count[i];
         const WorldParams& P = d.wparams[d.g_isl_world[i]];
-        float4* dv = d.dv + kDvF4 * (size_t)bs;
+        float4* dv = bc <= kJointDv ? sdv : d.dv + kDvF4 * (size_t)bs;
         float4* err = d.dv_err + kDvF4 * (size_t)bs;
         for (int k = lane; k < kDvF4 * bc; k += 32) { dv[k] = make_float4(0.f, 0.f, 0.f, 0.f); err[k] = dv[k]; }
         __syncwarp();
-        if (lane == 0) {
+        // one pass over the rows: joint(lane row, joint row) or contact(row)
+        // for each, the next joint row loaded one row ahead
+        auto pass = [&](auto&& joint, auto&& contact) {
+            JointLane L, N;
+            int c = d.rows[rs].contact, nc = 0;
+            if (c < 0) jl_load(d.jt.rows[-c - 1], lane, L);
+            int c2 = rc > 1 ? d.rows[rs + 1].contact : 0;
             for (int r = rs; r < rs + rc; r++) {
-                const int c = d.rows[r].contact;
-                if (c >= 0) row_warm(d.rows[r], d.rows[r].imp, dv);
-                else jwarm(d.jt.rows[-c - 1], dv);
+                nc = c2;
+                if (r + 1 < rs + rc && nc < 0) jl_load(d.jt.rows[-nc - 1], lane, N);
+                if (r + 2 < rs + rc) c2 = d.rows[r + 2].contact;
+                if (c < 0) joint(L, d.jt.rows[-c - 1]);
+                else contact(d.rows[r]);
+                c = nc;
+                L = N;
             }
-            const int n_vel = P.pgs_vel, n_pos = P.pgs_pos;   // read once: the row stores could alias P
-            for (int it = 0; it < n_vel; it++)
-                for (int r = rs; r < rs + rc; r++) {
-                    RowBlock& R = d.rows[r];
-                    if (R.contact < 0) { jstep(d.jt.rows[-R.contact - 1], dv, false); continue; }
-                    float4 imp = R.imp;
-                    int st = R.stat;
-                    row_vel(R, imp, st, dv);
-                    R.imp = imp;
-                    R.stat = st;
-                }
-            for (int it = 0; it < n_pos; it++)
-                for (int r = rs; r < rs + rc; r++) {
-                    RowBlock& R = d.rows[r];
-                    if (R.contact < 0) {
-                        JointRow& Jr = d.jt.rows[-R.contact - 1];
-                        if (Jr.pos) jstep(Jr, dv, true);   // needsPosCorrect
-                        continue;
+            __syncwarp();
+        };
+        const int n_vel = P.pgs_vel, n_pos = P.pgs_pos;   // read once: the row stores could alias P
+        pass([&](const JointLane& L, JointRow&) { jl_warm(L, dv, lane); },
+             [&](RowBlock& R) {
+                 if (lane == 0) row_warm(R, R.imp, dv);
+                 __syncwarp();
+             });
+        for (int it = 0; it < n_vel; it++)
+            pass([&](const JointLane& L, JointRow& R) { jl_step(L, R, dv, false, lane); },
+                 [&](RowBlock& R) {
+                     if (lane == 0) {
+                         float4 imp = R.imp;
+                         int st = R.stat;
+                         row_vel(R, imp, st, dv);
+                         R.imp = imp;
+                         R.stat = st;
+                     }
+                     __syncwarp();
+                 });
+        for (int it = 0; it < n_pos; it++)
+            pass([&](const JointLane& L, JointRow& R) { if (L.pos) jl_step(L, R, dv, true, lane); },   // needsPosCorrect
+                 [&](RowBlock& R) {
+                     if (lane == 0) {
+                         float4 imp = R.imp;
+                         row_pos(R, imp, dv);
+                         R.imp = imp;
+                     }
+                     __syncwarp();
+                 });
+        if (first && P.pgs_holo > 0) {
+            const int ss = d.g_isl_sys_start[i], sn = d.g_isl_sys_count[i];
+            for (int it = 0; it < P.pgs_holo; it++)
+                for (int k = 0; k < sn; k++) {
+                    const int s = d.isl_sys[ss + k];
+                    if (d.hs.fp64[s]) {
+                        holo_apply<double>(d, s, dv, err, false, -1.f, lane);
+                        holo_apply<double>(d, s, dv, err, true, d.lin_err_threshold, lane);
+                    } else {
+                        holo_apply<float>(d, s, dv, err, false, -1.f, lane);
+                        holo_apply<float>(d, s, dv, err, true, d.lin_err_threshold, lane);
                     }
-                    float4 imp = R.imp;
-                    row_pos(R, imp, dv);
-                    R.imp = imp;
                 }
-            if (first && P.pgs_holo > 0) {
-                const int ss = d.g_isl_sys_start[i], sn = d.g_isl_sys_count[i];
-                for (int it = 0; it < P.pgs_holo; it++)
-                    for (int k = 0; k < sn; k++) {
-                        const int s = d.isl_sys[ss + k];
-                        if (d.hs.fp64[s]) {
-                            holo_apply<double>(d, s, dv, err, false, -1.f);
-                            holo_apply<double>(d, s, dv, err, true, d.lin_err_threshold);
-                        } else {
-                            holo_apply<float>(d, s, dv, err, false, -1.f);
-                            holo_apply<float>(d, s, dv, err, true, d.lin_err_threshold);
-                        }
-                    }
-            }
         }
         __syncwarp();
         for (int r = rs + lane; r < rs + rc; r += 32) {
