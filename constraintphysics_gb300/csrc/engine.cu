@@ -1180,7 +1180,7 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
     std::vector<float4> j_power;
     std::vector<uint64_t> je_key;
     std::vector<int> je_jstart, je_jcount, je_jlist, je_sys, je_wstart{0}, je_wjstart{0}, hs_wstart{0};
-    std::vector<int> hs_cstart{0}, hs_cons, hs_vpos, hs_degree, hs_tstart{0}, hs_table, hs_bstart, hs_cap, hs_fp64, hs_wk;
+    std::vector<int> hs_cstart{0}, hs_cons, hs_vpos, hs_dim, hs_degree, hs_tstart{0}, hs_table, hs_bstart, hs_cap, hs_fp64, hs_wk;
     std::vector<int> hs_lbase, hs_lstart, hs_lrow, hs_lloc;   // per-column lists of the nonzero blocks below the diagonal
     std::vector<int> sp_b1, sp_b2, sp_wstart{0};
     std::vector<float4> sp_p1, sp_p2, sp_par;
@@ -1257,7 +1257,7 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
                 }
             }
             for (const HSystem& H : G.systems) {
-                for (int j : H.cons) hs_cons.push_back(jbase + j);
+                for (int j : H.cons) { hs_cons.push_back(jbase + j); hs_dim.push_back(j_n[jbase + j]); }
                 hs_vpos.insert(hs_vpos.end(), H.vpos.begin(), H.vpos.end());
                 hs_cstart.push_back((int)hs_cons.size());
                 hs_degree.push_back(H.degree);
@@ -1282,7 +1282,7 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
                 if (H.fp64) { hs_bstart.push_back((int)pool64_n); pool64_n += need; }
                 else { hs_bstart.push_back((int)pool32_n); pool32_n += (need + 3) & ~size_t(3); }
                 hs_wk.push_back((int)work_n);
-                work_n += 2 * (size_t)H.degree;
+                work_n += (size_t)H.degree + 8;   // the solve reads up to five entries past a block
             }
         }
         je_wstart.push_back((int)je_key.size());
@@ -1459,6 +1459,7 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
             HoloStore& H = x.hs;
             H.n = n_sys;
             H.cstart = A.take<int>(n_sys + 1); H.cons = A.take<int>(hs_cons.size()); H.vpos = A.take<int>(hs_vpos.size());
+            H.dim = A.take<int>(hs_dim.size());
             H.degree = A.take<int>(n_sys); H.tstart = A.take<int>(n_sys + 1); H.table = A.take<int>(hs_table.size());
             H.lbase = A.take<int>(n_sys); H.lstart = A.take<int>(hs_lstart.size());
             H.lrow = A.take<int>(hs_lrow.size()); H.lloc = A.take<int>(hs_lloc.size());
@@ -1546,6 +1547,7 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
         up((void*)E.world_jstart, je_wjstart.data(), je_wjstart.size() * 4);
         const HoloStore& H = x.hs;
         up((void*)H.cstart, hs_cstart.data(), hs_cstart.size() * 4); up((void*)H.cons, hs_cons.data(), hs_cons.size() * 4);
+        up((void*)H.dim, hs_dim.data(), hs_dim.size() * 4);
         up((void*)H.vpos, hs_vpos.data(), hs_vpos.size() * 4); up((void*)H.degree, hs_degree.data(), hs_degree.size() * 4);
         up((void*)H.tstart, hs_tstart.data(), hs_tstart.size() * 4); up((void*)H.table, hs_table.data(), hs_table.size() * 4);
         up((void*)H.lbase, hs_lbase.data(), hs_lbase.size() * 4); up((void*)H.lstart, hs_lstart.data(), hs_lstart.size() * 4);

@@ -57,25 +57,24 @@ __device__ __forceinline__ void jl_load(const JointRow& R, int lane, JointLane& 
     L.ptarget = R.ptarget[i];
     L.acc = R.impulse[i];
     L.pacc = R.pimpulse[i];
-}
-// Δv of a body for `which`, zeros for infinite mass
-__device__ __forceinline__ void jl_dv(const float4* dv, int slot, int which, float* o) {
-    if (slot < 0) {
 #pragma unroll
-        for (int k = 0; k < 6; k++) o[k] = 0.f;
-        return;
+    for (int k = 0; k < 6; k++) {
+        L.minv[k] = k < L.n ? L.minv[k] : 0.f;
+        L.it[k] = k < L.n ? L.it[k] : 0.f;
     }
-    jl_row6(reinterpret_cast<const float*>(dv + kDvF4 * slot) + 6 * which, o);
+}
+// Δv of a body for `which`; `zero` (six floats) for infinite mass
+__device__ __forceinline__ void jl_dv(const float4* dv, const float* zero, int slot, int which, float* o) {
+    jl_row6(slot < 0 ? zero : reinterpret_cast<const float*>(dv + kDvF4 * slot) + 6 * which, o);
 }
 // component lane: sum of imp_i M^-1 J^T added to its component of Δv, where
-// lane i holds imp_i (zero beyond the row's dofs)
+// lane i holds imp_i (finite beyond the row's dofs)
 __device__ __forceinline__ void jl_apply(const JointLane& L, float imp, float4* dv, int which, int lane) {
     const int slot = lane < 6 ? L.sa : L.sb;
     float x = 0.f;
 #pragma unroll
     for (int i = 0; i < 6; i++) {
-        const float v = __shfl_sync(0xffffffffu, imp, i);
-        if (i < L.n) x = __fmaf_rn(v, L.it[i], x);
+        x = __fmaf_rn(__shfl_sync(0xffffffffu, imp, i), L.it[i], x);
     }
     if (lane < 12 && slot >= 0) {
         float* f = reinterpret_cast<float*>(dv + kDvF4 * slot) + 6 * which + (lane < 6 ? lane : lane - 6);
@@ -85,41 +84,40 @@ __device__ __forceinline__ void jl_apply(const JointLane& L, float imp, float4* 
 }
 // warm start (DegreedConstraint::applyWarmStartVelocityChange)
 __device__ __forceinline__ void jl_warm(const JointLane& L, float4* dv, int lane) {
-    if (__any_sync(0xffffffffu, lane < L.n && fabsf(L.acc) > kJZero)) jl_apply(L, L.acc, dv, 0, lane);
+    if (__any_sync(0xffffffffu, lane < L.n && fabsf(L.acc) > kJZero)) jl_apply(L, lane < L.n ? L.acc : 0.f, dv, 0, lane);
 }
 // PGSConstraintStep<n> (ConstraintSolver.cpp:12-40): the accumulated impulse
 // plus the row's correction, projected (ConeLimitConstraint /
 // TwistLimitConstraint::projectValidImpulse, ConstraintSolver.cpp:434-436,
 // 463-465: one-sided limits; MotorConstraint / PistonConstraint, :591-606,
 // 728-731), applied when the change is not zero
-__device__ __forceinline__ void jl_step(const JointLane& L, JointRow& R, float4* dv, bool pseudo, int lane) {
+__device__ __forceinline__ void jl_step(const JointLane& L, JointRow& R, float4* dv, const float* zero, bool pseudo, int lane) {
     const int which = pseudo ? 1 : 0;
     float va[6], vb[6];
-    jl_dv(dv, L.sa, which, va);
-    jl_dv(dv, L.sb, which, vb);
+    jl_dv(dv, zero, L.sa, which, va);
+    jl_dv(dv, zero, L.sb, which, vb);
     float x = 0.f, y = 0.f;
 #pragma unroll
     for (int k = 0; k < 6; k++) {
         x = __fmaf_rn(va[k], L.ja[k], x);
         y = __fmaf_rn(vb[k], L.jb[k], y);
     }
-    const float delta = __fsub_rn(pseudo ? L.ptarget : L.target, __fadd_rn(x, y));
+    const float delta = lane < L.n ? __fsub_rn(pseudo ? L.ptarget : L.target, __fadd_rn(x, y)) : 0.f;
     const float acc = pseudo ? L.pacc : L.acc;
     float s = 0.f;
 #pragma unroll
     for (int k = 0; k < 6; k++) {
-        const float v = __shfl_sync(0xffffffffu, delta, k);
-        if (k < L.n) s = __fmaf_rn(v, L.minv[k], s);
+        s = __fmaf_rn(__shfl_sync(0xffffffffu, delta, k), L.minv[k], s);
     }
     float nw = __fadd_rn(acc, s);
-    if (L.n == 1 && L.proj != 0) {
+    if (L.proj != 0) {   // rows of one dof
         if (L.proj == 1) nw = fmaxf(nw, 0.f);
         else if (L.proj == 2) nw = fminf(nw, 0.f);
         else nw = nw > 0.f ? fminf(nw, L.lim) : fmaxf(nw, -L.lim);
     }
     const float diff = __fsub_rn(nw, acc);
     if (__any_sync(0xffffffffu, lane < L.n && fabsf(diff) > kJZero)) {
-        jl_apply(L, diff, dv, which, lane);
+        jl_apply(L, lane < L.n ? diff : 0.f, dv, which, lane);
         if (lane < L.n) (pseudo ? R.pimpulse : R.impulse)[lane] = __fadd_rn(acc, diff);
     } else {
         __syncwarp();
@@ -131,55 +129,105 @@ __device__ __forceinline__ int holo_loc(const int* table, int n, int row, int co
     return table[row - col + ((2 * n + 1) * col - col * col) / 2];
 }
 
+// The tables of one system as the solve reads them: in shared memory when the
+// system is small enough (each column's solve is a chain of dependent loads),
+// else where the host put them.
+struct HoloView {
+    int n;
+    const int *cons, *vpos, *ls, *lrow, *lloc;   // ls: column col's blocks below the diagonal, [ls[col], ls[col + 1]) - ls0
+    const int* dim;                              // dofs per constraint
+    int ls0;
+};
+__device__ __forceinline__ double jfma(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float jfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+
 // multInverseWithVector (HolonomicBlockSolver.cpp:251-317): v <- L^-T D^-1 L^-1 v
 // by one warp, a lane per entry of the blocks of a column (each entry summed in
-// the order of the one-thread form).
+// the order of the one-thread form); the next column's first blocks are loaded
+// while this one is solved.
 template <class T>
-__device__ void holo_solve(const HoloStore& hs, int s, const JointRow* rows, const T* B, T* v, int lane) {
-    const int c0 = hs.cstart[s], n = hs.cstart[s + 1] - c0;
-    const int* cons = hs.cons + c0;
-    const int* vp = hs.vpos + c0;
-    const int* table = hs.table + hs.tstart[s];
-    const int* ls = hs.lstart + hs.lbase[s];   // column col's blocks below the diagonal
+__device__ __forceinline__ void holo_solve(const HoloView& h, const int* table, const T* B, T* v, int lane) {
+    const int n = h.n;
     const int r8 = lane >> 3, i8 = lane & 7;   // four blocks at a time, eight lanes each
+    T b[kJMax], nb[kJMax];
+    int row = 0, nrow = 0;
+    bool act = false, nact = false;
+    auto lower = [&](int col, int q, T* o, int* r) {   // block q's row i8
+        bool a = q < h.ls[col + 1] - h.ls0;
+        *r = a ? h.lrow[q] : 0;
+        a = a && i8 < h.dim[*r];
+        const int bw = h.dim[col], l = a ? h.lloc[q] : 0;
+#pragma unroll
+        for (int k = 0; k < kJMax; k++) o[k] = a && k < bw ? B[l + i8 * bw + k] : (T)0;
+        return a;
+    };
+    if (n > 1) act = lower(0, h.ls[0] - h.ls0 + r8, b, &row);
     for (int col = 0; col + 1 < n; col++) {
-        const int bw = rows[cons[col]].n;
-        for (int q0 = ls[col]; q0 < ls[col + 1]; q0 += 4) {
-            const int q = q0 + r8;
-            if (q < ls[col + 1]) {
-                const int row = hs.lrow[q], l = hs.lloc[q];
-                if (i8 < rows[cons[row]].n) {
-                    T x = 0;
-                    for (int k = 0; k < bw; k++) x += B[l + i8 * bw + k] * v[vp[col] + k];
-                    v[vp[row] + i8] -= x;
-                }
+        const int bw = h.dim[col];
+        const T* vc = v + h.vpos[col];
+        if (col + 2 < n) nact = lower(col + 1, h.ls[col + 1] - h.ls0 + r8, nb, &nrow);
+        T x = 0;
+#pragma unroll
+        for (int k = 0; k < kJMax; k++) x = k < bw ? jfma(b[k], vc[k], x) : x;
+        if (act) v[h.vpos[row] + i8] -= x;
+        for (int q0 = h.ls[col] - h.ls0 + 4; q0 < h.ls[col + 1] - h.ls0; q0 += 4) {   // more than four blocks
+            T c[kJMax];
+            int r;
+            if (lower(col, q0 + r8, c, &r)) {
+                T y = 0;
+                for (int k = 0; k < bw; k++) y = jfma(c[k], vc[k], y);
+                v[h.vpos[r] + i8] -= y;
             }
         }
         __syncwarp();
+        act = nact;
+        row = nrow;
+#pragma unroll
+        for (int k = 0; k < kJMax; k++) b[k] = nb[k];
     }
     for (int col = r8; col < n; col += 4) {
-        const int w = rows[cons[col]].n, l = holo_loc(table, n, col, col);
+        const int w = h.dim[col], l = holo_loc(table, n, col, col);
         T x = 0;
         if (i8 < w)
-            for (int k = 0; k < w; k++) x += B[l + i8 * w + k] * v[vp[col] + k];
+            for (int k = 0; k < w; k++) x = jfma(B[l + i8 * w + k], v[h.vpos[col] + k], x);
         __syncwarp(0xffu << (lane & 24));   // the eight lanes of the block
-        if (i8 < w) v[vp[col] + i8] = x;
+        if (i8 < w) v[h.vpos[col] + i8] = x;
     }
     __syncwarp();
+    auto upper = [&](int col, int q, T* o, int* r) {   // block q's column `lane`
+        const bool a = q < h.ls[col + 1] - h.ls0;
+        *r = a ? h.lrow[q] : 0;
+        const int bw = h.dim[col], bh = a ? h.dim[*r] : 0, l = a ? h.lloc[q] : 0;
+#pragma unroll
+        for (int j = 0; j < kJMax; j++) o[j] = lane < bw && j < bh ? B[l + lane + bw * j] : (T)0;
+        return bh;
+    };
+    int bh = 0, nbh = 0;
+    if (n > 1) bh = upper(n - 2, h.ls[n - 2] - h.ls0, b, &row);
     for (int col = n - 2; col >= 0; col--) {
-        const int bw = rows[cons[col]].n;
+        const int bw = h.dim[col];
+        if (col > 0) nbh = upper(col - 1, h.ls[col - 1] - h.ls0, nb, &nrow);
         if (lane < bw) {
             T e = 0;
-            for (int q = ls[col]; q < ls[col + 1]; q++) {
-                const int row = hs.lrow[q], l = hs.lloc[q];
-                const int bh = rows[cons[row]].n;
-                T dp = 0;
-                for (int j = 0; j < bh; j++) dp += v[vp[row] + j] * B[l + lane + bw * j];
-                e += dp;
+            T dp = 0;
+            const T* vr = v + h.vpos[row];
+#pragma unroll
+            for (int j = 0; j < kJMax; j++) dp = j < bh ? jfma(vr[j], b[j], dp) : dp;
+            if (h.ls[col] < h.ls[col + 1]) e += dp;
+            for (int q = h.ls[col] - h.ls0 + 1; q < h.ls[col + 1] - h.ls0; q++) {
+                const int r = h.lrow[q], l = h.lloc[q];
+                const int rh = h.dim[r];
+                T y = 0;
+                for (int j = 0; j < rh; j++) y = jfma(v[h.vpos[r] + j], B[l + lane + bw * j], y);
+                e += y;
             }
-            v[vp[col] + lane] -= e;
+            v[h.vpos[col] + lane] -= e;
         }
         __syncwarp();
+        bh = nbh;
+        row = nrow;
+#pragma unroll
+        for (int j = 0; j < kJMax; j++) b[j] = nb[j];
     }
 }
 

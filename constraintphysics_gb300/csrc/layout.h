@@ -197,7 +197,7 @@ constexpr int kJMax = 6;
 struct alignas(16) JointRow {
     float ja[kJMax * 6], jb[kJMax * 6];     // [n][6]
     float ita[6 * kJMax], itb[6 * kJMax];   // [6][n]
-    float itv[kJMax * kJMax], minv[kJMax * kJMax];
+    float minv[kJMax * kJMax];
     float target[kJMax], ptarget[kJMax];
     float impulse[kJMax], pimpulse[kJMax], holo[kJMax];
     int n, sa, sb;                          // island body slots (-1: infinite mass)
@@ -207,7 +207,10 @@ struct alignas(16) JointRow {
     float vt;                               // motor / piston: target = vt - value
     int has_vt;
     int pos;                                // needsPosCorrect: solved in the position passes
+    float itv[kJMax * kJMax];               // J M^-1 J^T (the solver passes read only what comes before)
 };
+constexpr int kJointStage = 880;            // bytes of a row the solver passes use, up to a multiple of 16
+static_assert(offsetof(JointRow, itv) <= kJointStage && kJointStage <= (int)sizeof(JointRow), "staged part of a joint row");
 
 // Joint kinds (PersistentConstraint.h:90-420).  The limits are inequality
 // rows outside the holonomic systems, listed in an island only while active.
@@ -287,6 +290,7 @@ struct HoloStore {
     const int* cstart;      // [n + 1] into cons / vpos
     const int* cons;        // joint indices in elimination order
     const int* vpos;        // vector offset of each constraint
+    const int* dim;         // dofs of each constraint
     const int* degree;
     const int* tstart;      // [n + 1] into table
     const int* table;       // block_location_table (-1 empty)
@@ -297,7 +301,7 @@ struct HoloStore {
     const int* bstart;      // offset into the FP32 or FP64 pool
     const int* cap;         // block storage (the diagonal scratch follows)
     const int* fp64;
-    const int* wstart;      // offset into the solve workspace (degree doubles)
+    const int* wstart;      // offset into the solve workspace (degree + 8 doubles)
     float* pool32;
     double* pool64;
     double* work;

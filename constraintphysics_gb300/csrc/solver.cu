@@ -899,44 +899,42 @@ __global__ void __launch_bounds__(32) k_pgs_big(Dev d, int dv_cap) {
 // HolonomicSystem::computeAndApplyImpulses (HolonomicBlockSolver.cpp:319-378)
 // for system s by one warp: solve A d = t - J dv with the factorisation, then
 // (with a threshold) discard a pseudo solution whose angular velocity change
-// exceeds it anywhere, else apply d.
-template <class T>
-__device__ __noinline__ void holo_apply(const Dev& d, int s, float4* dv, float4* err, bool pseudo, float thr, int lane) {
+// exceeds it anywhere, else apply d.  `v`: the solve's vector; row(i): the
+// staged part of constraint i's row.
+template <class T, class Row>
+__device__ __forceinline__ void holo_apply(const Dev& d, int s, const HoloView& h, T* v, const Row& row_of, float4* dv, float4* err,
+                                           bool pseudo, float thr, int lane) {
     const HoloStore& hs = d.hs;
-    const int c0 = hs.cstart[s], n = hs.cstart[s + 1] - c0;
-    const int* cons = hs.cons + c0;
-    const int* vp = hs.vpos + c0;
     const T* B = reinterpret_cast<const T*>(hs.fp64[s] ? (const void*)(hs.pool64 + hs.bstart[s])
                                                        : (const void*)(hs.pool32 + hs.bstart[s]));
-    T* v = reinterpret_cast<T*>(hs.work + hs.wstart[s]);
-    const int which = pseudo ? 1 : 0;
+    const int which = pseudo ? 1 : 0, n = h.n;
     for (int i = lane; i < n; i += 32) {
-        const JointRow& R = d.jt.rows[cons[i]];
+        const JointRow& R = *row_of(i);
         float va[6], vb[6], cur[kJMax];
         jload(dv, R.sa, which, va);
         jload(dv, R.sb, which, vb);
         jvalue(R, va, vb, cur);
         const float* tgt = pseudo ? R.ptarget : R.target;
-        for (int k = 0; k < R.n; k++) v[vp[i] + k] = (T)tgt[k] - (T)cur[k];
+        for (int k = 0; k < R.n; k++) v[h.vpos[i] + k] = (T)tgt[k] - (T)cur[k];
     }
     __syncwarp();
-    holo_solve<T>(hs, s, d.jt.rows, B, v, lane);
+    holo_solve<T>(h, hs.table + hs.tstart[s], B, v, lane);
     // the solution's change of Δv, constraint by constraint in order (bodies
     // are shared); the next constraint's row is loaded meanwhile
     auto apply = [&](float4* to, int wh, bool store) {
         JointLane L, N;
         float imp = 0.f, nimp = 0.f;
         auto load = [&](int i, JointLane& x, float& z) {
-            jl_load(d.jt.rows[cons[i]], lane, x);
-            z = lane < x.n ? (float)v[vp[i] + lane] : 0.f;
+            jl_load(*row_of(i), lane, x);
+            z = lane < x.n ? (float)v[h.vpos[i] + lane] : 0.f;
         };
         load(0, L, imp);
         for (int i = 0; i < n; i++) {
             if (i + 1 < n) load(i + 1, N, nimp);
-            if (__any_sync(0xffffffffu, lane < L.n && fabsf(imp) > kJZero)) {
+            if (__any_sync(0xffffffffu, fabsf(imp) > kJZero)) {
                 jl_apply(L, imp, to, wh, lane);
                 if (store && lane < L.n) {
-                    JointRow& R = d.jt.rows[cons[i]];
+                    JointRow& R = d.jt.rows[h.cons[i]];
                     (pseudo ? R.pimpulse : R.holo)[lane] += imp;
                 }
             }
@@ -949,7 +947,7 @@ __device__ __noinline__ void holo_apply(const Dev& d, int s, float4* dv, float4*
         apply(err, 0, false);
         bool over = false;
         for (int i = lane; i < n; i += 32) {
-            const JointRow& R = d.jt.rows[cons[i]];
+            const JointRow& R = *row_of(i);
             float ea[6], eb[6];
             jload(err, R.sa, 0, ea);
             jload(err, R.sb, 0, eb);
@@ -962,41 +960,156 @@ __device__ __noinline__ void holo_apply(const Dev& d, int s, float4* dv, float4*
     apply(dv, which, true);
 }
 
+// a system's tables in shared memory: up to kHoloN constraints, kHoloL blocks
+// below the diagonal
+constexpr int kHoloN = 64, kHoloL = 96;
+struct HoloSm {
+    double v[kHoloN * kJMax + kJMax];
+    int cons[kHoloN], vpos[kHoloN], dim[kHoloN], ls[kHoloN + 1], lrow[kHoloL], lloc[kHoloL];
+    JointRow* rows[kHoloN];
+};
+// both solves of system s; res: find(j) gives joint j's row in shared memory or null
+template <class T, class Find>
+__device__ __noinline__ void holo_system(const Dev& d, int s, HoloSm& sm, bool res, const Find find, float4* dv, float4* err, int lane) {
+    const HoloStore& hs = d.hs;
+    const int c0 = hs.cstart[s], n = hs.cstart[s + 1] - c0;
+    const int* ls = hs.lstart + hs.lbase[s];
+    const int l0 = ls[0], nl = ls[n] - l0;
+    T* work = reinterpret_cast<T*>(hs.work + hs.wstart[s]);
+    if (n <= kHoloN && nl <= kHoloL) {
+        for (int i = lane; i < n; i += 32) {
+            const int j = hs.cons[c0 + i];
+            sm.cons[i] = j;
+            sm.vpos[i] = hs.vpos[c0 + i];
+            sm.dim[i] = d.jt.rows[j].n;
+            JointRow* r = res ? find(j) : nullptr;
+            sm.rows[i] = r ? r : d.jt.rows + j;
+        }
+        for (int i = lane; i <= n; i += 32) sm.ls[i] = ls[i];
+        for (int i = lane; i < nl; i += 32) { sm.lrow[i] = hs.lrow[l0 + i]; sm.lloc[i] = hs.lloc[l0 + i]; }
+        __syncwarp();
+        const HoloView h{n, sm.cons, sm.vpos, sm.ls, sm.lrow, sm.lloc, sm.dim, l0};
+        auto row = [&](int i) { return sm.rows[i]; };
+        for (int p = 0; p < 2; p++)
+            holo_apply<T>(d, s, h, reinterpret_cast<T*>(sm.v), row, dv, err, p == 1, p == 1 ? d.lin_err_threshold : -1.f, lane);
+        __syncwarp();
+    } else {
+        const HoloView h{n, hs.cons + c0, hs.vpos + c0, ls, hs.lrow, hs.lloc, hs.dim + c0, 0};
+        auto row = [&](int i) { return d.jt.rows + h.cons[i]; };
+        for (int p = 0; p < 2; p++)
+            holo_apply<T>(d, s, h, work, row, dv, err, p == 1, p == 1 ? d.lin_err_threshold : -1.f, lane);
+    }
+}
+
 // Islands with joint rows: one warp per island, contact rows and joint rows in
 // island order, then the island's holonomic systems (first substep).  A joint
-// row is spread over the lanes (joints.cuh), a contact row runs on lane 0;
-// Δv in shared memory for islands of up to kJointDv bodies.  Bound by
-// the chain of row-steps: on 512 chains of 16-64 links one lane and Δv in
-// global memory took 568 us a substep.
-constexpr int kJointDv = 128;
-__global__ void __launch_bounds__(32, 4) k_pgs_joint(Dev d, int first) {
-    __shared__ float4 sdv[kDvF4 * kJointDv];
+// row is spread over the lanes (joints.cuh), a contact row runs on lane 0.
+// Bound by the chain of row-steps, each a few dependent loads: the joint rows
+// (up to kJointRes of an island of up to kJointList rows) and the Δv of islands
+// of up to kJointDv bodies are held in shared memory.  On 512 chains of 16-64
+// links: one lane and everything in global memory 568 us a substep, the rows
+// in global memory 263, in shared memory 219 (the first, with the solve, 1,880
+// -> 594).
+constexpr int kJointDv = 68, kJointRes = 64, kJointList = 128;
+// sched[kJointNext]: the next joint-list entry
+constexpr int kJointNext = kBigNext + 2;
+constexpr int kJointFixed = 64 + kJointList * 6 + (int)sizeof(HoloSm);   // barrier, zero entry, row list, joint list, solve
+constexpr int kJointSmem = ((kJointFixed + 15) & ~15) + kDvF4 * kJointDv * 16 + kJointRes * kJointStage;
+__global__ void __launch_bounds__(32, 3) k_pgs_joint(Dev d, int first) {
+    extern __shared__ __align__(16) uint8_t sm[];
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sm);
+    float* zero = reinterpret_cast<float*>(sm + 32);       // Δv of a body of infinite mass
+    int* held_j = reinterpret_cast<int*>(sm + 64);         // resident island: the joint in each slot
+    int16_t* list = reinterpret_cast<int16_t*>(sm + 64 + kJointList * 4);   // the row's joint slot, -1 a contact row
+    HoloSm& hsm = *reinterpret_cast<HoloSm*>(sm + 64 + kJointList * 6);
+    float4* sdv = reinterpret_cast<float4*>(sm + ((kJointFixed + 15) & ~15));
+    uint8_t* srows = reinterpret_cast<uint8_t*>(sdv + kDvF4 * kJointDv);
     const int lane = threadIdx.x;
     const int nj = d.sched[3];
-    for (int q = blockIdx.x; q < nj; q += gridDim.x) {
+    uint32_t parity = 0;
+    if (lane == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(bar)), "r"(1) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (lane < 8) zero[lane] = 0.f;
+    __syncwarp();
+    while (true) {
+        int q = 0;
+        if (lane == 0) q = atomicAdd(&d.sched[kJointNext], 1);
+        q = __shfl_sync(0xffffffffu, q, 0);
+        if (q >= nj) break;
         const int i = d.joint_list[q];
         const int rs = d.g_isl_row_start[i], rc = d.g_isl_row_count[i];
         const int bs = d.g_isl_body_start[i], bc = d.g_isl_body_count[i];
         const WorldParams& P = d.wparams[d.g_isl_world[i]];
         float4* dv = bc <= kJointDv ? sdv : d.dv + kDvF4 * (size_t)bs;
         float4* err = d.dv_err + kDvF4 * (size_t)bs;
+        // the island's joint rows into shared memory, if they fit
+        int held = 0;
+        bool res = rc <= kJointList;
+        for (int base = 0; res && base < rc; base += 32) {
+            const bool in = base + lane < rc;
+            const int c = in ? d.rows[rs + base + lane].contact : 0;
+            const unsigned m = __ballot_sync(0xffffffffu, c < 0);
+            const int slot = held + __popc(m & ((1u << lane) - 1u));
+            if (in) {
+                list[base + lane] = c < 0 ? (int16_t)slot : (int16_t)-1;
+                if (c < 0 && slot < kJointList) held_j[slot] = -c - 1;
+            }
+            held += __popc(m);
+            res = held <= kJointRes;
+        }
+        if (res && held > 0) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the last island's rows were written in place
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(saddr(bar)), "r"((uint32_t)(held * kJointStage))
+                             : "memory");
+            __syncwarp();
+            for (int r = lane; r < rc; r += 32)
+                if (list[r] >= 0)
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                     saddr(srows + list[r] * kJointStage)),
+                                 "l"(d.jt.rows + (-d.rows[rs + r].contact - 1)), "r"((uint32_t)kJointStage), "r"(saddr(bar))
+                                 : "memory");
+        }
         for (int k = lane; k < kDvF4 * bc; k += 32) { dv[k] = make_float4(0.f, 0.f, 0.f, 0.f); err[k] = dv[k]; }
         __syncwarp();
+        if (res && held > 0) {
+            const bool ok = ring_wait(bar, parity, d.wait_limit);
+            parity ^= 1u;
+            if (!__all_sync(0xffffffffu, ok)) {
+                ring_wait(bar, parity ^ 1u, kDefaultWaitLimit);   // let the copies in flight land (bounded)
+                if (lane == 0) atomicOr(d.status, ST_TIMEOUT);
+                return;
+            }
+        }
+        // the island's row r: its joint row, or null for a contact row
+        auto joint_of = [&](int r) -> JointRow* {
+            if (res) return list[r] < 0 ? nullptr : reinterpret_cast<JointRow*>(srows + list[r] * kJointStage);
+            const int c = d.rows[rs + r].contact;
+            return c < 0 ? d.jt.rows + (-c - 1) : nullptr;
+        };
         // one pass over the rows: joint(lane row, joint row) or contact(row)
         // for each, the next joint row loaded one row ahead
         auto pass = [&](auto&& joint, auto&& contact) {
-            JointLane L, N;
-            int c = d.rows[rs].contact, nc = 0;
-            if (c < 0) jl_load(d.jt.rows[-c - 1], lane, L);
-            int c2 = rc > 1 ? d.rows[rs + 1].contact : 0;
-            for (int r = rs; r < rs + rc; r++) {
-                nc = c2;
-                if (r + 1 < rs + rc && nc < 0) jl_load(d.jt.rows[-nc - 1], lane, N);
-                if (r + 2 < rs + rc) c2 = d.rows[r + 2].contact;
-                if (c < 0) joint(L, d.jt.rows[-c - 1]);
-                else contact(d.rows[r]);
-                c = nc;
-                L = N;
+            JointRow* any = res ? reinterpret_cast<JointRow*>(srows) : d.jt.rows;   // loaded in the place of a contact row
+            JointRow *c = joint_of(0), *n = joint_of(min(1, rc - 1));
+            JointLane A, B;
+            jl_load(c ? *c : *any, lane, A);
+            int r = 0;
+            auto one = [&](JointLane& L, JointLane& N) {
+                jl_load(n ? *n : *any, lane, N);
+                JointRow* n2 = joint_of(min(r + 2, rc - 1));
+                if (c) joint(L, *c);
+                else contact(d.rows[rs + r]);
+                c = n;
+                n = n2;
+                r++;
+            };
+            while (true) {
+                one(A, B);
+                if (r >= rc) break;
+                one(B, A);
+                if (r >= rc) break;
             }
             __syncwarp();
         };
@@ -1007,7 +1120,7 @@ __global__ void __launch_bounds__(32, 4) k_pgs_joint(Dev d, int first) {
                  __syncwarp();
              });
         for (int it = 0; it < n_vel; it++)
-            pass([&](const JointLane& L, JointRow& R) { jl_step(L, R, dv, false, lane); },
+            pass([&](const JointLane& L, JointRow& R) { jl_step(L, R, dv, zero, false, lane); },
                  [&](RowBlock& R) {
                      if (lane == 0) {
                          float4 imp = R.imp;
@@ -1019,7 +1132,7 @@ __global__ void __launch_bounds__(32, 4) k_pgs_joint(Dev d, int first) {
                      __syncwarp();
                  });
         for (int it = 0; it < n_pos; it++)
-            pass([&](const JointLane& L, JointRow& R) { if (L.pos) jl_step(L, R, dv, true, lane); },   // needsPosCorrect
+            pass([&](const JointLane& L, JointRow& R) { if (L.pos) jl_step(L, R, dv, zero, true, lane); },   // needsPosCorrect
                  [&](RowBlock& R) {
                      if (lane == 0) {
                          float4 imp = R.imp;
@@ -1033,13 +1146,13 @@ __global__ void __launch_bounds__(32, 4) k_pgs_joint(Dev d, int first) {
             for (int it = 0; it < P.pgs_holo; it++)
                 for (int k = 0; k < sn; k++) {
                     const int s = d.isl_sys[ss + k];
-                    if (d.hs.fp64[s]) {
-                        holo_apply<double>(d, s, dv, err, false, -1.f, lane);
-                        holo_apply<double>(d, s, dv, err, true, d.lin_err_threshold, lane);
-                    } else {
-                        holo_apply<float>(d, s, dv, err, false, -1.f, lane);
-                        holo_apply<float>(d, s, dv, err, true, d.lin_err_threshold, lane);
-                    }
+                    auto find = [=](int j) -> JointRow* {
+                        for (int q = 0; q < held; q++)
+                            if (held_j[q] == j) return reinterpret_cast<JointRow*>(srows + q * kJointStage);
+                        return nullptr;
+                    };
+                    if (d.hs.fp64[s]) holo_system<double>(d, s, hsm, res, find, dv, err, lane);
+                    else holo_system<float>(d, s, hsm, res, find, dv, err, lane);
                 }
         }
         __syncwarp();
@@ -1047,8 +1160,14 @@ __global__ void __launch_bounds__(32, 4) k_pgs_joint(Dev d, int first) {
             const int c = d.rows[r].contact;
             if (c >= 0) continue;
             const int j = -c - 1;
-            const JointRow& R = d.jt.rows[j];
-            for (int k = 0; k < R.n; k++) d.jt.impulse[kJMax * j + k] = R.impulse[k];
+            const JointRow& R = *joint_of(r - rs);
+            for (int k = 0; k < R.n; k++) {
+                d.jt.impulse[kJMax * j + k] = R.impulse[k];
+                if (res) {   // a row that is kept (a limit, a motor) goes on from these
+                    d.jt.rows[j].impulse[k] = R.impulse[k];
+                    d.jt.rows[j].pimpulse[k] = R.pimpulse[k];
+                }
+            }
         }
         island_finish(d, rs, rc, bs, bc, dv, lane, 32);
         __syncwarp();
@@ -1198,6 +1317,7 @@ int pgs_big_blocks_per_sm(int dv_cap) {
 // a smaller one does not lower the limit under an earlier batch's launches
 void prepare_pgs(int dv_cap) {
     (void)dv_cap;
+    cudaFuncSetAttribute(k_pgs_joint, cudaFuncAttributeMaxDynamicSharedMemorySize, kJointSmem);
     cudaFuncSetAttribute(k_pgs_big<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, pgs_big_smem_bytes(kPgsDvCapMax));
 }
 
@@ -1209,7 +1329,7 @@ void launch_pgs_schedule(const Dev& d, const Launch& L) {
 
 void launch_pgs_joint(const Dev& d, bool first, const Launch& L) {
     if (d.n_joint_edges == 0) return;
-    k_pgs_joint<<<L.n_sms * 8, 32, 0, L.st>>>(d, first ? 1 : 0);
+    k_pgs_joint<<<L.n_sms * 3, 32, kJointSmem, L.st>>>(d, first ? 1 : 0);
 }
 
 void launch_pgs(const Dev& d, int dv_cap, int max_world, int big_blocks, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join,
@@ -1217,7 +1337,7 @@ void launch_pgs(const Dev& d, int dv_cap, int max_world, int big_blocks, cudaStr
     // large islands on the main stream, small ones (and islands whose Δv does
     // not fit in shared memory, where a world is large enough to hold one)
     // concurrently on a side branch
-    cudaMemsetAsync(d.sched + kBigNext, 0, 2 * sizeof(int), L.st);
+    cudaMemsetAsync(d.sched + kBigNext, 0, 3 * sizeof(int), L.st);
     cudaEventRecord(fork, L.st);
     cudaStreamWaitEvent(side, fork, 0);
     if (max_world > dv_cap) k_pgs_big<false><<<L.n_sms, 32, pgs_big_smem_bytes(0), side>>>(d, dv_cap);
