@@ -598,6 +598,20 @@ struct Batch {
     std::vector<int> world_jstart;     // joint ranges of the worlds
     std::vector<uint8_t> movement;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    // ray queries' device buffer (rays, results, ignored ids), kept between calls
+    // and grown as needed; freed with the batch
+    uint8_t* ray_mem = nullptr;
+    size_t ray_bytes = 0;
+    uint8_t* ray_buffer(size_t n) {
+        if (n > ray_bytes) {
+            if (ray_mem) CK(cudaFree(ray_mem));
+            ray_mem = nullptr;
+            ray_bytes = 0;
+            CK(cudaMalloc(&ray_mem, n));
+            ray_bytes = n;
+        }
+        return ray_mem;
+    }
     double* audit = nullptr;           // FP64 audit values (kAuditValues per world), null when disabled
 
     void drop_graphs() {
@@ -608,6 +622,7 @@ struct Batch {
         drop_graphs();
         if (pre_done) cudaEventDestroy(pre_done);
         if (audit) cudaFree(audit);
+        if (ray_mem) cudaFree(ray_mem);
         if (snap) cudaFree(snap);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
@@ -2750,26 +2765,23 @@ int cpgpu_raycast(cpgpu_world* w, const double* origins, const double* dirs, int
         if (n_rays > 0 && !w->w.bodies.empty()) {
             ensure_device(w->w);
             Batch& B = *w->w.dev;
-            std::vector<float> rays(6 * (size_t)n_rays);
+            // rays, then the ignored ids: one copy in, one out
+            const size_t nr = 6 * (size_t)n_rays, in_bytes = sizeof(float) * nr + sizeof(uint32_t) * (size_t)n_ignore;
+            const size_t out_at = (in_bytes + 255) & ~size_t(255);
+            std::vector<float> rays(nr + (size_t)n_ignore);
             for (size_t i = 0; i < 3 * (size_t)n_rays; i++) {
                 const size_t k = i / 3, c = i % 3;
                 rays[6 * k + c] = (float)origins[i];
                 rays[6 * k + 3 + c] = (float)dirs[i];
             }
-            float *d_rays = nullptr, *d_out = nullptr;
-            uint32_t* d_ig = nullptr;
-            CK(cudaMalloc(&d_rays, sizeof(float) * rays.size()));
-            CK(cudaMalloc(&d_out, sizeof(float) * out.size()));
-            CK(cudaMalloc(&d_ig, sizeof(uint32_t) * std::max(n_ignore, 1)));
-            CK(cudaMemcpyAsync(d_rays, rays.data(), sizeof(float) * rays.size(), cudaMemcpyHostToDevice, B.st));
-            if (n_ignore > 0) CK(cudaMemcpyAsync(d_ig, ignore, sizeof(uint32_t) * n_ignore, cudaMemcpyHostToDevice, B.st));
-            launch_raycast(B.cur(), 0, (int)w->w.bodies.size(), d_rays, n_rays, d_ig, n_ignore, d_out, B.st);
+            if (n_ignore > 0) std::memcpy(&rays[nr], ignore, sizeof(uint32_t) * (size_t)n_ignore);
+            uint8_t* mem = B.ray_buffer(out_at + sizeof(float) * out.size());
+            CK(cudaMemcpyAsync(mem, rays.data(), in_bytes, cudaMemcpyHostToDevice, B.st));
+            launch_raycast(B.cur(), 0, (int)w->w.bodies.size(), reinterpret_cast<float*>(mem), n_rays,
+                           reinterpret_cast<uint32_t*>(mem + sizeof(float) * nr), n_ignore, reinterpret_cast<float*>(mem + out_at), B.st);
             CK(cudaGetLastError());
-            CK(cudaMemcpyAsync(out.data(), d_out, sizeof(float) * out.size(), cudaMemcpyDeviceToHost, B.st));
+            CK(cudaMemcpyAsync(out.data(), mem + out_at, sizeof(float) * out.size(), cudaMemcpyDeviceToHost, B.st));
             CK(cudaStreamSynchronize(B.st));
-            cudaFree(d_rays);
-            cudaFree(d_out);
-            cudaFree(d_ig);
         }
         for (int k = 0; k < n_rays; k++) {
             const float* r = &out[8 * (size_t)k];
@@ -2792,10 +2804,31 @@ int cpgpu_num_bodies(cpgpu_world* w, int* n) {
     return CPGPU_OK;
 }
 
+// The poses and velocities alone, straight from the device: the contact graph,
+// pairs, joints and sleep records stay there (the host mirror is refreshed by
+// the calls that need it).
 int cpgpu_get_body_state(cpgpu_world* w, double* com, double* quat, double* vel, double* ang) {
     W_OR_FAIL(w);
     return guarded([&] {
-        if (w->w.dev && w->w.dev_valid) download_state(w->w);
+        if (w->w.dev && w->w.dev_valid && !w->w.bodies.empty()) {
+            Batch& B = *w->w.dev;
+            const Dev& x = B.cur();
+            const size_t N = w->w.bodies.size();
+            // the four arrays lie one after the other in the arena: one copy
+            const size_t rot0 = x.rot - x.pos, vel0 = x.vel - x.pos, ang0 = x.angv - x.pos;
+            std::vector<float4> a(ang0 + N);
+            CK(cudaMemcpyAsync(a.data(), x.pos, a.size() * sizeof(float4), cudaMemcpyDeviceToHost, B.st));
+            CK(cudaStreamSynchronize(B.st));
+            for (size_t i = 0; i < N; i++) {
+                const bool fixed = w->w.bodies[i].movement == CPGPU_FIXED;
+                const float4 p = a[i], q = a[rot0 + i], v = a[vel0 + i], o = a[ang0 + i];
+                if (com) { com[3 * i] = p.x; com[3 * i + 1] = p.y; com[3 * i + 2] = p.z; }
+                if (quat) { quat[4 * i] = q.x; quat[4 * i + 1] = q.y; quat[4 * i + 2] = q.z; quat[4 * i + 3] = q.w; }
+                if (vel) { vel[3 * i] = fixed ? 0 : v.x; vel[3 * i + 1] = fixed ? 0 : v.y; vel[3 * i + 2] = fixed ? 0 : v.z; }
+                if (ang) { ang[3 * i] = fixed ? 0 : o.x; ang[3 * i + 1] = fixed ? 0 : o.y; ang[3 * i + 2] = fixed ? 0 : o.z; }
+            }
+            return CPGPU_OK;
+        }
         for (size_t i = 0; i < w->w.bodies.size(); i++) {
             const Body& b = w->w.bodies[i];
             D3 v = b.movement == CPGPU_FIXED ? D3() : b.vel, a = b.movement == CPGPU_FIXED ? D3() : b.angv;
@@ -2812,10 +2845,17 @@ int cpgpu_get_asleep(cpgpu_world* w, int* flags) {
     W_OR_FAIL(w);
     return guarded([&] {
         if (!flags) throw ApiFail{CPGPU_ERR_INVALID_ARG, "null output"};
-        if (w->w.dev && w->w.dev_valid) download_state(w->w);
-        for (size_t i = 0; i < w->w.bodies.size(); i++) {
+        const size_t N = w->w.bodies.size();
+        // on a device batch without sleep state the mirror's flags hold
+        std::vector<int> a;
+        if (w->w.dev && w->w.dev_valid && w->w.dev->cur().has_sleep && N > 0) {
+            a.resize(N);
+            CK(cudaMemcpyAsync(a.data(), w->w.dev->cur().asleep, N * sizeof(int), cudaMemcpyDeviceToHost, w->w.dev->st));
+            CK(cudaStreamSynchronize(w->w.dev->st));
+        }
+        for (size_t i = 0; i < N; i++) {
             const Body& b = w->w.bodies[i];
-            flags[i] = (b.asleep && b.movement == CPGPU_DYNAMIC) ? 1 : 0;
+            flags[i] = ((a.empty() ? b.asleep : a[i]) && b.movement == CPGPU_DYNAMIC) ? 1 : 0;
         }
         return CPGPU_OK;
     });
