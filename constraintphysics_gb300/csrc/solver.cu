@@ -399,6 +399,8 @@ __global__ void k_sched_reset(Dev d) {
     if (threadIdx.x < 96) d.sched[threadIdx.x] = 0;
 }
 
+// sched[kLongIslands]: islands of at least 2^kLongBucket rows
+constexpr int kLongIslands = 4, kLongBucket = 9;
 __device__ __forceinline__ int size_bucket(int rows) { return 31 - __clz(rows); }
 
 __global__ void k_sched_count(Dev d) {
@@ -422,16 +424,31 @@ __global__ void k_sched_place(Dev d) {
         d.big_list[off + atomicAdd(&d.sched[64 + b], 1)] = i;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        int n = 0;
-        for (int k = 0; k < 32; k++) n += d.sched[32 + k];
+        int n = 0, lng = 0;
+        for (int k = 0; k < 32; k++) {
+            n += d.sched[32 + k];
+            if (k >= kLongBucket) lng += d.sched[32 + k];
+        }
         d.sched[0] = n;
+        d.sched[kLongIslands] = lng;
     }
 }
 
-// small islands: one thread walks the island's rows in global memory
+// small islands: one thread walks the island's rows in global memory.  Islands
+// are dealt to the warps in turn, so that a warp holds a few lanes' scattered
+// rows instead of 32 (6,300 islands of a world of 20,000 bodies: 1,203 -> 466
+// us); but to consecutive threads of half the blocks when there are more of
+// them than that (150,000 islands: 652 us, dealt out 1,217), or when a chain
+// of 512 rows or more bounds the step anyway: the fewer warps then slow that
+// chain less (96 served worlds 75 ms, dealt out 80).
 __global__ void k_pgs_small(Dev d) {
     const int n = d.sched[1];
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    const int nt = gridDim.x * blockDim.x, nw = nt >> 5;
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, warp = tid >> 5;
+    const bool dense = 2 * n > nt || d.sched[kLongIslands] > 0;
+    if (dense && 2 * blockIdx.x >= gridDim.x) return;
+    const int step = dense ? nt / 2 : nt;
+    for (int q = dense ? tid : warp + nw * (threadIdx.x & 31); q < n; q += step) {
         const int i = d.small_list[q];
         const int rs = d.g_isl_row_start[i], rc = d.g_isl_row_count[i];
         const int bs = d.g_isl_body_start[i], bc = d.g_isl_body_count[i];
@@ -1341,7 +1358,7 @@ void launch_pgs(const Dev& d, int dv_cap, int max_world, int big_blocks, cudaStr
     cudaEventRecord(fork, L.st);
     cudaStreamWaitEvent(side, fork, 0);
     if (max_world > dv_cap) k_pgs_big<false><<<L.n_sms, 32, pgs_big_smem_bytes(0), side>>>(d, dv_cap);
-    k_pgs_small<<<L.n_sms * 4, 64, 0, side>>>(d);
+    k_pgs_small<<<L.n_sms * 8, 64, 0, side>>>(d);
     cudaEventRecord(join, side);
     k_pgs_big<true><<<big_blocks, 32, pgs_big_smem_bytes(dv_cap), L.st>>>(d, dv_cap);
     cudaStreamWaitEvent(L.st, join, 0);
