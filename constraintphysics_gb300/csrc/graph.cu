@@ -226,22 +226,22 @@ __device__ __forceinline__ long long islands_need(int nb, int ne_w, int nj) {
 // systems, and once more to write them at the prefix of those counts.  The
 // result is the serial search's, position for position.
 
-// exclusive prefix of one value per thread (blockDim.x == 256) with the
-// block's total in *total; `ws` holds 8 ints
+// exclusive prefix of one value per thread (whole warps, at most 32) with the
+// block's total in *total; `ws` holds an int per warp
 __device__ int block_excl(int v, int* ws, int* total) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     int x = v;
     for (int o = 1; o < 32; o <<= 1) { int t = __shfl_up_sync(0xffffffffu, x, o); if (lane >= o) x += t; }
     if (lane == 31) ws[wid] = x;
     __syncthreads();
     if (wid == 0) {
-        int y = lane < 8 ? ws[lane] : 0;
-        for (int o = 1; o < 8; o <<= 1) { int t = __shfl_up_sync(0xffffffffu, y, o); if (lane >= o) y += t; }
-        if (lane < 8) ws[lane] = y;
+        int y = lane < nw ? ws[lane] : 0;
+        for (int o = 1; o < nw; o <<= 1) { int t = __shfl_up_sync(0xffffffffu, y, o); if (lane >= o) y += t; }
+        if (lane < nw) ws[lane] = y;
     }
     __syncthreads();
     const int incl = x + (wid > 0 ? ws[wid - 1] : 0);
-    *total = ws[7];
+    *total = ws[nw - 1];
     __syncthreads();
     return incl - v;
 }
@@ -626,10 +626,13 @@ __device__ void islands_small(const Dev& d, int w, int s, int nb, int e0, int ro
     }
 }
 
-__global__ void __launch_bounds__(256) k_islands(Dev d, int smem_bytes) {
+// NT threads a block: 256, or 1,024 for a batch of a few large worlds, whose
+// islands one block each walks through (4.3 -> 1.5 ms on 20,000 bodies)
+template <int NT>
+__global__ void __launch_bounds__(NT) k_islands(Dev d, int smem_bytes) {
     extern __shared__ int sm_isl[];
     __shared__ int sh_carry, sh_rows_end;
-    __shared__ int warp_sums[8];
+    __shared__ int warp_sums[NT / 32];
     const int w = blockIdx.x;
     const int s = d.world_start[w], e = d.world_start[w + 1];
     const int ne = *d.n_edges_new, ncon = *d.n_contacts_new;
@@ -707,7 +710,7 @@ __global__ void __launch_bounds__(256) k_islands(Dev d, int smem_bytes) {
         if (wid == 0) {
             int y = (lane < (nt >> 5)) ? warp_sums[lane] : 0;
             for (int o = 1; o < 32; o <<= 1) { int t = __shfl_up_sync(0xffffffffu, y, o); if (lane >= o) y += t; }
-            if (lane < 8) warp_sums[lane] = y;
+            if (lane < (nt >> 5)) warp_sums[lane] = y;
         }
         __syncthreads();
         const int incl = x + (wid > 0 ? warp_sums[wid - 1] : 0);
@@ -961,12 +964,14 @@ int islands_smem_bytes(int max_bodies) {
     // about four constraint edges per body, at most kIslandsSmemMax; the
     // kernel's limit (shared by every batch of the process) is that maximum
     const long long want = 4LL * (8LL * max_bodies + 7LL * 4 * max_bodies) + max_bodies + 64;
-    cudaFuncSetAttribute(k_islands, cudaFuncAttributeMaxDynamicSharedMemorySize, kIslandsSmemMax);
+    cudaFuncSetAttribute(k_islands<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, kIslandsSmemMax);
+    cudaFuncSetAttribute(k_islands<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, kIslandsSmemMax);
     return (int)std::min<long long>(want, kIslandsSmemMax);
 }
 
 void launch_islands(const Dev& d, int smem_bytes, const Launch& L) {
-    k_islands<<<d.n_worlds, 256, smem_bytes, L.st>>>(d, smem_bytes);
+    if (d.grid_buckets > 0 && d.n_worlds <= L.n_sms) k_islands<1024><<<d.n_worlds, 1024, smem_bytes, L.st>>>(d, smem_bytes);
+    else k_islands<256><<<d.n_worlds, 256, smem_bytes, L.st>>>(d, smem_bytes);
     scan_exclusive(d.isl_count_w, d.isl_scan, nullptr, d.n_worlds, d.n_worlds, d.n_islands, d.scan_tmp, L);
     k_island_copy<<<grid_for(d.n_bodies, 128, L.n_sms), 128, 0, L.st>>>(d);
 }
