@@ -647,7 +647,7 @@ struct Batch {
         mark(0);
         launch_step_begin(x, L);   mark(1);
         launch_pairs(x, L);        mark(2);
-        launch_narrowphase(x, slot_bytes, n_sms, prims, st); mark(3);   // + mesh pairs
+        launch_narrowphase(x, slot_bytes, n_sms, prims, side, fork, join, st); mark(3);   // + mesh pairs
         launch_merge(x, L);        mark(4);
         launch_islands(x, isl_smem, L);
         launch_pgs_schedule(x, L); mark(5);
@@ -1381,6 +1381,7 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
             x.sys_mark = A.take<int>(std::max<size_t>(hs_degree.size(), 1));
         }
         x.pair_a = A.take<int>(cap_pairs); x.pair_b = A.take<int>(cap_pairs);
+        x.np_next = A.take<int>(2);
         x.mf_n = A.take<float4>(cap_pairs); x.mf_cnt = A.take<int>(cap_pairs);
         x.mf_pt = A.take<float4>(4 * (size_t)cap_pairs); x.mf_magic = A.take<uint64_t>(4 * (size_t)cap_pairs);
         x.mf_feat = A.take<int2>(cap_pairs);

@@ -25,7 +25,8 @@ void launch_pairs(const Dev& d, const Launch& L);
 void launch_geometry(const Dev& d, int mode, const Launch& L);   // mode 0 moved bodies, 2 a batch's first pass
 // hull-hull pairs, then (when the batch holds spheres or cylinders) the pairs
 // that involve one
-void launch_narrowphase(const Dev& d, int slot_bytes, int n_sms, bool prims, cudaStream_t st);
+void launch_narrowphase(const Dev& d, int slot_bytes, int n_sms, bool prims, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join,
+                        cudaStream_t st);
 int mesh_scratch_warps(int n_sms);   // per-warp scratch entries the mesh narrowphase uses
 // ray queries against the bodies [s, e): rays 6 floats each (origin, unit
 // direction), `out` 8 floats per ray (body id bits, 0 = no hit; point;

@@ -1746,6 +1746,15 @@ __global__ void __launch_bounds__(128) k_clip(Dev d) {
     }
 }
 
+// The next pair for a warp.  A pair costs anything from a skip to a clipped
+// polygon, so the warps take pairs one by one: dealt out in advance, on average
+// 3.3 of a SM's 8 warps of k_narrow_prim still had work (333 mixed worlds).
+__device__ __forceinline__ int next_pair(int* counter, int lane) {
+    int p = 0;
+    if (lane == 0) p = atomicAdd(counter, 1);
+    return __shfl_sync(0xffffffffu, p, 0);
+}
+
 // One warp per candidate pair that involves a sphere or a cylinder (the other
 // pairs are k_narrowphase's).  Same staging as k_narrowphase.
 __global__ void __launch_bounds__(256, 1) k_narrow_prim(Dev d, int slot_bytes) {
@@ -1762,7 +1771,7 @@ __global__ void __launch_bounds__(256, 1) k_narrow_prim(Dev d, int slot_bytes) {
     Scratch scratch;
     CP clipped[kMaxClip];
     const int n_pairs = *d.n_pairs;
-    for (int p = blockIdx.x * warps_per_block + wib; p < n_pairs; p += gridDim.x * warps_per_block) {
+    for (int p = next_pair(&d.np_next[0], lane); p < n_pairs; p = next_pair(&d.np_next[0], lane)) {
         const int a = d.pair_a[p], b = d.pair_b[p];
         const uint8_t* ga = d.shapes + d.shape[a];
         const uint8_t* gb = d.shapes + d.shape[b];
@@ -1876,7 +1885,7 @@ __global__ void __launch_bounds__(256) k_narrow_mesh(Dev d, int slot_bytes) {
     Scratch scratch;
     CP clipped[kMaxClip];
     const int n_pairs = *d.n_pairs;
-    for (int p = gw; p < n_pairs; p += d.mesh_warps) {
+    for (int p = next_pair(&d.np_next[1], lane); p < n_pairs; p = next_pair(&d.np_next[1], lane)) {
         const int a = d.pair_a[p], b = d.pair_b[p];
         const uint8_t* ga = d.shapes + d.shape[a];
         const uint8_t* gb = d.shapes + d.shape[b];
@@ -2377,14 +2386,25 @@ void launch_raycast(const Dev& d, int s, int e, const float* rays, int n, const 
     k_raycast<<<n, nt, 0, st>>>(d, s, e, rays, n, ignore, n_ignore, out);
 }
 
-void launch_narrowphase(const Dev& d, int slot_bytes, int n_sms, bool prims, cudaStream_t st) {
+void launch_narrowphase(const Dev& d, int slot_bytes, int n_sms, bool prims, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join,
+                        cudaStream_t st) {
     const int warps = 8;
-    size_t smem = 16 * warps + (size_t)warps * (slot_bytes + kQueueBytes);
+    const size_t smem = 16 * warps + (size_t)warps * (slot_bytes + kQueueBytes);
+    const size_t smem_p = 16 * warps + (size_t)warps * slot_bytes;
+    // the kernels write different pairs' manifolds and run side by side (with
+    // unions, whose pairs k_narrowphase clears first, the mesh kernel follows)
+    const bool mesh = d.has_mesh || d.has_union, mesh_side = mesh && !d.has_union;
+    if (prims || mesh_side) {
+        cudaEventRecord(fork, st);
+        cudaStreamWaitEvent(side, fork, 0);
+        if (mesh_side) k_narrow_mesh<<<n_sms * kMeshBlocksPerSm, warps * 32, smem_p, side>>>(d, slot_bytes);
+        if (prims) k_narrow_prim<<<n_sms * 4, warps * 32, smem_p, side>>>(d, slot_bytes);
+        cudaEventRecord(join, side);
+    }
     k_narrowphase<<<n_sms * 4, warps * 32, smem, st>>>(d, slot_bytes);
     k_clip<<<n_sms * 16, 128, 0, st>>>(d);
-    if (prims) k_narrow_prim<<<n_sms * 4, warps * 32, 16 * warps + (size_t)warps * slot_bytes, st>>>(d, slot_bytes);
-    if (d.has_mesh || d.has_union)
-        k_narrow_mesh<<<n_sms * kMeshBlocksPerSm, warps * 32, 16 * warps + (size_t)warps * slot_bytes, st>>>(d, slot_bytes);
+    if (prims || mesh_side) cudaStreamWaitEvent(st, join, 0);
+    if (mesh && !mesh_side) k_narrow_mesh<<<n_sms * kMeshBlocksPerSm, warps * 32, smem_p, st>>>(d, slot_bytes);
 }
 
 }  // namespace cpgpu
