@@ -199,6 +199,7 @@ __global__ void k_clamp_pairs(Dev d) {
     if (*d.n_pairs > d.cap_pairs) { atomicOr(d.status, ST_PAIR_OVERFLOW); *d.n_pairs = d.cap_pairs; }
     if (d.has_mesh || d.has_union) *d.mm_count = 0;   // mesh store of this step's narrowphase
     d.np_next[0] = d.np_next[1] = 0;
+    for (int k = 0; k < 32; k++) d.prim_count_k[k] = 0;
 }
 
 // RigidBody::updateGeometry (RigidBody.cpp:281-312) for moved bodies: the

@@ -670,11 +670,11 @@ struct Batch {
         launch_audit(x, L);
     }
     // kernels per step: gravity 1, pairs 2 + scan 3 + clamp 1, narrowphase 2
-    // (+1 with spheres / cylinders, +1 with meshes), merge 6 + 3 scans, islands 2 + scan 3,
+    // (+3 with spheres / cylinders, +1 with meshes), merge 6 + 3 scans, islands 2 + scan 3,
     // schedule 3, 5 per substep (rows, small + grouped + large PGS, integrate), geometry 1
     // (+2 per substep and 1 factorisation with joints)
     int launches_per_step() const {
-        return 1 + 6 + 2 + (prims ? 1 : 0) + ((meshes || unions) ? 1 : 0) + (6 + 9) + (2 + 3) + 3 + 5 * substeps + 1 + (joints ? 2 * substeps : 0) +
+        return 1 + 6 + 2 + (prims ? 3 : 0) + ((meshes || unions) ? 1 : 0) + (6 + 9) + (2 + 3) + 3 + 5 * substeps + 1 + (joints ? 2 * substeps : 0) +
                (systems ? 1 : 0) + (audit ? 1 : 0) + (springs ? substeps : 0) + (tiles ? (all_tiles ? 6 : 8) : 0) +
                (max_world > dv_cap ? substeps : 0);
     }
@@ -1382,6 +1382,8 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
         }
         x.pair_a = A.take<int>(cap_pairs); x.pair_b = A.take<int>(cap_pairs);
         x.np_next = A.take<int>(2);
+        x.prim_count_k = A.take<int>(32);
+        x.prim_list = B->prims ? A.take<int>(cap_pairs) : nullptr;
         x.mf_n = A.take<float4>(cap_pairs); x.mf_cnt = A.take<int>(cap_pairs);
         x.mf_pt = A.take<float4>(4 * (size_t)cap_pairs); x.mf_magic = A.take<uint64_t>(4 * (size_t)cap_pairs);
         x.mf_feat = A.take<int2>(cap_pairs);

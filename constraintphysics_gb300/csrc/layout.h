@@ -351,6 +351,8 @@ struct Dev {
     int* mf_cnt;
     float4* mf_pt;                 // [4] per pair: pos xyz, w pen
     uint64_t* mf_magic;            // [4] per pair
+    int* prim_list;                // pairs with a round shape by kind (null: the batch holds none), and
+    int* prim_count_k;             // their counts per kind, then the cursors (32 ints)
     int* np_next;                  // next pair of the primitive and the mesh narrowphase
     int2* mf_feat;                 // hull pairs: features of the minimum axis (vertex of A, of B) for k_clip
     // static meshes (has_mesh == 0: none in the batch).  A mesh pair's points

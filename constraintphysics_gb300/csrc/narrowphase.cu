@@ -1757,6 +1757,46 @@ __device__ __forceinline__ int next_pair(int* counter, int lane) {
 
 // One warp per candidate pair that involves a sphere or a cylinder (the other
 // pairs are k_narrowphase's).  Same staging as k_narrowphase.
+// Pairs with a round shape listed by kind, the costliest kinds first: the
+// kernel holds nine detectors, far more code than the instruction cache, and
+// warps of one SM that run different ones wait for instructions most of the
+// time (4.2 of 10 cycles an instruction); a list by kind has them on the same
+// detector together, and the longest pairs start first.  Pass 0 counts the
+// kinds, pass 1 places.
+constexpr int kPrimKinds = 9;
+__device__ __forceinline__ int prim_kind(uint32_t ka, uint32_t kb) {
+    const uint32_t lo = ka < kb ? ka : kb, hi = ka < kb ? kb : ka;
+    if (lo == SHAPE_CYLINDER) return hi == SHAPE_CYLINDER ? 0 : 2;        // with a cylinder, a capsule
+    if (lo == SHAPE_HULL) return hi == SHAPE_CYLINDER ? 1 : hi == SHAPE_CAPSULE ? 3 : 4;
+    if (lo == SHAPE_CAPSULE) return 5;
+    return hi == SHAPE_CYLINDER ? 6 : hi == SHAPE_CAPSULE ? 7 : 8;         // a sphere
+}
+__global__ void __launch_bounds__(256) k_prim_list(Dev d, int pass) {
+    const int n = *d.n_pairs, lane = threadIdx.x & 31;
+    for (int p0 = blockIdx.x * blockDim.x; p0 < n; p0 += gridDim.x * blockDim.x) {
+        const int p = p0 + threadIdx.x;
+        int kind = -1;
+        if (p < n) {
+            const int a = d.pair_a[p], b = d.pair_b[p];
+            const uint32_t ka = reinterpret_cast<const HullHeader*>(d.shapes + d.shape[a])->kind;
+            const uint32_t kb = reinterpret_cast<const HullHeader*>(d.shapes + d.shape[b])->kind;
+            if ((ka | kb) != SHAPE_HULL && ka != SHAPE_MESH && kb != SHAPE_MESH && !is_union(d, a) && !is_union(d, b)) kind = prim_kind(ka, kb);
+        }
+        const unsigned same = __match_any_sync(0xffffffffu, kind);
+        if (kind < 0) continue;
+        const int first = __ffs(same) - 1, rank = __popc(same & ((1u << lane) - 1u));
+        int at = 0;
+        if (pass == 0) {
+            if (lane == first) atomicAdd(&d.prim_count_k[kind], __popc(same));
+        } else {
+            if (lane == first) at = atomicAdd(&d.prim_count_k[kPrimKinds + kind], __popc(same));
+            at = __shfl_sync(same, at, first);
+            for (int k = 0; k < kind; k++) at += d.prim_count_k[k];
+            d.prim_list[at + rank] = p;
+        }
+    }
+}
+
 __global__ void __launch_bounds__(256, 1) k_narrow_prim(Dev d, int slot_bytes) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int lane = threadIdx.x & 31;
@@ -1770,8 +1810,10 @@ __global__ void __launch_bounds__(256, 1) k_narrow_prim(Dev d, int slot_bytes) {
     bool failed = false;
     Scratch scratch;
     CP clipped[kMaxClip];
-    const int n_pairs = *d.n_pairs;
-    for (int p = next_pair(&d.np_next[0], lane); p < n_pairs; p = next_pair(&d.np_next[0], lane)) {
+    int n_pairs = 0;
+    for (int k = 0; k < kPrimKinds; k++) n_pairs += d.prim_count_k[k];
+    for (int q = next_pair(&d.np_next[0], lane); q < n_pairs; q = next_pair(&d.np_next[0], lane)) {
+        const int p = d.prim_list[q];
         const int a = d.pair_a[p], b = d.pair_b[p];
         const uint8_t* ga = d.shapes + d.shape[a];
         const uint8_t* gb = d.shapes + d.shape[b];
@@ -2398,6 +2440,10 @@ void launch_narrowphase(const Dev& d, int slot_bytes, int n_sms, bool prims, cud
         cudaEventRecord(fork, st);
         cudaStreamWaitEvent(side, fork, 0);
         if (mesh_side) k_narrow_mesh<<<n_sms * kMeshBlocksPerSm, warps * 32, smem_p, side>>>(d, slot_bytes);
+        if (prims) {
+            k_prim_list<<<n_sms * 2, 256, 0, side>>>(d, 0);
+            k_prim_list<<<n_sms * 2, 256, 0, side>>>(d, 1);
+        }
         if (prims) k_narrow_prim<<<n_sms * 4, warps * 32, smem_p, side>>>(d, slot_bytes);
         cudaEventRecord(join, side);
     }
