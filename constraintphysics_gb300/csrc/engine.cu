@@ -581,8 +581,7 @@ struct Batch {
     bool all_tiles = false;            // ... and no others
     bool systems = false;              // ... and holonomic systems
     cudaStream_t st = nullptr;
-    cudaStream_t side = nullptr;       // concurrent branch (small-island PGS)
-    cudaEvent_t fork = nullptr, join = nullptr;
+    Branches br;                       // concurrent branches (narrowphase kernels, PGS of smaller islands)
     int max_world = 0;                 // bodies of the largest world
     int dv_cap = 64;                   // island bodies whose Δv fits in shared memory
     int pgs_blocks = 0;                // k_pgs_big grid: one resident chain per block
@@ -627,9 +626,8 @@ struct Batch {
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         if (mem) cudaFree(mem);
-        if (fork) cudaEventDestroy(fork);
-        if (join) cudaEventDestroy(join);
-        if (side) cudaStreamDestroy(side);
+        for (cudaEvent_t e : {br.fork, br.join, br.join2}) if (e) cudaEventDestroy(e);
+        for (cudaStream_t q : {br.side, br.side2}) if (q) cudaStreamDestroy(q);
         if (st) cudaStreamDestroy(st);
     }
 
@@ -647,7 +645,7 @@ struct Batch {
         mark(0);
         launch_step_begin(x, L);   mark(1);
         launch_pairs(x, L);        mark(2);
-        launch_narrowphase(x, slot_bytes, n_sms, prims, side, fork, join, st); mark(3);   // + mesh pairs
+        launch_narrowphase(x, slot_bytes, n_sms, prims, br, st); mark(3);   // + mesh pairs
         launch_merge(x, L);        mark(4);
         launch_islands(x, isl_smem, L);
         launch_pgs_schedule(x, L); mark(5);
@@ -662,7 +660,7 @@ struct Batch {
             launch_springs(x, L);                          // impulses before the rows read the velocities
             launch_rows(x, s == 0, s == substeps - 1, L);
             launch_joint_rows(x, s == 0, L);               mark(6 + 3 * s);
-            launch_pgs(x, dv_cap, max_world, pgs_blocks, side, fork, join, L);
+            launch_pgs(x, dv_cap, max_world, pgs_blocks, br, L);
             launch_pgs_joint(x, s == 0, L);                mark(7 + 3 * s);
             launch_integrate(x, s == substeps - 1, L);     mark(8 + 3 * s);
         }
@@ -671,7 +669,7 @@ struct Batch {
     }
     // kernels per step: gravity 1, pairs 2 + scan 3 + clamp 1, narrowphase 2
     // (+3 with spheres / cylinders, +1 with meshes), merge 6 + 3 scans, islands 2 + scan 3,
-    // schedule 3, 5 per substep (rows, small + grouped + large PGS, integrate), geometry 1
+    // schedule 3, 5 per substep (rows, small + middling + large PGS, integrate), geometry 1
     // (+2 per substep and 1 factorisation with joints)
     int launches_per_step() const {
         return 1 + 6 + 2 + (prims ? 3 : 0) + ((meshes || unions) ? 1 : 0) + (6 + 9) + (2 + 3) + 3 + 5 * substeps + 1 + (joints ? 2 * substeps : 0) +
@@ -990,9 +988,8 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
     CK(cudaDeviceGetStreamPriorityRange(&prio_least, &prio_greatest));
     const int prio = rank < 0 ? prio_least : std::min(prio_least, prio_greatest + rank);
     CK(cudaStreamCreateWithPriority(&B->st, cudaStreamNonBlocking, prio));
-    CK(cudaStreamCreateWithPriority(&B->side, cudaStreamNonBlocking, prio));
-    CK(cudaEventCreateWithFlags(&B->fork, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&B->join, cudaEventDisableTiming));
+    for (cudaStream_t* q : {&B->br.side, &B->br.side2}) CK(cudaStreamCreateWithPriority(q, cudaStreamNonBlocking, prio));
+    for (cudaEvent_t* e : {&B->br.fork, &B->br.join, &B->br.join2}) CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     CK(cudaEventCreate(&B->ev0));
     CK(cudaEventCreate(&B->ev1));
 

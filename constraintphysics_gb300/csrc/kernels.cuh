@@ -11,6 +11,13 @@ struct Launch {
     cudaStream_t st;
 };
 
+// concurrent branches of a step: two side streams, the event that starts them
+// and the ones that join them
+struct Branches {
+    cudaStream_t side = nullptr, side2 = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr, join2 = nullptr;
+};
+
 // device-counted exclusive scan: out[i] = sum(in[0..i)), *total = sum(in[0..n))
 // where n = *n_dev (or n_host when n_dev is null); tmp needs 2 + cap/1024 ints.
 void scan_exclusive(const int* in, int* out, const int* n_dev, int n_host, int cap, int* total, int* tmp, const Launch& L);
@@ -25,8 +32,7 @@ void launch_pairs(const Dev& d, const Launch& L);
 void launch_geometry(const Dev& d, int mode, const Launch& L);   // mode 0 moved bodies, 2 a batch's first pass
 // hull-hull pairs, then (when the batch holds spheres or cylinders) the pairs
 // that involve one
-void launch_narrowphase(const Dev& d, int slot_bytes, int n_sms, bool prims, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join,
-                        cudaStream_t st);
+void launch_narrowphase(const Dev& d, int slot_bytes, int n_sms, bool prims, const Branches& b, cudaStream_t st);
 int mesh_scratch_warps(int n_sms);   // per-warp scratch entries the mesh narrowphase uses
 // ray queries against the bodies [s, e): rays 6 floats each (origin, unit
 // direction), `out` 8 floats per ray (body id bits, 0 = no hit; point;
@@ -57,8 +63,7 @@ void prepare_pgs(int dv_cap);
 int pgs_big_smem_bytes(int dv_cap);
 int pgs_big_blocks_per_sm(int dv_cap);
 // `max_world`: bodies of the batch's largest world
-void launch_pgs(const Dev& d, int dv_cap, int max_world, int big_blocks, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join,
-                const Launch& L);
+void launch_pgs(const Dev& d, int dv_cap, int max_world, int big_blocks, const Branches& b, const Launch& L);
 void launch_integrate(const Dev& d, int last, const Launch& L);
 // joints: rows every substep, the holonomic systems' factorisation on the
 // first; islands with joint rows solved by their own kernel

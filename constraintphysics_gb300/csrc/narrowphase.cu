@@ -2428,8 +2428,7 @@ void launch_raycast(const Dev& d, int s, int e, const float* rays, int n, const 
     k_raycast<<<n, nt, 0, st>>>(d, s, e, rays, n, ignore, n_ignore, out);
 }
 
-void launch_narrowphase(const Dev& d, int slot_bytes, int n_sms, bool prims, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join,
-                        cudaStream_t st) {
+void launch_narrowphase(const Dev& d, int slot_bytes, int n_sms, bool prims, const Branches& br, cudaStream_t st) {
     const int warps = 8;
     const size_t smem = 16 * warps + (size_t)warps * (slot_bytes + kQueueBytes);
     const size_t smem_p = 16 * warps + (size_t)warps * slot_bytes;
@@ -2437,19 +2436,19 @@ void launch_narrowphase(const Dev& d, int slot_bytes, int n_sms, bool prims, cud
     // unions, whose pairs k_narrowphase clears first, the mesh kernel follows)
     const bool mesh = d.has_mesh || d.has_union, mesh_side = mesh && !d.has_union;
     if (prims || mesh_side) {
-        cudaEventRecord(fork, st);
-        cudaStreamWaitEvent(side, fork, 0);
-        if (mesh_side) k_narrow_mesh<<<n_sms * kMeshBlocksPerSm, warps * 32, smem_p, side>>>(d, slot_bytes);
+        cudaEventRecord(br.fork, st);
+        cudaStreamWaitEvent(br.side, br.fork, 0);
+        if (mesh_side) k_narrow_mesh<<<n_sms * kMeshBlocksPerSm, warps * 32, smem_p, br.side>>>(d, slot_bytes);
         if (prims) {
-            k_prim_list<<<n_sms * 2, 256, 0, side>>>(d, 0);
-            k_prim_list<<<n_sms * 2, 256, 0, side>>>(d, 1);
+            k_prim_list<<<n_sms * 2, 256, 0, br.side>>>(d, 0);
+            k_prim_list<<<n_sms * 2, 256, 0, br.side>>>(d, 1);
         }
-        if (prims) k_narrow_prim<<<n_sms * 4, warps * 32, smem_p, side>>>(d, slot_bytes);
-        cudaEventRecord(join, side);
+        if (prims) k_narrow_prim<<<n_sms * 4, warps * 32, smem_p, br.side>>>(d, slot_bytes);
+        cudaEventRecord(br.join, br.side);
     }
     k_narrowphase<<<n_sms * 4, warps * 32, smem, st>>>(d, slot_bytes);
     k_clip<<<n_sms * 16, 128, 0, st>>>(d);
-    if (prims || mesh_side) cudaStreamWaitEvent(st, join, 0);
+    if (prims || mesh_side) cudaStreamWaitEvent(st, br.join, 0);
     if (mesh && !mesh_side) k_narrow_mesh<<<n_sms * kMeshBlocksPerSm, warps * 32, smem_p, st>>>(d, slot_bytes);
 }
 

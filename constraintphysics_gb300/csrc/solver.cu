@@ -401,14 +401,19 @@ __global__ void k_sched_reset(Dev d) {
 
 // sched[kLongIslands]: islands of at least 2^kLongBucket rows
 constexpr int kLongIslands = 4, kLongBucket = 9;
+// islands of kMidRows to kMidMax rows below the big ones: sched[kMidIslands];
+// from kMidRowsFew rows in a batch of up to kMidFew islands
+constexpr int kMidIslands = 5, kMidRows = 16, kMidMax = 48, kMidRowsFew = 4, kMidFew = 8192;
 __device__ __forceinline__ int size_bucket(int rows) { return 31 - __clz(rows); }
 
 __global__ void k_sched_count(Dev d) {
     const int ni = *d.n_islands;
+    const int mid = ni <= kMidFew ? kMidRowsFew : kMidRows;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ni; i += gridDim.x * blockDim.x) {
         if (d.n_joint_edges > 0 && d.g_isl_flags[i]) { d.joint_list[atomicAdd(&d.sched[3], 1)] = i; continue; }
         int rc = d.g_isl_row_count[i];
         if (rc >= d.big_rows) atomicAdd(&d.sched[32 + size_bucket(rc)], 1);
+        else if (rc >= mid && rc <= kMidMax && d.g_isl_body_count[i] <= kMidMax + 1) d.big_list[d.n_bodies - 1 - atomicAdd(&d.sched[kMidIslands], 1)] = i;   // from the list's end
         else d.small_list[atomicAdd(&d.sched[1], 1)] = i;
     }
 }
@@ -913,6 +918,62 @@ __global__ void __launch_bounds__(32) k_pgs_big(Dev d, int dv_cap) {
     big_worker<SH>(d, dv_cap, sm, &d.sched[kBigNext + (SH ? 0 : 1)], d.sched[0]);
 }
 
+// Islands of a few rows: the chain with all of the island's rows in shared
+// memory, 21 KB a warp, so that many run beside each other (the big islands'
+// workers take two to five to an SM).  A thread walking its rows in global
+// memory takes 0.2 to 0.45 us a row-step against 0.13 here, but a warp's start
+// and end cost ~4 us an island: from 4 rows while one or a few islands fall to a
+// warp, from 16 in batches of more islands.  Beside a chain of 512 rows or more,
+// which bounds the step, only `few` blocks run (the others would hold shared
+// memory that the big islands' workers need).
+constexpr int kMidSmem = 64 + kMidMax * (int)sizeof(RowBlock) + (kMidMax + 2) * 16 * kDvF4;
+constexpr int kMidNext = kBigNext + 3;   // sched: the next list entry
+__global__ void __launch_bounds__(32) k_pgs_mid(Dev d, int few) {
+    extern __shared__ __align__(16) uint8_t sm[];
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sm);
+    RowBlock* ring = reinterpret_cast<RowBlock*>(sm + 64);
+    float4* dv = reinterpret_cast<float4*>(sm + 64 + kMidMax * sizeof(RowBlock)) + kDvF4;   // after the zero entry
+    if ((int)blockIdx.x >= few && d.sched[kLongIslands] > 0) return;
+    const int lane = threadIdx.x, n = d.sched[kMidIslands];
+    if ((int)blockIdx.x >= n) return;
+    if (lane == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(bar)), "r"(1) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (lane < kDvF4) dv[lane - kDvF4] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncwarp();
+    uint32_t parity = 0;
+    while (true) {
+        int q = 0;
+        if (lane == 0) q = atomicAdd(&d.sched[kMidNext], 1);
+        q = __shfl_sync(0xffffffffu, q, 0);
+        if (q >= n) break;
+        const int i = d.big_list[d.n_bodies - 1 - q];
+        const int bs = d.g_isl_body_start[i], bc = d.g_isl_body_count[i];   // at most kMidMax + 1 bodies
+        const int rs = d.g_isl_row_start[i], rc = d.g_isl_row_count[i];
+        const WorldParams& P = d.wparams[d.g_isl_world[i]];
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the last island's rows were written in place
+        __syncwarp();
+        if (lane == 0) ring_load(ring, d.rows + rs, rc, bar, false);
+        for (int k = lane; k < kDvF4 * bc; k += 32) dv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int n_vel = P.pgs_vel, n_pos = P.pgs_pos;
+        const bool ok = ring_wait(bar, parity, d.wait_limit);
+        parity ^= 1u;
+        if (!__all_sync(0xffffffffu, ok)) {
+            ring_wait(bar, parity ^ 1u, kDefaultWaitLimit);   // let the copy land (bounded)
+            if (lane == 0) atomicOr(d.status, ST_TIMEOUT);
+            return;
+        }
+        RowFeed x;
+        x.ring = ring;
+        x.rows = d.rows + rs;
+        x.rc = rc;
+        x.t = x.total = 0;   // nothing left to arrive
+        chain_passes<true, true>(x, dv, lane, n_vel, n_pos);
+        __syncwarp();
+        island_finish(d, rs, rc, bs, bc, dv, lane, 32);
+        __syncwarp();
+    }
+}
+
 // HolonomicSystem::computeAndApplyImpulses (HolonomicBlockSolver.cpp:319-378)
 // for system s by one warp: solve A d = t - J dv with the factorisation, then
 // (with a threshold) discard a pseudo solution whose angular velocity change
@@ -1349,19 +1410,22 @@ void launch_pgs_joint(const Dev& d, bool first, const Launch& L) {
     k_pgs_joint<<<L.n_sms * 3, 32, kJointSmem, L.st>>>(d, first ? 1 : 0);
 }
 
-void launch_pgs(const Dev& d, int dv_cap, int max_world, int big_blocks, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join,
-                const Launch& L) {
-    // large islands on the main stream, small ones (and islands whose Δv does
-    // not fit in shared memory, where a world is large enough to hold one)
-    // concurrently on a side branch
-    cudaMemsetAsync(d.sched + kBigNext, 0, 3 * sizeof(int), L.st);
-    cudaEventRecord(fork, L.st);
-    cudaStreamWaitEvent(side, fork, 0);
-    if (max_world > dv_cap) k_pgs_big<false><<<L.n_sms, 32, pgs_big_smem_bytes(0), side>>>(d, dv_cap);
-    k_pgs_small<<<L.n_sms * 8, 64, 0, side>>>(d);
-    cudaEventRecord(join, side);
+void launch_pgs(const Dev& d, int dv_cap, int max_world, int big_blocks, const Branches& b, const Launch& L) {
+    // large islands on the main stream, middling and small ones (and islands
+    // whose Δv does not fit in shared memory, where a world is large enough to
+    // hold one) concurrently on side branches
+    cudaMemsetAsync(d.sched + kBigNext, 0, 4 * sizeof(int), L.st);
+    cudaEventRecord(b.fork, L.st);
+    cudaStreamWaitEvent(b.side, b.fork, 0);
+    cudaStreamWaitEvent(b.side2, b.fork, 0);
+    if (max_world > dv_cap) k_pgs_big<false><<<L.n_sms, 32, pgs_big_smem_bytes(0), b.side>>>(d, dv_cap);
+    k_pgs_small<<<L.n_sms * 8, 64, 0, b.side>>>(d);
+    cudaEventRecord(b.join, b.side);
+    k_pgs_mid<<<L.n_sms * 10, 32, kMidSmem, b.side2>>>(d, L.n_sms * 2);
+    cudaEventRecord(b.join2, b.side2);
     k_pgs_big<true><<<big_blocks, 32, pgs_big_smem_bytes(dv_cap), L.st>>>(d, dv_cap);
-    cudaStreamWaitEvent(L.st, join, 0);
+    cudaStreamWaitEvent(L.st, b.join, 0);
+    cudaStreamWaitEvent(L.st, b.join2, 0);
 }
 
 void launch_integrate(const Dev& d, int last, const Launch& L) {
