@@ -1,5 +1,4 @@
-// broadphase.cu — gravity, candidate pairs, geometry/AABB update and the
-// device-counted exclusive scan used by the graph kernels.
+// broadphase.cu — gravity, candidate pairs and the geometry/AABB update.
 //
 // Pair generation returns exactly the set the reference's AABB tree returns:
 // every pair of bodies of the same world whose true AABBs overlap under the
@@ -18,74 +17,12 @@
 #include "kernels.cuh"
 #include "devmath.cuh"
 #include "pairs.cuh"
+#include "scan.cuh"
 #include "shapes.cuh"
 
 namespace cpgpu {
 
 namespace {
-constexpr int kScanBlock = 1024;
-
-// inclusive block scan of one value per thread (blockDim.x == kScanBlock)
-__device__ int block_scan_incl(int v, int* warp_sums) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int o = 1; o < 32; o <<= 1) {
-        int t = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += t;
-    }
-    if (lane == 31) warp_sums[wid] = v;
-    __syncthreads();
-    if (wid == 0) {
-        int s = (lane < (blockDim.x >> 5)) ? warp_sums[lane] : 0;
-        for (int o = 1; o < 32; o <<= 1) {
-            int t = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o) s += t;
-        }
-        warp_sums[lane] = s;
-    }
-    __syncthreads();
-    if (wid > 0) v += warp_sums[wid - 1];
-    __syncthreads();
-    return v;
-}
-
-__global__ void k_scan_chunks(const int* in, int* out, const int* n_dev, int n_host, int* chunk_sums) {
-    __shared__ int ws[32];
-    const int n = n_dev ? *n_dev : n_host;
-    const int nchunks = (n + kScanBlock - 1) / kScanBlock;
-    for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
-        int i = c * kScanBlock + threadIdx.x;
-        int v = (i < n) ? in[i] : 0;
-        int inc = block_scan_incl(v, ws);
-        if (i < n) out[i] = inc - v;
-        if (threadIdx.x == kScanBlock - 1) chunk_sums[c] = inc;
-    }
-}
-
-__global__ void k_scan_top(int* chunk_sums, const int* n_dev, int n_host, int* total) {
-    __shared__ int ws[32];
-    __shared__ int carry;
-    const int n = n_dev ? *n_dev : n_host;
-    const int nchunks = (n + kScanBlock - 1) / kScanBlock;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int base = 0; base < nchunks; base += kScanBlock) {
-        int i = base + threadIdx.x;
-        int v = (i < nchunks) ? chunk_sums[i] : 0;
-        int inc = block_scan_incl(v, ws);
-        int c0 = carry;
-        if (i < nchunks) chunk_sums[i] = c0 + inc - v;
-        __syncthreads();
-        if (threadIdx.x == kScanBlock - 1) carry = c0 + inc;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *total = carry;
-}
-
-__global__ void k_scan_add(int* out, const int* n_dev, int n_host, const int* chunk_sums) {
-    const int n = n_dev ? *n_dev : n_host;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] += chunk_sums[i / kScanBlock];
-}
-
 __global__ void k_gravity(Dev d) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < d.n_bodies; i += gridDim.x * blockDim.x) {
         if (d.movement[i] != 0) continue;
@@ -195,12 +132,19 @@ __global__ void __launch_bounds__(256) k_grid_write(Dev d) {
     }
 }
 
-__global__ void k_clamp_pairs(Dev d) {
-    if (*d.n_pairs > d.cap_pairs) { atomicOr(d.status, ST_PAIR_OVERFLOW); *d.n_pairs = d.cap_pairs; }
-    if (d.has_mesh || d.has_union) *d.mm_count = 0;   // mesh store of this step's narrowphase
-    d.np_next[0] = d.np_next[1] = 0;
-    for (int k = 0; k < 32; k++) d.prim_count_k[k] = 0;
-}
+// pair counts to offsets; the total is clamped to the capacity, and this
+// step's narrowphase counters start at zero
+struct PairScan {
+    static __device__ int in(const Dev& d, int i) { return d.pair_count[i]; }
+    static __device__ void out(const Dev& d, int i, int x) { d.pair_count[i] = x; }
+    static __device__ void done(const Dev& d, int total) {
+        if (total > d.cap_pairs) { atomicOr(d.status, ST_PAIR_OVERFLOW); total = d.cap_pairs; }
+        *d.n_pairs = total;
+        if (d.has_mesh || d.has_union) *d.mm_count = 0;   // mesh store of this step's narrowphase
+        d.np_next[0] = d.np_next[1] = 0;
+        for (int k = 0; k < 32; k++) d.prim_count_k[k] = 0;
+    }
+};
 
 // RigidBody::updateGeometry (RigidBody.cpp:281-312) for moved bodies: the
 // orientation is renormalised and the AABB recomputed from the world geometry
@@ -242,14 +186,6 @@ __global__ void k_geometry(Dev d, int mode) {
 }
 }  // namespace
 
-void scan_exclusive(const int* in, int* out, const int* n_dev, int n_host, int cap, int* total, int* tmp, const Launch& L) {
-    int max_chunks = (cap + kScanBlock - 1) / kScanBlock;
-    int g = max_chunks < L.n_sms * 2 ? (max_chunks > 0 ? max_chunks : 1) : L.n_sms * 2;
-    k_scan_chunks<<<g, kScanBlock, 0, L.st>>>(in, out, n_dev, n_host, tmp);
-    k_scan_top<<<1, kScanBlock, 0, L.st>>>(tmp, n_dev, n_host, total);
-    k_scan_add<<<L.n_sms * 4, 256, 0, L.st>>>(out, n_dev, n_host, tmp);
-}
-
 static int grid_for(int n, int per_block, int n_sms) {
     int g = (n + per_block - 1) / per_block;
     int cap = n_sms * 8;
@@ -272,13 +208,12 @@ void launch_pairs(const Dev& d, const Launch& L) {
         k_grid_far<<<64, 1024, 0, L.st>>>(d, 0);
     }
     if (!d.all_grid) k_pairs<<<g, 256, 0, L.st>>>(d, 0);
-    scan_exclusive(d.pair_count, d.pair_count, nullptr, d.n_bodies, d.n_bodies, d.n_pairs, d.scan_tmp, L);
+    launch_scan<PairScan>(d, nullptr, d.n_bodies, d.n_bodies, L);
     if (grid) {
         k_grid_far<<<64, 1024, 0, L.st>>>(d, 1);
         k_grid_write<<<gw, 256, 0, L.st>>>(d);
     }
     if (!d.all_grid) k_pairs<<<g, 256, 0, L.st>>>(d, 1);
-    k_clamp_pairs<<<1, 1, 0, L.st>>>(d);
 }
 
 void launch_geometry(const Dev& d, int mode, const Launch& L) {

@@ -667,12 +667,12 @@ struct Batch {
         launch_geometry(x, 0, L);  mark(6 + 3 * substeps);
         launch_audit(x, L);
     }
-    // kernels per step: gravity 1, pairs 2 + scan 3 + clamp 1, narrowphase 2
-    // (+3 with spheres / cylinders, +1 with meshes), merge 6 + 3 scans, islands 2 + scan 3,
-    // schedule 3, 5 per substep (rows, small + middling + large PGS, integrate), geometry 1
+    // kernels per step: gravity 1, pairs 2 + scan 1, narrowphase 2
+    // (+3 with spheres / cylinders, +1 with meshes), merge 3 + 3 scans, islands 2 + scan 1,
+    // schedule 2, 5 per substep (rows, small + middling + large PGS, integrate), geometry 1
     // (+2 per substep and 1 factorisation with joints)
     int launches_per_step() const {
-        return 1 + 6 + 2 + (prims ? 3 : 0) + ((meshes || unions) ? 1 : 0) + (6 + 9) + (2 + 3) + 3 + 5 * substeps + 1 + (joints ? 2 * substeps : 0) +
+        return 1 + 3 + 2 + (prims ? 3 : 0) + ((meshes || unions) ? 1 : 0) + (3 + 3) + (2 + 1) + 2 + 5 * substeps + 1 + (joints ? 2 * substeps : 0) +
                (systems ? 1 : 0) + (audit ? 1 : 0) + (springs ? substeps : 0) + (tiles ? (all_tiles ? 6 : 8) : 0) +
                (max_world > dv_cap ? substeps : 0);
     }
@@ -1321,7 +1321,7 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
     const bool mstore = B->meshes || B->unions;   // pairs through the mesh store
     const int cap_mesh = mstore ? std::max(4096, env_int("CPGPU_MESH_POINTS_PER_BODY", 32) * N) : 0;
     const int mesh_warps = mstore ? mesh_scratch_warps(B->n_sms) : 0;
-    const int scan_tmp = std::max(cap_pairs, cap_contacts) / 1024 + 64;
+    const size_t scan_words = std::max({cap_pairs, cap_contacts, cap_edges, N}) / 1024 + 64;   // more than the scans' chunks
     Dev x;
     EdgeStore es[2];
     ContactStore cs[2];
@@ -1395,10 +1395,10 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
         counts = A.take<int>(64);   // n_pairs, n_edges[2], n_contacts[2], n_islands, status, .., cnt[16..]
         x.n_pairs = counts + 0;
         x.surv = A.take<int>(cap_edges); x.surv_scan = A.take<int>(cap_edges);
-        x.unm = A.take<int>(cap_pairs); x.unm_scan = A.take<int>(cap_pairs); x.pair_edge = A.take<int>(cap_pairs);
+        x.unm = A.take<int>(cap_pairs); x.unm_scan = A.take<int>(cap_pairs);
         x.edge_src = A.take<int>(cap_edges); x.edge_pair = A.take<int>(cap_edges); x.edge_cnt = A.take<int>(cap_edges);
         x.edge_live = A.take<int>(cap_edges); x.edge_row = A.take<int>(cap_edges);
-        x.scan_tmp = A.take<int>(scan_tmp);
+        x.scan_tmp = reinterpret_cast<ScanTmp*>(A.take<unsigned long long>(scan_words));
         x.adj_ofs = A.take<int>(N); x.adj_cursor = A.take<int>(N);
         x.adj_list = A.take<int>(2 * (2 * ((size_t)cap_edges + n_je) + N));
         x.visited = A.take<int>(N);
@@ -1502,6 +1502,7 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
     // ---- upload
     auto up = [&](void* dst, const void* src, size_t n) { if (n) CK(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, B->st)); };
     CK(cudaMemsetAsync(counts, 0, 64 * sizeof(int), B->st));
+    CK(cudaMemsetAsync(x.scan_tmp, 0, scan_words * sizeof(unsigned long long), B->st));
     up(d_wp, wp.data(), wp.size() * sizeof(WorldParams));
     up(d_wstart, wstart.data(), wstart.size() * sizeof(int));
     up(d_map, map_order.data(), N * sizeof(int));

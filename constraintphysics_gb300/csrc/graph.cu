@@ -19,6 +19,7 @@
 // connected components in parallel (islands_big), with the same result.
 #include "kernels.cuh"
 #include "devmath.cuh"
+#include "scan.cuh"
 
 namespace cpgpu {
 
@@ -46,26 +47,54 @@ __device__ __forceinline__ int lower_bound_pairs(const Dev& d, int n, uint64_t k
     return lo;
 }
 
-__global__ void k_surv(Dev d) {
-    const int n = *d.n_edges_old;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+// the previous step's edges that keep a contact, and their prefix
+struct SurvScan {
+    static __device__ int in(const Dev& d, int e) {
         int s = d.e_old.cstart[e], c = d.e_old.ccount[e], alive = 0;
         for (int k = s; k < s + c; k++) alive += !cs_dead(d.c_old.state[k]);
-        d.surv[e] = alive > 0;
+        return d.surv[e] = alive > 0;
     }
-}
-
-__global__ void k_pair_match(Dev d) {
-    const int np = *d.n_pairs, ne = *d.n_edges_old;
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
+    static __device__ void out(const Dev& d, int e, int x) { d.surv_scan[e] = x; }
+    static __device__ void done(const Dev& d, int total) { d.cnt[0] = total; }
+};
+// the pairs with a manifold and no surviving edge, and their prefix; the two
+// totals give the new edge count
+struct UnmatchedScan {
+    static __device__ int in(const Dev& d, int p) {
         bool hasm = d.mf_n[p].w > 0.f;
+        const int ne = *d.n_edges_old;
         uint64_t key = pair_key(d, p);
         int e = lower_bound_u64(d.e_old.key, ne, key);
         bool matched = e < ne && d.e_old.key[e] == key && d.surv[e];
-        d.pair_edge[p] = matched ? e : -1;
-        d.unm[p] = hasm && !matched;
+        return d.unm[p] = hasm && !matched;
     }
-}
+    static __device__ void out(const Dev& d, int p, int x) { d.unm_scan[p] = x; }
+    static __device__ void done(const Dev& d, int total) {
+        d.cnt[1] = total;
+        int n = d.cnt[0] + total;
+        if (n > d.cap_edges) { atomicOr(d.status, ST_EDGE_OVERFLOW); n = d.cap_edges; }
+        *d.n_edges_new = n;
+    }
+};
+// contacts per new edge to their first contacts
+struct ContactScan {
+    static __device__ int in(const Dev& d, int e) { return d.edge_cnt[e]; }
+    static __device__ void out(const Dev& d, int e, int x) { d.e_new.cstart[e] = x; }
+    static __device__ void done(const Dev& d, int total) {
+        if (total > d.cap_contacts) { atomicOr(d.status, ST_CONTACT_OVERFLOW); total = d.cap_contacts; }
+        *d.n_contacts_new = total;
+    }
+};
+// islands per world to their places in the batch's list; the solver schedule's
+// counters start at zero
+struct IslandScan {
+    static __device__ int in(const Dev& d, int w) { return d.isl_count_w[w]; }
+    static __device__ void out(const Dev& d, int w, int x) { d.isl_scan[w] = x; }
+    static __device__ void done(const Dev& d, int total) {
+        *d.n_islands = total;
+        for (int k = 0; k < 96; k++) d.sched[k] = 0;
+    }
+};
 
 // cnt[0] = surviving old edges, cnt[1] = unmatched manifolds (both from scans)
 __global__ void k_place(Dev d, const int* cnt) {
@@ -95,16 +124,6 @@ __global__ void k_place(Dev d, const int* cnt) {
             d.edge_pair[pos] = p;
         }
     }
-}
-
-__global__ void k_edge_total(Dev d, const int* cnt) {
-    int n = cnt[0] + cnt[1];
-    if (n > d.cap_edges) { atomicOr(d.status, ST_EDGE_OVERFLOW); n = d.cap_edges; }
-    *d.n_edges_new = n;
-}
-
-__global__ void k_contact_total(Dev d) {
-    if (*d.n_contacts_new > d.cap_contacts) { atomicOr(d.status, ST_CONTACT_OVERFLOW); *d.n_contacts_new = d.cap_contacts; }
 }
 
 // per new edge: surviving old contacts (in order), then this step's manifold
@@ -925,16 +944,11 @@ int grid_for(int n, int per_block, int n_sms) {
 
 void launch_merge(const Dev& d, const Launch& L) {
     const int gb = L.n_sms * 4, bs = 256;
-    int* cnt = d.cnt;
-    k_surv<<<gb, bs, 0, L.st>>>(d);
-    scan_exclusive(d.surv, d.surv_scan, d.n_edges_old, 0, d.cap_edges, cnt + 0, d.scan_tmp, L);
-    k_pair_match<<<gb, bs, 0, L.st>>>(d);
-    scan_exclusive(d.unm, d.unm_scan, d.n_pairs, 0, d.cap_pairs, cnt + 1, d.scan_tmp, L);
-    k_place<<<gb, bs, 0, L.st>>>(d, cnt);
-    k_edge_total<<<1, 1, 0, L.st>>>(d, cnt);
+    launch_scan<SurvScan>(d, d.n_edges_old, 0, d.cap_edges, L);
+    launch_scan<UnmatchedScan>(d, d.n_pairs, 0, d.cap_pairs, L);
+    k_place<<<gb, bs, 0, L.st>>>(d, d.cnt);
     k_contacts<<<gb, 128, 0, L.st>>>(d, 0);
-    scan_exclusive(d.edge_cnt, d.e_new.cstart, d.n_edges_new, 0, d.cap_edges, d.n_contacts_new, d.scan_tmp, L);
-    k_contact_total<<<1, 1, 0, L.st>>>(d);
+    launch_scan<ContactScan>(d, d.n_edges_new, 0, d.cap_edges, L);
     k_contacts<<<gb, 128, 0, L.st>>>(d, 1);
 }
 
@@ -972,7 +986,7 @@ int islands_smem_bytes(int max_bodies) {
 void launch_islands(const Dev& d, int smem_bytes, const Launch& L) {
     if (d.grid_buckets > 0 && d.n_worlds <= L.n_sms) k_islands<1024><<<d.n_worlds, 1024, smem_bytes, L.st>>>(d, smem_bytes);
     else k_islands<256><<<d.n_worlds, 256, smem_bytes, L.st>>>(d, smem_bytes);
-    scan_exclusive(d.isl_count_w, d.isl_scan, nullptr, d.n_worlds, d.n_worlds, d.n_islands, d.scan_tmp, L);
+    launch_scan<IslandScan>(d, nullptr, d.n_worlds, d.n_worlds, L);
     k_island_copy<<<grid_for(d.n_bodies, 128, L.n_sms), 128, 0, L.st>>>(d);
 }
 

@@ -18,10 +18,6 @@ struct Branches {
     cudaEvent_t fork = nullptr, join = nullptr, join2 = nullptr;
 };
 
-// device-counted exclusive scan: out[i] = sum(in[0..i)), *total = sum(in[0..n))
-// where n = *n_dev (or n_host when n_dev is null); tmp needs 2 + cap/1024 ints.
-void scan_exclusive(const int* in, int* out, const int* n_dev, int n_host, int cap, int* total, int* tmp, const Launch& L);
-
 void prepare_kernels();   // one-time function attributes (outside graph capture)
 void set_last_error(const char* msg);   // message returned by cpgpu_last_error
 void launch_gravity(const Dev& d, const Launch& L);

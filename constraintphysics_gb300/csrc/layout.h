@@ -312,6 +312,14 @@ constexpr int kSchedInts = 1024;
 constexpr int kTileWorld = 2048;   // worlds above this many bodies take the pair grid and component-parallel islands
 constexpr int kCompArrays = 12;
 
+// Counters and chunk words of the prefix kernel (scan.cuh); zero before its
+// first launch, one word per chunk of the largest scan
+struct ScanTmp {
+    int next, left;
+    unsigned epoch, pad;
+    unsigned long long word[1];
+};
+
 struct Batch;  // host object, engine.cu
 
 // All device pointers of a batch, passed by value to kernels.
@@ -380,9 +388,9 @@ struct Dev {
     ContactStore c_old, c_new;
     int *n_edges_old, *n_edges_new, *n_contacts_old, *n_contacts_new;
     // merge scratch
-    int *surv, *surv_scan, *unm, *unm_scan, *pair_edge, *edge_src, *edge_pair, *edge_cnt;
+    int *surv, *surv_scan, *unm, *unm_scan, *edge_src, *edge_pair, *edge_cnt;
     int *edge_live, *edge_row;     // islands: live contacts per edge, first row of an emitted edge
-    int *scan_tmp;
+    ScanTmp* scan_tmp;
     // islands
     int* adj_ofs;                  // per body CSR offsets (scratch)
     int* adj_list;                 // other endpoint | edge index (scratch, 2 ints per entry)

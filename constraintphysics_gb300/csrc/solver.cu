@@ -395,10 +395,6 @@ __device__ void island_finish(const Dev& d, int rs, int rc, int bs, int bc, cons
 // largest first; the smaller ones a thread each (the two paths give identical
 // results, so the threshold is a pure schedule choice)
 
-__global__ void k_sched_reset(Dev d) {
-    if (threadIdx.x < 96) d.sched[threadIdx.x] = 0;
-}
-
 // sched[kLongIslands]: islands of at least 2^kLongBucket rows
 constexpr int kLongIslands = 4, kLongBucket = 9;
 // islands of kMidRows to kMidMax rows below the big ones: sched[kMidIslands];
@@ -1400,7 +1396,6 @@ void prepare_pgs(int dv_cap) {
 }
 
 void launch_pgs_schedule(const Dev& d, const Launch& L) {
-    k_sched_reset<<<1, 96, 0, L.st>>>(d);
     k_sched_count<<<L.n_sms * 2, 256, 0, L.st>>>(d);
     k_sched_place<<<L.n_sms * 2, 256, 0, L.st>>>(d);
 }
