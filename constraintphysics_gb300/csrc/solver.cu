@@ -519,12 +519,14 @@ __device__ __forceinline__ bool ring_wait(uint64_t* bar, uint32_t parity, long l
 // halves the loads, dot products and updates, and leaves the registers to
 // load the next row while the current one is solved.  A lane keeps its body
 // while consecutive rows share it, whichever side of the row it is on; the Δv
-// of a body that changes is read one row ahead.  A row's code has no branch (a
-// branch costs a lone warp ~40 cycles), and the whole warp runs it, even lanes
+// of a body that changes is read one row ahead.  A row's code has no branch but a
+// uniform one for rows that slide (any other costs a lone warp ~40 cycles), and
+// the whole warp runs it, even lanes
 // as lane 0 and odd lanes as lane 1 (same addresses, same values): two lanes
 // inside a branch would check for divergence at every shuffle (404 cycles per
-// row-step against 307).  Measured on a chain of 2,000 rows: 459 -> 274 cycles
-// per row-step; of 90 rows (held in shared memory): 523 -> 265.
+// row-step against 307).  Measured on a chain of 2,000 rows: 459 -> 233 cycles
+// per row-step where contacts stick, 252 with 28 % of them sliding, 304 where all
+// slide; of 90 rows (held in shared memory) with 28 %: 523 -> 253.
 
 struct HalfRow {
     float2 j[9];     // J of the normal and friction rows (u, w) for the lane's body, three component pairs each
@@ -628,16 +630,28 @@ __device__ __forceinline__ void half_vel(HalfRow& h, P3& v, int& stat) {
     float2 nf = __ffma2_rn(bc2(-diff), make_float2(h.nrm.z, h.nrm.w), A);
     const float mx = __fmul_rn(h.tgt.w, ix);
     const float s2 = __fmaf_rn(nf.x, nf.x, __fmul_rn(nf.y, nf.y));
-    // selected, not branched over: a branch costs a single warp more than the
-    // rsqrt it would save
+    // The clamp's rsqrt is ~49 cycles of dependent work: the row goes on as if
+    // it stuck, and is put right where it slides.  The vote makes that branch a
+    // uniform one (a branch on a lane's own condition costs a lone warp ~40
+    // cycles more).
+    const float2 old = make_float2(h.imp.z, h.imp.w);
     const bool slide = s2 > __fmul_rn(mx, mx);
-    const float2 cl = __fmul2_rn(nf, bc2(__fmul_rn(mx, rsqrtf(s2))));
-    nf = make_float2(slide ? cl.x : nf.x, slide ? cl.y : nf.y);
-    stat = slide ? 0 : 1;
-    float2 e = psub(nf, make_float2(h.imp.z, h.imp.w));
+    float2 e = psub(nf, old);
     if (!(fabsf(e.x) > kZero || fabsf(e.y) > kZero)) e = make_float2(0.f, 0.f);
-    half_axpy1(v, h.m + 3, e.x);
-    half_axpy1(v, h.m + 6, e.y);
+    P3 w = v;
+    half_axpy1(w, h.m + 3, e.x);
+    half_axpy1(w, h.m + 6, e.y);
+    stat = 1;
+    if (__any_sync(0xffffffffu, slide)) {
+        stat = 0;
+        nf = __fmul2_rn(nf, bc2(__fmul_rn(mx, rsqrtf(s2))));
+        e = psub(nf, old);
+        if (!(fabsf(e.x) > kZero || fabsf(e.y) > kZero)) e = make_float2(0.f, 0.f);
+        w = v;
+        half_axpy1(w, h.m + 3, e.x);
+        half_axpy1(w, h.m + 6, e.y);
+    }
+    v = w;
     h.imp.x = ix;
     h.imp.z = __fadd_rn(h.imp.z, e.x);
     h.imp.w = __fadd_rn(h.imp.w, e.y);
