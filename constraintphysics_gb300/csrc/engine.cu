@@ -673,7 +673,7 @@ struct Batch {
     // (+2 per substep and 1 factorisation with joints)
     int launches_per_step() const {
         return 1 + 3 + 2 + (prims ? 3 : 0) + ((meshes || unions) ? 1 : 0) + (3 + 3) + (2 + 1) + 2 + 5 * substeps + 1 + (joints ? 2 * substeps : 0) +
-               (systems ? 1 : 0) + (audit ? 1 : 0) + (springs ? substeps : 0) + (tiles ? (all_tiles ? 6 : 8) : 0) +
+               (systems ? 1 : 0) + (audit ? 1 : 0) + (springs ? substeps : 0) + (tiles ? (all_tiles ? 6 : 8) : 0) + (d[0].has_sleep ? 1 : 0) +
                (max_world > dv_cap ? substeps : 0);
     }
 
@@ -1356,7 +1356,7 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
         if (has_sleep) {
             x.has_sleep = 1;
             x.hist_cap = hist_cap;
-            x.asleep = A.take<int>(N); x.waking = A.take<int>(N); x.ready_cnt = A.take<int>(N);
+            x.asleep = A.take<int>(N); x.wakes = A.take<int>(worlds.size()); x.waking = A.take<int>(N); x.ready_cnt = A.take<int>(N);
             x.non_sleepy = A.take<int>(N); x.hist_n = A.take<int>(N); x.hist_head = A.take<int>(N);
             x.hist = A.take<float>((size_t)N * hist_cap * 6);
         }

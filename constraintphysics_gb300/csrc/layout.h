@@ -444,6 +444,7 @@ struct Dev {
     int has_sleep, hist_cap;
     int* asleep;
     int* waking;
+    int* wakes;                    // per world: 1 when a body of it is waking (set at the start of a step)
     int* ready_cnt;
     int* non_sleepy;
     int* hist_n;
