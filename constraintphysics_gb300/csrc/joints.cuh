@@ -57,11 +57,6 @@ __device__ __forceinline__ void jl_load(const JointRow& R, int lane, JointLane& 
     L.ptarget = R.ptarget[i];
     L.acc = R.impulse[i];
     L.pacc = R.pimpulse[i];
-#pragma unroll
-    for (int k = 0; k < 6; k++) {
-        L.minv[k] = k < L.n ? L.minv[k] : 0.f;
-        L.it[k] = k < L.n ? L.it[k] : 0.f;
-    }
 }
 // Δv of a body for `which`; `zero` (six floats) for infinite mass
 __device__ __forceinline__ void jl_dv(const float4* dv, const float* zero, int slot, int which, float* o) {
@@ -102,7 +97,7 @@ __device__ __forceinline__ void jl_step(const JointLane& L, JointRow& R, float4*
         x = __fmaf_rn(va[k], L.ja[k], x);
         y = __fmaf_rn(vb[k], L.jb[k], y);
     }
-    const float delta = lane < L.n ? __fsub_rn(pseudo ? L.ptarget : L.target, __fadd_rn(x, y)) : 0.f;
+    const float delta = __fsub_rn(pseudo ? L.ptarget : L.target, __fadd_rn(x, y));
     const float acc = pseudo ? L.pacc : L.acc;
     float s = 0.f;
 #pragma unroll

@@ -194,12 +194,9 @@ constexpr int kDvF4 = 3;
 // PistonConstraint (1, bounded by the max torque or force, with a velocity
 // target); row-major, sized for n = 6.
 constexpr int kJMax = 6;
+// Dofs beyond the row's stay zero (the rows are zeroed when a batch is made and
+// a joint's dof count never changes), so the solver may run over all six.
 struct alignas(16) JointRow {
-    float ja[kJMax * 6], jb[kJMax * 6];     // [n][6]
-    float ita[6 * kJMax], itb[6 * kJMax];   // [6][n]
-    float minv[kJMax * kJMax];
-    float target[kJMax], ptarget[kJMax];
-    float impulse[kJMax], pimpulse[kJMax], holo[kJMax];
     int n, sa, sb;                          // island body slots (-1: infinite mass)
     int proj;                               // 0 none, 1 impulse >= 0, 2 impulse <= 0 (limits),
                                             // 3 x > 0 ? min(x, lim) : max(x, -lim) (motor, piston)
@@ -207,6 +204,11 @@ struct alignas(16) JointRow {
     float vt;                               // motor / piston: target = vt - value
     int has_vt;
     int pos;                                // needsPosCorrect: solved in the position passes
+    float ja[kJMax * 6], jb[kJMax * 6];     // [n][6]
+    float ita[6 * kJMax], itb[6 * kJMax];   // [6][n]
+    float minv[kJMax * kJMax];
+    float target[kJMax], ptarget[kJMax];
+    float impulse[kJMax], pimpulse[kJMax], holo[kJMax];
     float itv[kJMax * kJMax];               // J M^-1 J^T (the solver passes read only what comes before)
 };
 constexpr int kJointStage = 880;            // bytes of a row the solver passes use, up to a multiple of 16

@@ -1089,6 +1089,123 @@ __device__ __noinline__ void holo_system(const Dev& d, int s, HoloSm& sm, bool r
     }
 }
 
+// A pass over an island held in shared memory (`list`: each row's joint slot, -1
+// a contact row, which lane 0 runs from global memory).  KIND 0: warm start, 1:
+// velocity, 2: position.  The same steps as jl_warm / jl_step with everything
+// typed as shared memory and only the pass's own fields loaded: a joint row is
+// bound by its instruction count on one warp (168 a row-step through generic
+// pointers) and its dependency chain.
+struct JointRes {
+    int n, sa, sb, proj, pos;
+    float lim, ja[6], jb[6], mv[6], it[6], tgt, acc;
+};
+template <int KIND>
+__device__ __forceinline__ void jr_load(const uint8_t* row, int lane, JointRes& L) {
+    const JointRow& R = *reinterpret_cast<const JointRow*>(row);
+    const int i = min(lane, 5), c = min(lane, 11);
+    const int4 h = *reinterpret_cast<const int4*>(&R.n);
+    L.n = h.x; L.sa = h.y; L.sb = h.z; L.proj = h.w;
+    jl_row6(R.ita + kJMax * c, L.it);   // body b's follow body a's
+    if (KIND == 0) {
+        L.acc = R.impulse[i];
+        return;
+    }
+    L.lim = R.lim;
+    L.pos = R.pos;
+    jl_row6(R.ja + 6 * i, L.ja);
+    jl_row6(R.jb + 6 * i, L.jb);
+    jl_row6(R.minv + kJMax * i, L.mv);
+    L.tgt = KIND == 1 ? R.target[i] : R.ptarget[i];
+    L.acc = KIND == 1 ? R.impulse[i] : R.pimpulse[i];
+}
+__device__ __forceinline__ const float* jr_dv(const float4* dv, const float* zero, int slot, int which) {
+    return slot < 0 ? zero : reinterpret_cast<const float*>(dv + kDvF4 * slot) + 6 * which;
+}
+template <int KIND>
+__device__ __forceinline__ void jr_row(const JointRes& L, uint8_t* row, float4* dv, const float* zero, int lane) {
+    constexpr int which = KIND == 2 ? 1 : 0;
+    if (KIND == 2 && !L.pos) return;   // needsPosCorrect
+    const int slot = lane < 6 ? L.sa : L.sb, comp = lane < 6 ? lane : min(lane, 11) - 6;
+    const float old = jr_dv(dv, zero, slot, which)[comp];
+    float imp;
+    if (KIND == 0) {
+        imp = L.acc;
+    } else {
+        float va[6], vb[6];
+        jl_row6(jr_dv(dv, zero, L.sa, which), va);
+        jl_row6(jr_dv(dv, zero, L.sb, which), vb);
+        float x = 0.f, y = 0.f;
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+            x = __fmaf_rn(va[k], L.ja[k], x);
+            y = __fmaf_rn(vb[k], L.jb[k], y);
+        }
+        const float delta = __fsub_rn(L.tgt, __fadd_rn(x, y));
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < 6; k++) s = __fmaf_rn(__shfl_sync(0xffffffffu, delta, k), L.mv[k], s);
+        float nw = __fadd_rn(L.acc, s);
+        if (__any_sync(0xffffffffu, L.proj != 0)) {   // rows of one dof
+            if (L.proj == 1) nw = fmaxf(nw, 0.f);
+            else if (L.proj == 2) nw = fminf(nw, 0.f);
+            else nw = nw > 0.f ? fminf(nw, L.lim) : fmaxf(nw, -L.lim);
+        }
+        imp = __fsub_rn(nw, L.acc);
+        if (lane >= L.n) imp = 0.f;   // a projection's value beyond the row's one dof
+    }
+    if (__any_sync(0xffffffffu, fabsf(imp) > kJZero)) {
+        float x = 0.f;
+#pragma unroll
+        for (int k = 0; k < 6; k++) x = __fmaf_rn(__shfl_sync(0xffffffffu, imp, k), L.it[k], x);
+        if (lane < 12 && slot >= 0) const_cast<float*>(jr_dv(dv, zero, slot, which))[comp] = __fadd_rn(old, x);
+        if (KIND != 0 && lane < L.n) {
+            JointRow& R = *reinterpret_cast<JointRow*>(row);
+            (KIND == 1 ? R.impulse : R.pimpulse)[lane] = __fadd_rn(L.acc, imp);
+        }
+    }
+    __syncwarp();
+}
+template <int KIND>
+__device__ __forceinline__ void jr_pass(uint8_t* srows, const int16_t* list, RowBlock* rows, int rc, float4* dv, const float* zero,
+                                        int lane) {
+    JointRes A, B;
+    int c = list[0], n = list[min(1, rc - 1)], r = 0;
+    jr_load<KIND>(srows + max(c, 0) * kJointStage, lane, A);
+    auto one = [&](JointRes& L, JointRes& N) {
+        jr_load<KIND>(srows + max(n, 0) * kJointStage, lane, N);
+        const int n2 = list[min(r + 2, rc - 1)];
+        if (__any_sync(0xffffffffu, c >= 0)) {
+            jr_row<KIND>(L, srows + c * kJointStage, dv, zero, lane);
+        } else {
+            if (lane == 0) {
+                RowBlock& R = rows[r];
+                float4 imp = R.imp;
+                if (KIND == 0) {
+                    row_warm(R, imp, dv);
+                } else if (KIND == 1) {
+                    int st = R.stat;
+                    row_vel(R, imp, st, dv);
+                    R.imp = imp;
+                    R.stat = st;
+                } else {
+                    row_pos(R, imp, dv);
+                    R.imp = imp;
+                }
+            }
+            __syncwarp();
+        }
+        c = n;
+        n = n2;
+        r++;
+    };
+    while (true) {
+        one(A, B);
+        if (r >= rc) break;
+        one(B, A);
+        if (r >= rc) break;
+    }
+}
+
 // Islands with joint rows: one warp per island, contact rows and joint rows in
 // island order, then the island's holonomic systems (first substep).  A joint
 // row is spread over the lanes (joints.cuh), a contact row runs on lane 0.
@@ -1132,7 +1249,7 @@ __global__ void __launch_bounds__(32, 3) k_pgs_joint(Dev d, int first) {
         float4* err = d.dv_err + kDvF4 * (size_t)bs;
         // the island's joint rows into shared memory, if they fit
         int held = 0;
-        bool res = rc <= kJointList;
+        bool res = rc <= kJointList && bc <= kJointDv;
         for (int base = 0; res && base < rc; base += 32) {
             const bool in = base + lane < rc;
             const int c = in ? d.rows[rs + base + lane].contact : 0;
@@ -1170,6 +1287,7 @@ __global__ void __launch_bounds__(32, 3) k_pgs_joint(Dev d, int first) {
                 return;
             }
         }
+        const int n_vel = P.pgs_vel, n_pos = P.pgs_pos;   // read once: the row stores could alias P
         // the island's row r: its joint row, or null for a contact row
         auto joint_of = [&](int r) -> JointRow* {
             if (res) return list[r] < 0 ? nullptr : reinterpret_cast<JointRow*>(srows + list[r] * kJointStage);
@@ -1179,7 +1297,7 @@ __global__ void __launch_bounds__(32, 3) k_pgs_joint(Dev d, int first) {
         // one pass over the rows: joint(lane row, joint row) or contact(row)
         // for each, the next joint row loaded one row ahead
         auto pass = [&](auto&& joint, auto&& contact) {
-            JointRow* any = res ? reinterpret_cast<JointRow*>(srows) : d.jt.rows;   // loaded in the place of a contact row
+            JointRow* any = d.jt.rows;   // loaded in the place of a contact row
             JointRow *c = joint_of(0), *n = joint_of(min(1, rc - 1));
             JointLane A, B;
             jl_load(c ? *c : *any, lane, A);
@@ -1201,34 +1319,39 @@ __global__ void __launch_bounds__(32, 3) k_pgs_joint(Dev d, int first) {
             }
             __syncwarp();
         };
-        const int n_vel = P.pgs_vel, n_pos = P.pgs_pos;   // read once: the row stores could alias P
-        pass([&](const JointLane& L, JointRow&) { jl_warm(L, dv, lane); },
-             [&](RowBlock& R) {
-                 if (lane == 0) row_warm(R, R.imp, dv);
-                 __syncwarp();
-             });
-        for (int it = 0; it < n_vel; it++)
-            pass([&](const JointLane& L, JointRow& R) { jl_step(L, R, dv, zero, false, lane); },
+        if (res) {
+            jr_pass<0>(srows, list, d.rows + rs, rc, sdv, zero, lane);
+            for (int it = 0; it < n_vel; it++) jr_pass<1>(srows, list, d.rows + rs, rc, sdv, zero, lane);
+            for (int it = 0; it < n_pos; it++) jr_pass<2>(srows, list, d.rows + rs, rc, sdv, zero, lane);
+        } else {
+            pass([&](const JointLane& L, JointRow&) { jl_warm(L, dv, lane); },
                  [&](RowBlock& R) {
-                     if (lane == 0) {
-                         float4 imp = R.imp;
-                         int st = R.stat;
-                         row_vel(R, imp, st, dv);
-                         R.imp = imp;
-                         R.stat = st;
-                     }
+                     if (lane == 0) row_warm(R, R.imp, dv);
                      __syncwarp();
                  });
-        for (int it = 0; it < n_pos; it++)
-            pass([&](const JointLane& L, JointRow& R) { if (L.pos) jl_step(L, R, dv, zero, true, lane); },   // needsPosCorrect
-                 [&](RowBlock& R) {
-                     if (lane == 0) {
-                         float4 imp = R.imp;
-                         row_pos(R, imp, dv);
-                         R.imp = imp;
-                     }
-                     __syncwarp();
-                 });
+            for (int it = 0; it < n_vel; it++)
+                pass([&](const JointLane& L, JointRow& R) { jl_step(L, R, dv, zero, false, lane); },
+                     [&](RowBlock& R) {
+                         if (lane == 0) {
+                             float4 imp = R.imp;
+                             int st = R.stat;
+                             row_vel(R, imp, st, dv);
+                             R.imp = imp;
+                             R.stat = st;
+                         }
+                         __syncwarp();
+                     });
+            for (int it = 0; it < n_pos; it++)
+                pass([&](const JointLane& L, JointRow& R) { if (L.pos) jl_step(L, R, dv, zero, true, lane); },   // needsPosCorrect
+                     [&](RowBlock& R) {
+                         if (lane == 0) {
+                             float4 imp = R.imp;
+                             row_pos(R, imp, dv);
+                             R.imp = imp;
+                         }
+                         __syncwarp();
+                     });
+        }
         if (first && P.pgs_holo > 0) {
             const int ss = d.g_isl_sys_start[i], sn = d.g_isl_sys_count[i];
             for (int it = 0; it < P.pgs_holo; it++)
