@@ -563,6 +563,8 @@ __global__ void k_springs(Dev d) {
     }
 }
 
+constexpr int kFactorBytes = 40 * 1024;   // blocks held in shared memory by k_holo_factor
+
 // computeBlockInitialValue (HolonomicBlockSolver.cpp:731-760)
 template <class T>
 __device__ void initial_block(const Dev& d, int j1, int j2, T* t, float cfm) {
@@ -591,18 +593,63 @@ __device__ void initial_block(const Dev& d, int j1, int j2, T* t, float cfm) {
     }
 }
 
-// One warp per system: the column loop stays in order (each column needs the
-// previous columns' updates); within a column the diagonal block is inverted
-// by lane 0 and the entries of the L blocks and of the trailing updates are
-// spread over the lanes, each entry summed in the same order as a serial
-// loop would.
+__device__ __forceinline__ double neg_fma(double a, double b, double c) { return __fma_rn(-a, b, c); }
+__device__ __forceinline__ float neg_fma(float a, float b, float c) { return __fmaf_rn(-a, b, c); }
+// invert_block by a warp for n >= 4 (the smaller closed forms run on lane 0):
+// the Gauss-Jordan steps of block and identity, an entry per lane, each the
+// same operations as there; `c`: 2 n^2 values of shared memory
 template <class T>
-__device__ void factorise(const Dev& d, int s, T* B, float cfm, int lane) {
+__device__ void invert_block_warp(int n, T* m, T* c, int lane) {
+    if (n < 4) {
+        if (lane == 0) invert_block<T>(n, m);
+        return;
+    }
+    const int w = 2 * n, E = n * w;
+    for (int e = lane; e < E; e += 32) {
+        const int r = e / w, k = e - r * w;
+        c[e] = k < n ? m[n * r + k] : (k - n == r ? T(1) : T(0));
+    }
+    __syncwarp();
+    for (int piv = 0; piv < n; piv++) {
+        const T rp = T(1) / c[w * piv + piv];
+        T nv[3];
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const int e = lane + 32 * q;
+            if (e >= E) continue;
+            const int r = e / w, k = e - r * w;
+            nv[q] = r == piv ? c[e] : neg_fma(c[w * r + piv] * rp, c[w * piv + k], c[e]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+            if (lane + 32 * q < E) c[lane + 32 * q] = nv[q];
+        __syncwarp();
+    }
+    for (int e = lane; e < n * n; e += 32) {
+        const int r = e / n, k = e - r * n;
+        m[e] = c[w * r + n + k] * (T(1) / c[w * r + r]);
+    }
+}
+
+// One warp per system: the column loop stays in order (each column needs the
+// previous columns' updates); within a column the diagonal block's inverse and
+// the entries of the L blocks and of the trailing updates are spread over the
+// lanes, each entry summed in the same order as a serial loop would.  Bound by
+// the chain of columns, each a few dependent loads and FP64 operations: the
+// blocks stay in shared memory until the end where they fit (512 systems of 16
+// to 64 constraints: 737 us with the blocks in global memory and lane 0
+// inverting, now 315).
+template <class T>
+__device__ void factorise(const Dev& d, int s, T* Bg, T* sh, float cfm, int lane) {
     const HoloStore& hs = d.hs;
     const int c0 = hs.cstart[s], n = hs.cstart[s + 1] - c0;
     const int* cons = hs.cons + c0;
     const int* table = hs.table + hs.tstart[s];
     const int* ls = hs.lstart + hs.lbase[s];   // column col's blocks below the diagonal: [ls[col], ls[col + 1])
+    T* scratch = sh;                      // invert_block_warp's
+    const bool fits = (hs.cap[s] + kJMax * hs.degree[s]) * (int)sizeof(T) <= kFactorBytes;
+    T* B = fits ? sh + 2 * kJMax * kJMax : Bg;
     T* Dg = B + hs.cap[s];
     for (int col = lane; col < n; col += 32) {
         initial_block<T>(d, cons[col], cons[col], B + holo_loc(table, n, col, col), cfm);
@@ -612,7 +659,7 @@ __device__ void factorise(const Dev& d, int s, T* B, float cfm, int lane) {
     for (int col = 0; col < n; col++) {
         const int w = d.jt.rows[cons[col]].n;
         T* diag = B + holo_loc(table, n, col, col);
-        if (lane == 0) invert_block<T>(w, diag);
+        invert_block_warp<T>(w, diag, scratch, lane);
         __syncwarp();
         if (col + 1 == n) break;
         const int q0 = ls[col], q1 = ls[col + 1];
@@ -652,15 +699,20 @@ __device__ void factorise(const Dev& d, int s, T* B, float cfm, int lane) {
         }
         __syncwarp();
     }
+    if (fits) {
+        for (int k = lane; k < hs.cap[s]; k += 32) Bg[k] = B[k];
+        __syncwarp();
+    }
 }
 
 __global__ void __launch_bounds__(32) k_holo_factor(Dev d) {
+    extern __shared__ __align__(16) double fac_sm[];
     const int lane = threadIdx.x;
     for (int s = blockIdx.x; s < d.hs.n; s += gridDim.x) {
         const int j0 = d.hs.cons[d.hs.cstart[s]];
         const float cfm = d.wparams[d.world[d.jt.b1[j0]]].cfm;
-        if (d.hs.fp64[s]) factorise<double>(d, s, d.hs.pool64 + d.hs.bstart[s], cfm, lane);
-        else factorise<float>(d, s, d.hs.pool32 + d.hs.bstart[s], cfm, lane);
+        if (d.hs.fp64[s]) factorise<double>(d, s, d.hs.pool64 + d.hs.bstart[s], fac_sm, cfm, lane);
+        else factorise<float>(d, s, d.hs.pool32 + d.hs.bstart[s], reinterpret_cast<float*>(fac_sm), cfm, lane);
     }
 }
 
@@ -682,7 +734,7 @@ void launch_joint_rows(const Dev& d, bool first, const Launch& L) {
         // a warp per system
         int gs = d.hs.n;
         gs = gs > L.n_sms * 32 ? L.n_sms * 32 : gs;
-        k_holo_factor<<<gs, 32, 0, L.st>>>(d);
+        k_holo_factor<<<gs, 32, kFactorBytes + 2 * kJMax * kJMax * 8, L.st>>>(d);
     }
 }
 
