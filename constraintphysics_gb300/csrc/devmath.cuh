@@ -7,6 +7,16 @@
 
 namespace cpgpu {
 
+// The first item of this thread in a loop over n items that steps by all of
+// the grid's threads.  Few items (one for each of the grid's first `warps`
+// warps) go to a warp each: the lanes of a warp with 32 divergent items wait for
+// one another.
+__device__ __forceinline__ int first_item(int n, int warps) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n > warps) return t;
+    return (t & 31) == 0 ? t >> 5 : n;
+}
+
 struct f3 { float x, y, z; };
 struct M33 { float m[9]; };  // row-major
 

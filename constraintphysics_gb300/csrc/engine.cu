@@ -647,7 +647,7 @@ struct Batch {
         launch_pairs(x, L);        mark(2);
         launch_narrowphase(x, slot_bytes, n_sms, prims, br, st); mark(3);   // + mesh pairs
         launch_merge(x, L);        mark(4);
-        launch_islands(x, isl_smem, L);
+        launch_islands(x, max_world, isl_smem, L);
         launch_pgs_schedule(x, L); mark(5);
     }
     void launch_step(const Dev& x) {

@@ -127,10 +127,11 @@ __global__ void k_place(Dev d, const int* cnt) {
 }
 
 // per new edge: surviving old contacts (in order), then this step's manifold
-// points matched by MagicID or appended
+// points matched by MagicID or appended; a warp each for up to 2,432 edges
+// (60 small worlds 20 -> 14 us)
 __global__ void k_contacts(Dev d, int write) {
     const int ne = *d.n_edges_new;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += gridDim.x * blockDim.x) {
+    for (int e = first_item(ne, gridDim.x * blockDim.x >> 5); e < ne; e += gridDim.x * blockDim.x) {
         int ids[kMaxEdgeContacts];
         signed char upd[kMaxEdgeContacts];
         uint64_t mags[kMaxEdgeContacts];
@@ -738,7 +739,8 @@ __device__ void islands_big(const Dev& d, const IslandCtx& x, int nb, int ne_w, 
 }
 
 // NT threads a block: 256, or 1,024 for a batch of a few large worlds, whose
-// islands one block each walks through (4.3 -> 1.5 ms on 20,000 bodies)
+// islands one block each walks through (20,000 bodies 4.3 -> 1.5 ms, 1,000
+// bodies 360 -> 327 us; worlds of up to 64 bodies the same with either)
 template <int NT>
 __global__ void __launch_bounds__(NT) k_islands(Dev d, int smem_bytes) {
     extern __shared__ int sm_isl[];
@@ -1075,8 +1077,8 @@ int islands_smem_bytes(int max_bodies) {
     return (int)std::min<long long>(want, kIslandsSmemMax);
 }
 
-void launch_islands(const Dev& d, int smem_bytes, const Launch& L) {
-    if (d.grid_buckets > 0 && d.n_worlds <= L.n_sms) k_islands<1024><<<d.n_worlds, 1024, smem_bytes, L.st>>>(d, smem_bytes);
+void launch_islands(const Dev& d, int max_world, int smem_bytes, const Launch& L) {
+    if (max_world > 256 && d.n_worlds <= L.n_sms) k_islands<1024><<<d.n_worlds, 1024, smem_bytes, L.st>>>(d, smem_bytes);
     else k_islands<256><<<d.n_worlds, 256, smem_bytes, L.st>>>(d, smem_bytes);
     launch_scan<IslandScan>(d, nullptr, d.n_worlds, d.n_worlds, L);
     k_island_copy<<<grid_for(d.n_bodies, 128, L.n_sms), 128, 0, L.st>>>(d);

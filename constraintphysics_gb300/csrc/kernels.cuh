@@ -47,7 +47,7 @@ constexpr int kIslandsSmemMax = 160 * 1024;
 // k_islands' dynamic shared memory for worlds of up to `max_bodies` bodies
 // (sets the kernel's limit); worlds that need more run from global memory
 int islands_smem_bytes(int max_bodies);
-void launch_islands(const Dev& d, int smem_bytes, const Launch& L);
+void launch_islands(const Dev& d, int max_world, int smem_bytes, const Launch& L);
 // per-world edge / contact ranges of the current graph (4 ints per world)
 void launch_world_ranges(const Dev& d, const int* worlds, int n, int* out, cudaStream_t st);
 void launch_rows(const Dev& d, int first, int last, const Launch& L);

@@ -1720,6 +1720,10 @@ __global__ void __launch_bounds__(256) k_narrowphase(Dev d, int slot_bytes) {
 // CollisionDetect.cpp:237-280), clipping (:394-620) and the 4-direction cull
 // (:2795-2830).  The clip is serial per pair; a thread each keeps all lanes of
 // a warp busy on 32 pairs, where a warp per pair would idle 31.
+// A few pairs (one for every fourth warp of the grid, 2,432 here) go to a warp
+// each: 1,800 pairs of 60 worlds 62 -> 31 us; with 14,000 pairs dealt to as many
+// warps 60 -> 76, so more take a thread each.
+
 // the contact points of two hulls along the axis n (depth bp) between the
 // features `feat`, before the cull; returns their count
 __device__ int clip_hulls(const HullG& A, const HullG& B, f3 n, float bp, int2 feat, Scratch& scratch, CP* clipped, int* status,
@@ -1744,7 +1748,7 @@ __global__ void __launch_bounds__(128) k_clip(Dev d) {
     const int n_pairs = *d.n_pairs;
     Scratch scratch;
     CP clipped[kMaxClip];
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n_pairs; p += gridDim.x * blockDim.x) {
+    for (int p = first_item(n_pairs, (gridDim.x * blockDim.x >> 5) / 4); p < n_pairs; p += gridDim.x * blockDim.x) {
         const float4 nn = d.mf_n[p];
         if (!(nn.w > 0.f)) continue;
         const int a = d.pair_a[p], b = d.pair_b[p];
