@@ -740,7 +740,7 @@ __device__ void islands_big(const Dev& d, const IslandCtx& x, int nb, int ne_w, 
 
 // NT threads a block: 256, or 1,024 for a batch of a few large worlds, whose
 // islands one block each walks through (20,000 bodies 4.3 -> 1.5 ms, 1,000
-// bodies 360 -> 327 us; worlds of up to 64 bodies the same with either)
+// bodies 360 -> 306 us; worlds of up to 64 bodies the same with either)
 template <int NT>
 __global__ void __launch_bounds__(NT) k_islands(Dev d, int smem_bytes) {
     extern __shared__ int sm_isl[];
@@ -749,8 +749,8 @@ __global__ void __launch_bounds__(NT) k_islands(Dev d, int smem_bytes) {
     const int w = blockIdx.x;
     const int s = d.world_start[w], e = d.world_start[w + 1];
     const int ne = *d.n_edges_new, ncon = *d.n_contacts_new;
-    // the batch's first and last world need no search (one world alone: a chain
-    // of loads less, 1 us of a 15-body world's 20, 8 of 2,400 bodies' 64)
+    // the batch's first and last world need no search (a chain of loads; a step of
+    // one world of 2,400 bodies 425 -> 419 us)
     const int e0 = s == 0 ? 0 : lower_bound_u64(d.e_new.key, ne, (uint64_t)s << 32);
     const int e1 = e == d.n_bodies ? ne : lower_bound_u64(d.e_new.key, ne, (uint64_t)e << 32);
     const int c0 = (e0 < ne) ? d.e_new.cstart[e0] : ncon;

@@ -52,8 +52,9 @@ void launch_islands(const Dev& d, int max_world, int smem_bytes, const Launch& L
 void launch_world_ranges(const Dev& d, const int* worlds, int n, int* out, cudaStream_t st);
 void launch_rows(const Dev& d, int first, int last, const Launch& L);
 // PGS: islands are split by size after the island pass (largest first); large
-// islands run one warp each with rows streamed through shared memory, small
-// ones one thread each on the `side` stream, concurrently.
+// islands run one warp each with rows streamed through shared memory, middling
+// ones one warp each with all rows there (side2) and small ones one thread each
+// (side), concurrently.
 void launch_pgs_schedule(const Dev& d, const Launch& L);
 void prepare_pgs(int dv_cap);
 int pgs_big_smem_bytes(int dv_cap);

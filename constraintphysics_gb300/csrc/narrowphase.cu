@@ -2145,7 +2145,7 @@ int mesh_scratch_warps(int n_sms) { return n_sms * kMeshBlocksPerSm * 8; }
 
 // ---- ray queries ------------------------------------------------------------------
 // PhysicsEngine::raycastFirstIntersection (PhysicsEngine.cpp:582-609) for one
-// ray per thread against the bodies [s, e) of one world: every body whose
+// ray per block against the bodies [s, e) of one world: every body whose
 // current AABB the ray crosses is tested with its primitive's ray test, the
 // nearest hit wins (strictly nearer replaces, in body order).
 namespace {
