@@ -71,10 +71,17 @@ RACE_FIX = (
 )
 
 
+def source_dirs(root):
+    return os.path.join(root, "ConstraintPhysics", "src"), os.path.join(root, "Math", "src")
+
+
+def has_sources(root):
+    return all(os.path.isdir(d) for d in source_dirs(root))
+
+
 def stage(ref_root):
-    src_engine = os.path.join(ref_root, "ConstraintPhysics", "src")
-    src_math = os.path.join(ref_root, "Math", "src")
-    if not (os.path.isdir(src_engine) and os.path.isdir(src_math)):
+    src_engine, src_math = source_dirs(ref_root)
+    if not has_sources(ref_root):
         raise SystemExit(f"reference sources not found under {ref_root}")
     out_src = os.path.join(DEST, "src")
     if os.path.isdir(out_src):
@@ -127,13 +134,15 @@ DEFAULT_REFERENCE_ROOT = "/root/reference"
 
 
 def reference_root():
-    """The reference checkout to stage from: $CONSTRAINTPHYSICS_REFERENCE, else
-    the default checkout location; None when neither is a directory (a
-    machine that only has the staged copy)."""
-    for root in (os.environ.get("CONSTRAINTPHYSICS_REFERENCE"), DEFAULT_REFERENCE_ROOT):
-        if root and os.path.isdir(root):
-            return root
-    return None
+    """The reference checkout to stage from: $CONSTRAINTPHYSICS_REFERENCE (a
+    directory without the sources there is an error when it is staged), else
+    the default checkout location; None when the variable names no directory
+    and the default location is absent or empty (a machine that only has the
+    staged copy, or neither)."""
+    root = os.environ.get("CONSTRAINTPHYSICS_REFERENCE")
+    if root and os.path.isdir(root):
+        return root
+    return DEFAULT_REFERENCE_ROOT if has_sources(DEFAULT_REFERENCE_ROOT) else None
 
 
 if __name__ == "__main__":
