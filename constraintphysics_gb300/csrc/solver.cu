@@ -582,11 +582,6 @@ template <bool SH>
 __device__ __forceinline__ P3 dv_load(const float4* dv, int slot, int which) {
     return SH ? dv_get_z(dv, slot, which) : dv_get(dv, slot, which);
 }
-template <bool SH>
-__device__ __forceinline__ void dv_store(float4* dv, int slot, int which, const P3& v) {
-    if (SH) dv_put_z(dv, slot, which, v);
-    else dv_put(dv, slot, which, v);
-}
 // the same by scalar FMAs: no broadcast of s into a register pair, which the
 // chain would wait for
 __device__ __forceinline__ void half_axpy1(P3& v, const float2* m, float s) {
@@ -725,7 +720,9 @@ struct RowFeed {
 // after the last one) is loaded while the row is solved, without a branch in a
 // row's code.  Impulses go to `out`; `fin`: also there (KIND 3).
 // SH: `dv` is in shared memory with a zero entry at index -1 for the bodies of
-// infinite mass (their M^-1 J^T is zero, so it stays zero).
+// infinite mass.  The entry is never written and every row reads it anew: M^-1 J^T
+// is zero there, but zero times an overflowing impulse is NaN, and the entry
+// serves every island of the worker.
 struct ChainState {
     P3 v, p;       // Δv and pseudo Δv of the lane's body
     int own;       // its slot
@@ -766,10 +763,10 @@ __device__ __forceinline__ void chain_run(const RowBlock* row, int n, const RowB
             }
             out++;
         }
-        if (kV) dv_store<SH>(dv, c.own, 0, c.v);
-        if (kP) dv_store<SH>(dv, c.own, 1, c.p);
+        if (kV) dv_put(dv, c.own, 0, c.v);
+        if (kP) dv_put(dv, c.own, 1, c.p);
         __syncwarp(0xffffffffu);   // the other lane may read this body next
-        const bool keep = nown == c.own;
+        const bool keep = nown == c.own && nown >= 0;
         if (kV) c.v = psel(keep, c.v, nv);
         if (kP) c.p = psel(keep, c.p, np);
         c.own = nown;
