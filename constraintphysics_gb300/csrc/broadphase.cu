@@ -86,7 +86,7 @@ __device__ __forceinline__ bool in_grid_world(const Dev& d, int i) {
     return d.world_start[w + 1] - d.world_start[w] > kTileWorld;
 }
 __global__ void __launch_bounds__(1024) k_grid_begin(Dev d) {
-    grid_begin(dev_grid(d), d.n_bodies, BodyBox{d.aabb_lo, d.aabb_hi}, [&](int i) { return in_grid_world(d, i); });
+    grid_begin(dev_grid(d), d.n_grid_sample, BodyBox{d.aabb_lo, d.aabb_hi}, [&](int k) { return d.grid_sample[k]; });
 }
 __global__ void __launch_bounds__(256) k_grid_put(Dev d, int pass) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < d.n_bodies; i += gridDim.x * blockDim.x)

@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "hull.hpp"
+#include "gridsample.h"
 #include "kernels.cuh"
 
 extern "C" {
@@ -1013,6 +1014,7 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
     int grid_buckets = 0;
     if (grid_bodies > 0)
         for (grid_buckets = 1024; grid_buckets < grid_bodies / 2 && grid_buckets < (1 << 17);) grid_buckets *= 2;
+    const std::vector<int> grid_sample = grid_samples(wstart, kTileWorld);
     B->tiles = grid_bodies > 0;
     B->all_tiles = grid_bodies == N;
     {
@@ -1369,6 +1371,8 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
             x.grid_bucket = A.take<int>(grid_buckets);
             x.grid_ids = A.take<int>(N); x.grid_far = A.take<int>(N); x.grid_n_far = A.take<int>(1);
             x.grid_inv = A.take<float>(1);
+            x.n_grid_sample = (int)grid_sample.size();
+            x.grid_sample = A.take<int>(grid_sample.size());
         }
         // CPGPU_ISLANDS_SERIAL=1: every world takes the one-thread search (a
         // test compares the searches)
@@ -1514,6 +1518,7 @@ static std::unique_ptr<Batch> build_batch(const std::vector<World*>& worlds, int
     up(d_shape, shape_off.data(), N * 4); up(d_world, world_of.data(), N * 4);
     up(d_mov, movement.data(), N); up(d_mat, mat.data(), N * sizeof(float4));
     up(d_pool, pool.data(), pool.size());
+    if (grid_buckets > 0) up((void*)x.grid_sample, grid_sample.data(), grid_sample.size() * 4);
     up(x.moved, fresh.data(), N * 4);   // the first geometry pass renormalises these orientations
     if (B->unions) {
         up((void*)x.prim_start, prim_start.data(), N * 4); up((void*)x.prim_count, prim_count.data(), N * 4);

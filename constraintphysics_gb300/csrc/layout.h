@@ -351,6 +351,8 @@ struct Dev {
     int grid_buckets, all_grid;
     int *grid_bucket, *grid_ids, *grid_far, *grid_n_far;
     float* grid_inv;
+    int n_grid_sample;
+    const int* grid_sample;        // the bodies that size the grid's cells (gridsample.h)
     // islands of worlds above kTileWorld bodies: one DFS per connected
     // component, the components in parallel (kCompArrays ints per body)
     int isl_serial;                // every world takes the one-thread search (a test compares)

@@ -106,7 +106,8 @@ struct NaWorld {   // one world
 };
 __global__ void __launch_bounds__(1024) k_na_begin(const float* aabbs, int n, NoAllocScratch* s) {
     if (blockIdx.x == 0 && threadIdx.x < kNoAllocMaxBodies / 1024) s->chunk[threadIdx.x] = 0;
-    grid_begin(na_grid(s), n, NaLoad(aabbs), [](int) { return true; });
+    const int step = grid_sample_step(n);
+    grid_begin(na_grid(s), grid_sample_count(n), NaLoad(aabbs), [=](int k) { return k * step; });
 }
 __global__ void __launch_bounds__(256) k_na_put(const float* aabbs, int n, NoAllocScratch* s, int pass) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -6,6 +6,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "gridsample.h"
+
 namespace cpgpu {
 
 // Boxes a warp tests together: each later box is loaded once for all of them.
@@ -127,28 +129,29 @@ __device__ __forceinline__ bool box_cell(const PairBox& b, float inv, PairCell* 
     return true;
 }
 
-// The first block (1,024 threads) sizes the cells from at most 4,096 of the n
-// boxes (`use(i)`: box i counts), the others empty the buckets.  A cell is as
+// The first block (1,024 threads) sizes the cells from the sampled boxes (at most
+// kGridSamples; sample(k): the k-th), the others empty the buckets.  A cell is as
 // wide as the widest box within three times the mean: those boxes are all in
 // the grid (a few hundred outside cost every warp a walk over them: on 20,000
 // mixed bodies 0.48 ms with cells of 1.25 times the mean).
-template <class Id, class Load, class Use>
-__device__ __forceinline__ void grid_begin(const PairGrid<Id>& g, int n, const Load& load, const Use& use) {
+template <class Id, class Load, class Sample>
+__device__ __forceinline__ void grid_begin(const PairGrid<Id>& g, int samples, const Load& load, const Sample& sample) {
     if (blockIdx.x > 0) {
         for (int i = (blockIdx.x - 1) * blockDim.x + threadIdx.x; i < g.buckets; i += (gridDim.x - 1) * blockDim.x) g.bucket[i] = 0;
         return;
     }
     __shared__ float ss[32];
     __shared__ int sm[32];
-    const int step = max(1, n / 4096), lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    float ext[5], sum = 0.f;   // n / step < 4096 + 1024
+    constexpr int kPer = kGridSamples / 1024;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    float ext[kPer], sum = 0.f;
     int m = 0;
 #pragma unroll
-    for (int k = 0; k < 5; k++) {
-        const long long i = (long long)(threadIdx.x + 1024 * k) * step;
+    for (int k = 0; k < kPer; k++) {
+        const int q = threadIdx.x + 1024 * k;
         ext[k] = -1.f;
-        if (i < n && use((int)i)) {
-            const PairBox b = load((int)i);
+        if (q < samples) {
+            const PairBox b = load(sample(q));
             const float e = fmaxf(b.hx - b.lx, fmaxf(b.hy - b.ly, b.hz - b.lz));
             if (box_plain(b) && e < 1e15f) { ext[k] = e; sum += e; m++; }
         }
@@ -162,7 +165,7 @@ __device__ __forceinline__ void grid_begin(const PairGrid<Id>& g, int n, const L
     const float cap = m > 0 ? 3.f * sum / (float)m : 0.f;
     float top = 0.f;
 #pragma unroll
-    for (int k = 0; k < 5; k++) if (ext[k] <= cap) top = fmaxf(top, ext[k]);
+    for (int k = 0; k < kPer; k++) if (ext[k] <= cap) top = fmaxf(top, ext[k]);
     for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
     __syncthreads();
     if (lane == 0) ss[wid] = top;
