@@ -3003,7 +3003,8 @@ int cpgpu_set_joint_state(cpgpu_world* w, const double* impulse, const double* u
 // CPGPU_BATCH_SECOND_SHARE (percent, three or more parts),
 // CPGPU_PGS_REST_PER_SM, CPGPU_PGS_MID_PER_SM (the second part's chain
 // workers per SM, three or more parts) and CPGPU_PGS_BIG_ROWS (the island
-// rows from which an island takes the warp-per-island solver) override it.
+// rows from which an island takes the warp-per-island solver; from 2^20 on
+// every island takes a thread, the middling ones too) override it.
 static std::vector<int> size_order(const std::vector<World*>& ws) {
     std::vector<int> order(ws.size());
     for (size_t i = 0; i < ws.size(); i++) order[i] = (int)i;

@@ -392,19 +392,23 @@ __device__ void island_finish(const Dev& d, int rs, int rc, int bs, int bc, cons
 }
 
 // ---- scheduling: islands with at least d.big_rows rows get a warp each,
-// largest first; the smaller ones a thread each (the two paths give identical
-// results, so the threshold is a pure schedule choice)
+// largest first; middling ones a warp with all their rows in shared memory, the
+// smaller ones a thread each (the three paths give identical results, so the
+// thresholds are pure schedule choices)
 
 // sched[kLongIslands]: islands of at least 2^kLongBucket rows
 constexpr int kLongIslands = 4, kLongBucket = 9;
 // islands of kMidRows to kMidMax rows below the big ones: sched[kMidIslands];
 // from kMidRowsFew rows in a batch of up to kMidFew islands
 constexpr int kMidIslands = 5, kMidRows = 16, kMidMax = 48, kMidRowsFew = 4, kMidFew = 8192;
+// a big_rows that no island reaches (the caller wants no island on a warp): from
+// here up the middling class is off too
+constexpr int kNoWarps = 1 << 20;
 __device__ __forceinline__ int size_bucket(int rows) { return 31 - __clz(rows); }
 
 __global__ void k_sched_count(Dev d) {
     const int ni = *d.n_islands;
-    const int mid = ni <= kMidFew ? kMidRowsFew : kMidRows;
+    const int mid = d.big_rows >= kNoWarps ? kMidMax + 1 : ni <= kMidFew ? kMidRowsFew : kMidRows;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ni; i += gridDim.x * blockDim.x) {
         if (d.n_joint_edges > 0 && d.g_isl_flags[i]) { d.joint_list[atomicAdd(&d.sched[3], 1)] = i; continue; }
         int rc = d.g_isl_row_count[i];
