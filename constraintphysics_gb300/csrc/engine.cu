@@ -662,7 +662,7 @@ struct Batch {
             launch_rows(x, s == 0, s == substeps - 1, L);
             launch_joint_rows(x, s == 0, L);               mark(6 + 3 * s);
             launch_pgs(x, dv_cap, max_world, pgs_blocks, br, L);
-            launch_pgs_joint(x, s == 0, L);                mark(7 + 3 * s);
+            launch_pgs_joint(x, s == 0, dv_cap, L);        mark(7 + 3 * s);
             launch_integrate(x, s == substeps - 1, L);     mark(8 + 3 * s);
         }
         launch_geometry(x, 0, L);  mark(6 + 3 * substeps);

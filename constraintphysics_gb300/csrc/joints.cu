@@ -571,7 +571,9 @@ __global__ void k_springs(Dev d) {
     }
 }
 
-constexpr int kFactorBytes = 40 * 1024;   // blocks held in shared memory by k_holo_factor
+// blocks held in shared memory by k_holo_factor: chains of up to ~64 constraints in
+// FP64 (k_pgs_joint gives times past the line)
+constexpr int kFactorBytes = 40 * 1024;
 
 // computeBlockInitialValue (HolonomicBlockSolver.cpp:731-760)
 template <class T>

@@ -34,12 +34,11 @@ __device__ __forceinline__ void jvalue(const JointRow& R, const float* va, const
 // component c of M^-1 J^T and of the two bodies' Δv (a's six, then b's); lanes
 // meet by shuffles.  Every sum runs in the order of the one-thread form with
 // FMAs from zero, so the results are the same bits; dofs beyond the row's are
-// zeros.  Loaded one row ahead of its use.
+// zeros.  Loaded one row ahead of its use.  (The passes over the rows are
+// joint_pass in solver.cu; here is what the block solve shares with them.)
 struct JointLane {
-    float ja[6], jb[6], minv[6];   // dof lane
-    float it[6];                   // component lane
-    float target, ptarget, acc, pacc, lim;
-    int n, sa, sb, proj, pos;
+    float it[6];   // component lane
+    int n, sa, sb;
 };
 __device__ __forceinline__ void jl_row6(const float* p, float* o) {   // 8-byte aligned
     const float2* q = reinterpret_cast<const float2*>(p);
@@ -47,20 +46,8 @@ __device__ __forceinline__ void jl_row6(const float* p, float* o) {   // 8-byte 
     o[0] = x.x; o[1] = x.y; o[2] = y.x; o[3] = y.y; o[4] = z.x; o[5] = z.y;
 }
 __device__ __forceinline__ void jl_load(const JointRow& R, int lane, JointLane& L) {
-    const int i = min(lane, 5), c = min(lane, 11);
-    L.n = R.n; L.sa = R.sa; L.sb = R.sb; L.proj = R.proj; L.pos = R.pos; L.lim = R.lim;
-    jl_row6(R.ja + 6 * i, L.ja);
-    jl_row6(R.jb + 6 * i, L.jb);
-    jl_row6(R.minv + kJMax * i, L.minv);
-    jl_row6(c < 6 ? R.ita + kJMax * c : R.itb + kJMax * (c - 6), L.it);
-    L.target = R.target[i];
-    L.ptarget = R.ptarget[i];
-    L.acc = R.impulse[i];
-    L.pacc = R.pimpulse[i];
-}
-// Δv of a body for `which`; `zero` (six floats) for infinite mass
-__device__ __forceinline__ void jl_dv(const float4* dv, const float* zero, int slot, int which, float* o) {
-    jl_row6(slot < 0 ? zero : reinterpret_cast<const float*>(dv + kDvF4 * slot) + 6 * which, o);
+    L.n = R.n; L.sa = R.sa; L.sb = R.sb;
+    jl_row6(R.ita + kJMax * min(lane, 11), L.it);   // body b's follow body a's
 }
 // component lane: sum of imp_i M^-1 J^T added to its component of Δv, where
 // lane i holds imp_i (finite beyond the row's dofs)
@@ -76,47 +63,6 @@ __device__ __forceinline__ void jl_apply(const JointLane& L, float imp, float4* 
         *f = __fadd_rn(*f, x);
     }
     __syncwarp();
-}
-// warm start (DegreedConstraint::applyWarmStartVelocityChange)
-__device__ __forceinline__ void jl_warm(const JointLane& L, float4* dv, int lane) {
-    if (__any_sync(0xffffffffu, lane < L.n && fabsf(L.acc) > kJZero)) jl_apply(L, lane < L.n ? L.acc : 0.f, dv, 0, lane);
-}
-// PGSConstraintStep<n> (ConstraintSolver.cpp:12-40): the accumulated impulse
-// plus the row's correction, projected (ConeLimitConstraint /
-// TwistLimitConstraint::projectValidImpulse, ConstraintSolver.cpp:434-436,
-// 463-465: one-sided limits; MotorConstraint / PistonConstraint, :591-606,
-// 728-731), applied when the change is not zero
-__device__ __forceinline__ void jl_step(const JointLane& L, JointRow& R, float4* dv, const float* zero, bool pseudo, int lane) {
-    const int which = pseudo ? 1 : 0;
-    float va[6], vb[6];
-    jl_dv(dv, zero, L.sa, which, va);
-    jl_dv(dv, zero, L.sb, which, vb);
-    float x = 0.f, y = 0.f;
-#pragma unroll
-    for (int k = 0; k < 6; k++) {
-        x = __fmaf_rn(va[k], L.ja[k], x);
-        y = __fmaf_rn(vb[k], L.jb[k], y);
-    }
-    const float delta = __fsub_rn(pseudo ? L.ptarget : L.target, __fadd_rn(x, y));
-    const float acc = pseudo ? L.pacc : L.acc;
-    float s = 0.f;
-#pragma unroll
-    for (int k = 0; k < 6; k++) {
-        s = __fmaf_rn(__shfl_sync(0xffffffffu, delta, k), L.minv[k], s);
-    }
-    float nw = __fadd_rn(acc, s);
-    if (L.proj != 0) {   // rows of one dof
-        if (L.proj == 1) nw = fmaxf(nw, 0.f);
-        else if (L.proj == 2) nw = fminf(nw, 0.f);
-        else nw = nw > 0.f ? fminf(nw, L.lim) : fmaxf(nw, -L.lim);
-    }
-    const float diff = __fsub_rn(nw, acc);
-    if (__any_sync(0xffffffffu, lane < L.n && fabsf(diff) > kJZero)) {
-        jl_apply(L, lane < L.n ? diff : 0.f, dv, which, lane);
-        if (lane < L.n) (pseudo ? R.pimpulse : R.impulse)[lane] = __fadd_rn(acc, diff);
-    } else {
-        __syncwarp();
-    }
 }
 
 // ---- holonomic systems (HolonomicBlockSolver.cpp) ------------------------------

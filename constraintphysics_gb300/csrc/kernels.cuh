@@ -67,7 +67,7 @@ void launch_integrate(const Dev& d, int last, const Launch& L);
 void launch_joint_rows(const Dev& d, bool first, const Launch& L);
 // springs: impulse pairs at the start of every substep (no-op without springs)
 void launch_springs(const Dev& d, const Launch& L);
-void launch_pgs_joint(const Dev& d, bool first, const Launch& L);
+void launch_pgs_joint(const Dev& d, bool first, int dv_cap, const Launch& L);
 // external state write: apply the staged state (d.stage); bodies whose pose
 // changed get their world inertia tensors and AABBs recomputed
 void launch_apply_state(const Dev& d, const Launch& L);

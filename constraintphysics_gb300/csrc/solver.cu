@@ -19,6 +19,8 @@
 //
 // Integration (PhysicsEngine.cpp:390-419, RigidBody.cpp:207-279): one thread
 // per body.
+#include <algorithm>
+
 #include "kernels.cuh"
 #include "devmath.cuh"
 #include "shapes.cuh"
@@ -1090,12 +1092,38 @@ __device__ __noinline__ void holo_system(const Dev& d, int s, HoloSm& sm, bool r
     }
 }
 
-// A pass over an island held in shared memory (`list`: each row's joint slot, -1
-// a contact row, which lane 0 runs from global memory).  KIND 0: warm start, 1:
-// velocity, 2: position.  The same steps as jl_warm / jl_step with everything
-// typed as shared memory and only the pass's own fields loaded: a joint row is
-// bound by its instruction count on one warp (168 a row-step through generic
-// pointers) and its dependency chain.
+// A joint-island warp's shared memory (k_pgs_joint): what is held and up to which
+// island (more in global memory).
+constexpr int kJointDv = 68, kJointRes = 64, kJointList = 1024;
+constexpr int kRowF4 = (int)(sizeof(RowBlock) / 16);
+struct alignas(16) JointSm {
+    uint64_t bar;
+    float zero[8];              // Δv of a body of infinite mass
+    int held[kJointRes];        // the joint in each slot
+    int16_t list[kJointList];   // the row's joint slot, -1 a contact row
+    HoloSm holo;
+    float4 crow[2][kRowF4];     // contact rows on their way to the lanes
+    float4 dv[kDvF4 * kJointDv];
+    uint8_t rows[kJointRes * kJointStage];
+};
+constexpr int kJointSmem = (int)sizeof(JointSm);
+static_assert(offsetof(JointSm, rows) % 16 == 0 && kJointStage % 16 == 0, "bulk copies into the held rows");
+__device__ __forceinline__ JointSm& joint_sm() {
+    extern __shared__ __align__(16) uint8_t sm[];
+    return *reinterpret_cast<JointSm*>(sm);
+}
+
+// The passes over a joint island's rows.  A joint row takes the lanes of joints.cuh
+// with only the pass's own fields loaded and, where the island is held in shared
+// memory, everything typed as such: it is bound by its instruction count on one
+// warp (168 a row-step through generic pointers) and its dependency chain.  A
+// step is PGSConstraintStep<n> (ConstraintSolver.cpp:12-40): the accumulated impulse
+// plus the row's correction, projected (ConeLimitConstraint /
+// TwistLimitConstraint::projectValidImpulse, ConstraintSolver.cpp:434-436,
+// 463-465: one-sided limits; MotorConstraint / PistonConstraint, :591-606,
+// 728-731), applied when the change is not zero.  A contact row is shared by two
+// lanes like the large islands' (half_vel and the others above; by lane 0 alone,
+// from global memory: 32 chains of 30 links lying on a plate 5.6 ms a step, now 3.5).
 struct JointRes {
     int n, sa, sb, proj, pos;
     float lim, ja[6], jb[6], mv[6], it[6], tgt, acc;
@@ -1166,34 +1194,54 @@ __device__ __forceinline__ void jr_row(const JointRes& L, uint8_t* row, float4* 
     }
     __syncwarp();
 }
+// a contact row in shared memory at `sr`, its own place `R`
 template <int KIND>
-__device__ __forceinline__ void jr_pass(uint8_t* srows, const int16_t* list, RowBlock* rows, int rc, float4* dv, const float* zero,
-                                        int lane) {
+__device__ __forceinline__ void jc_row(const RowBlock* sr, RowBlock* R, float4* dv, int lane) {
+    constexpr int which = KIND == 2 ? 1 : 0;
+    HalfRow h;
+    half_load(sr, lane & 1, h);
+    const int slot = lane & 1 ? sr->sb : sr->sa;
+    P3 v = dv_get(dv, slot, which);
+    int stat = 0;
+    if (KIND == 0) half_warm(h, v);
+    else if (KIND == 1) half_vel(h, v, stat);
+    else half_pos(h, v);
+    if (KIND != 0) R->imp = h.imp;   // all lanes, the same value
+    if (KIND == 1) R->stat = stat;
+    dv_put(dv, slot, which, v);
+    __syncwarp();
+}
+// One pass.  KIND 0: warm start, 1: velocity, 2: position.  RES: joint rows and Δv
+// are in shared memory; MIXED: the island holds contact rows.  The next contact
+// row is loaded by 24 lanes, 16 bytes each, and goes through shared memory.
+template <int KIND, bool RES, bool MIXED>
+__device__ __forceinline__ void joint_pass(JointSm& sm, JointRow* joints, RowBlock* rows, int rc, float4* dv, int lane) {
     JointRes A, B;
-    int c = list[0], n = list[min(1, rc - 1)], r = 0;
-    jr_load<KIND>(srows + max(c, 0) * kJointStage, lane, A);
+    float4 piece{};
+    const float* zero = sm.zero;
+    // row r's joint slot (RES) or joint, -1 a contact row
+    auto kind = [&](int r) {
+        if (RES) return (int)sm.list[r];
+        const int c = rows[r].contact;
+        return c < 0 ? -c - 1 : -1;
+    };
+    auto joint = [&](int k) { return RES ? sm.rows + k * kJointStage : reinterpret_cast<uint8_t*>(joints + k); };
+    auto load = [&](int k, int at, JointRes& J) {
+        jr_load<KIND>(joint(max(k, 0)), lane, J);   // without a branch: some joint's in the place of a contact row
+        if (MIXED) piece = reinterpret_cast<const float4*>(rows + at)[min(lane, kRowF4 - 1)];
+    };
+    int c = kind(0), n = kind(min(1, rc - 1)), r = 0;
+    load(c, 0, A);
     auto one = [&](JointRes& L, JointRes& N) {
-        jr_load<KIND>(srows + max(n, 0) * kJointStage, lane, N);
-        const int n2 = list[min(r + 2, rc - 1)];
-        if (__any_sync(0xffffffffu, c >= 0)) {
-            jr_row<KIND>(L, srows + c * kJointStage, dv, zero, lane);
+        float4* sr = sm.crow[r & 1];
+        if (MIXED && lane < kRowF4) sr[lane] = piece;
+        load(n, min(r + 1, rc - 1), N);
+        const int n2 = kind(min(r + 2, rc - 1));
+        if (!MIXED || __any_sync(0xffffffffu, c >= 0)) {   // a vote: a uniform branch
+            jr_row<KIND>(L, joint(c), dv, zero, lane);
         } else {
-            if (lane == 0) {
-                RowBlock& R = rows[r];
-                float4 imp = R.imp;
-                if (KIND == 0) {
-                    row_warm(R, imp, dv);
-                } else if (KIND == 1) {
-                    int st = R.stat;
-                    row_vel(R, imp, st, dv);
-                    R.imp = imp;
-                    R.stat = st;
-                } else {
-                    row_pos(R, imp, dv);
-                    R.imp = imp;
-                }
-            }
             __syncwarp();
+            jc_row<KIND>(reinterpret_cast<const RowBlock*>(sr), rows + r, dv, lane);
         }
         c = n;
         n = n2;
@@ -1205,37 +1253,45 @@ __device__ __forceinline__ void jr_pass(uint8_t* srows, const int16_t* list, Row
         one(B, A);
         if (r >= rc) break;
     }
+    __syncwarp();
+}
+// the island's passes; a function of its own for the registers (inlined three
+// times into the kernel they spilled)
+template <bool RES, bool MIXED>
+__device__ __forceinline__ void joint_passes(JointRow* joints, RowBlock* rows, int rc, float4* gdv, int n_vel, int n_pos, int lane) {
+    JointSm& sm = joint_sm();
+    float4* dv = RES ? sm.dv : gdv;
+    joint_pass<0, RES, MIXED>(sm, joints, rows, rc, dv, lane);
+    for (int it = 0; it < n_vel; it++) joint_pass<1, RES, MIXED>(sm, joints, rows, rc, dv, lane);
+    for (int it = 0; it < n_pos; it++) joint_pass<2, RES, MIXED>(sm, joints, rows, rc, dv, lane);
 }
 
 // Islands with joint rows: one warp per island, contact rows and joint rows in
-// island order, then the island's holonomic systems (first substep).  A joint
-// row is spread over the lanes (joints.cuh), a contact row runs on lane 0.
-// Bound by the chain of row-steps, each a few dependent loads: the joint rows
-// (up to kJointRes of an island of up to kJointList rows) and the Δv of islands
-// of up to kJointDv bodies are held in shared memory.  On 512 chains of 16-64
+// island order, then the island's holonomic systems (first substep).  Bound by the
+// chain of row-steps, each a few dependent loads: the joint rows (up to kJointRes
+// of an island of up to kJointList rows) and the Δv of islands of up to kJointDv
+// bodies (`dv_cap` lowers it) are held in shared memory.  On 512 chains of 16-64
 // links: one lane and everything in global memory 568 us a substep, the rows
 // in global memory 263, in shared memory 219 (the first, with the solve, 1,880
-// -> 594).
-constexpr int kJointDv = 68, kJointRes = 64, kJointList = 128;
+// -> 594).  Past the lines (and past those of the block solve: kHoloN, kHoloL and
+// the factor's kFactorBytes), a step of 256 hung chains of 64 / 65 / 69 / 100
+// links, FP64 systems: 1.98 / 3.17 / 4.31 / 6.61 ms (6.78 / 6.84 / 7.64 / 12.8 by
+// one lane with everything in global memory).
 // sched[kJointNext]: the next joint-list entry
 constexpr int kJointNext = kBigNext + 2;
-constexpr int kJointFixed = 64 + kJointList * 6 + (int)sizeof(HoloSm);   // barrier, zero entry, row list, joint list, solve
-constexpr int kJointSmem = ((kJointFixed + 15) & ~15) + kDvF4 * kJointDv * 16 + kJointRes * kJointStage;
-__global__ void __launch_bounds__(32, 3) k_pgs_joint(Dev d, int first) {
-    extern __shared__ __align__(16) uint8_t sm[];
-    uint64_t* bar = reinterpret_cast<uint64_t*>(sm);
-    float* zero = reinterpret_cast<float*>(sm + 32);       // Δv of a body of infinite mass
-    int* held_j = reinterpret_cast<int*>(sm + 64);         // resident island: the joint in each slot
-    int16_t* list = reinterpret_cast<int16_t*>(sm + 64 + kJointList * 4);   // the row's joint slot, -1 a contact row
-    HoloSm& hsm = *reinterpret_cast<HoloSm*>(sm + 64 + kJointList * 6);
-    float4* sdv = reinterpret_cast<float4*>(sm + ((kJointFixed + 15) & ~15));
-    uint8_t* srows = reinterpret_cast<uint8_t*>(sdv + kDvF4 * kJointDv);
+__global__ void __launch_bounds__(32, 3) k_pgs_joint(Dev d, int first, int dv_cap) {
+    JointSm& sm = joint_sm();
+    uint64_t* bar = &sm.bar;
+    int* held_j = sm.held;
+    int16_t* list = sm.list;
+    float4* sdv = sm.dv;
+    uint8_t* srows = sm.rows;
     const int lane = threadIdx.x;
     const int nj = d.sched[3];
     uint32_t parity = 0;
     if (lane == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(bar)), "r"(1) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    if (lane < 8) zero[lane] = 0.f;
+    if (lane < 8) sm.zero[lane] = 0.f;
     __syncwarp();
     while (true) {
         int q = 0;
@@ -1246,11 +1302,11 @@ __global__ void __launch_bounds__(32, 3) k_pgs_joint(Dev d, int first) {
         const int rs = d.g_isl_row_start[i], rc = d.g_isl_row_count[i];
         const int bs = d.g_isl_body_start[i], bc = d.g_isl_body_count[i];
         const WorldParams& P = d.wparams[d.g_isl_world[i]];
-        float4* dv = bc <= kJointDv ? sdv : d.dv + kDvF4 * (size_t)bs;
+        float4* dv = bc <= dv_cap ? sdv : d.dv + kDvF4 * (size_t)bs;
         float4* err = d.dv_err + kDvF4 * (size_t)bs;
         // the island's joint rows into shared memory, if they fit
         int held = 0;
-        bool res = rc <= kJointList && bc <= kJointDv;
+        bool res = rc <= kJointList && bc <= dv_cap;
         for (int base = 0; res && base < rc; base += 32) {
             const bool in = base + lane < rc;
             const int c = in ? d.rows[rs + base + lane].contact : 0;
@@ -1258,7 +1314,7 @@ __global__ void __launch_bounds__(32, 3) k_pgs_joint(Dev d, int first) {
             const int slot = held + __popc(m & ((1u << lane) - 1u));
             if (in) {
                 list[base + lane] = c < 0 ? (int16_t)slot : (int16_t)-1;
-                if (c < 0 && slot < kJointList) held_j[slot] = -c - 1;
+                if (c < 0 && slot < kJointRes) held_j[slot] = -c - 1;
             }
             held += __popc(m);
             res = held <= kJointRes;
@@ -1289,70 +1345,9 @@ __global__ void __launch_bounds__(32, 3) k_pgs_joint(Dev d, int first) {
             }
         }
         const int n_vel = P.pgs_vel, n_pos = P.pgs_pos;   // read once: the row stores could alias P
-        // the island's row r: its joint row, or null for a contact row
-        auto joint_of = [&](int r) -> JointRow* {
-            if (res) return list[r] < 0 ? nullptr : reinterpret_cast<JointRow*>(srows + list[r] * kJointStage);
-            const int c = d.rows[rs + r].contact;
-            return c < 0 ? d.jt.rows + (-c - 1) : nullptr;
-        };
-        // one pass over the rows: joint(lane row, joint row) or contact(row)
-        // for each, the next joint row loaded one row ahead
-        auto pass = [&](auto&& joint, auto&& contact) {
-            JointRow* any = d.jt.rows;   // loaded in the place of a contact row
-            JointRow *c = joint_of(0), *n = joint_of(min(1, rc - 1));
-            JointLane A, B;
-            jl_load(c ? *c : *any, lane, A);
-            int r = 0;
-            auto one = [&](JointLane& L, JointLane& N) {
-                jl_load(n ? *n : *any, lane, N);
-                JointRow* n2 = joint_of(min(r + 2, rc - 1));
-                if (c) joint(L, *c);
-                else contact(d.rows[rs + r]);
-                c = n;
-                n = n2;
-                r++;
-            };
-            while (true) {
-                one(A, B);
-                if (r >= rc) break;
-                one(B, A);
-                if (r >= rc) break;
-            }
-            __syncwarp();
-        };
-        if (res) {
-            jr_pass<0>(srows, list, d.rows + rs, rc, sdv, zero, lane);
-            for (int it = 0; it < n_vel; it++) jr_pass<1>(srows, list, d.rows + rs, rc, sdv, zero, lane);
-            for (int it = 0; it < n_pos; it++) jr_pass<2>(srows, list, d.rows + rs, rc, sdv, zero, lane);
-        } else {
-            pass([&](const JointLane& L, JointRow&) { jl_warm(L, dv, lane); },
-                 [&](RowBlock& R) {
-                     if (lane == 0) row_warm(R, R.imp, dv);
-                     __syncwarp();
-                 });
-            for (int it = 0; it < n_vel; it++)
-                pass([&](const JointLane& L, JointRow& R) { jl_step(L, R, dv, zero, false, lane); },
-                     [&](RowBlock& R) {
-                         if (lane == 0) {
-                             float4 imp = R.imp;
-                             int st = R.stat;
-                             row_vel(R, imp, st, dv);
-                             R.imp = imp;
-                             R.stat = st;
-                         }
-                         __syncwarp();
-                     });
-            for (int it = 0; it < n_pos; it++)
-                pass([&](const JointLane& L, JointRow& R) { if (L.pos) jl_step(L, R, dv, zero, true, lane); },   // needsPosCorrect
-                     [&](RowBlock& R) {
-                         if (lane == 0) {
-                             float4 imp = R.imp;
-                             row_pos(R, imp, dv);
-                             R.imp = imp;
-                         }
-                         __syncwarp();
-                     });
-        }
+        if (res && held == rc) joint_passes<true, false>(d.jt.rows, d.rows + rs, rc, dv, n_vel, n_pos, lane);
+        else if (res) joint_passes<true, true>(d.jt.rows, d.rows + rs, rc, dv, n_vel, n_pos, lane);
+        else joint_passes<false, true>(d.jt.rows, d.rows + rs, rc, dv, n_vel, n_pos, lane);
         if (first && P.pgs_holo > 0) {
             const int ss = d.g_isl_sys_start[i], sn = d.g_isl_sys_count[i];
             for (int it = 0; it < P.pgs_holo; it++)
@@ -1363,8 +1358,8 @@ __global__ void __launch_bounds__(32, 3) k_pgs_joint(Dev d, int first) {
                             if (held_j[q] == j) return reinterpret_cast<JointRow*>(srows + q * kJointStage);
                         return nullptr;
                     };
-                    if (d.hs.fp64[s]) holo_system<double>(d, s, hsm, res, find, dv, err, lane);
-                    else holo_system<float>(d, s, hsm, res, find, dv, err, lane);
+                    if (d.hs.fp64[s]) holo_system<double>(d, s, sm.holo, res, find, dv, err, lane);
+                    else holo_system<float>(d, s, sm.holo, res, find, dv, err, lane);
                 }
         }
         __syncwarp();
@@ -1372,7 +1367,7 @@ __global__ void __launch_bounds__(32, 3) k_pgs_joint(Dev d, int first) {
             const int c = d.rows[r].contact;
             if (c >= 0) continue;
             const int j = -c - 1;
-            const JointRow& R = *joint_of(r - rs);
+            const JointRow& R = res ? *reinterpret_cast<const JointRow*>(srows + list[r - rs] * kJointStage) : d.jt.rows[j];
             for (int k = 0; k < R.n; k++) {
                 d.jt.impulse[kJMax * j + k] = R.impulse[k];
                 if (res) {   // a row that is kept (a limit, a motor) goes on from these
@@ -1538,9 +1533,9 @@ void launch_pgs_schedule(const Dev& d, const Launch& L) {
     k_sched_place<<<L.n_sms * 2, 256, 0, L.st>>>(d);
 }
 
-void launch_pgs_joint(const Dev& d, bool first, const Launch& L) {
+void launch_pgs_joint(const Dev& d, bool first, int dv_cap, const Launch& L) {
     if (d.n_joint_edges == 0) return;
-    k_pgs_joint<<<L.n_sms * 3, 32, kJointSmem, L.st>>>(d, first ? 1 : 0);
+    k_pgs_joint<<<L.n_sms * 3, 32, kJointSmem, L.st>>>(d, first ? 1 : 0, std::min(dv_cap, kJointDv));
 }
 
 void launch_pgs(const Dev& d, int dv_cap, int max_world, int big_blocks, const Branches& b, const Launch& L) {
