@@ -1025,7 +1025,7 @@ __device__ __forceinline__ void holo_apply(const Dev& d, int s, const HoloView& 
             if (__any_sync(0xffffffffu, fabsf(imp) > kJZero)) {
                 jl_apply(L, imp, to, wh, lane);
                 if (store && lane < L.n) {
-                    JointRow& R = d.jt.rows[h.cons[i]];
+                    JointRow& R = *row_of(i);
                     (pseudo ? R.pimpulse : R.holo)[lane] += imp;
                 }
             }
@@ -1373,6 +1373,7 @@ __global__ void __launch_bounds__(32, 3) k_pgs_joint(Dev d, int first, int dv_ca
                 if (res) {   // a row that is kept (a limit, a motor) goes on from these
                     d.jt.rows[j].impulse[k] = R.impulse[k];
                     d.jt.rows[j].pimpulse[k] = R.pimpulse[k];
+                    d.jt.rows[j].holo[k] = R.holo[k];
                 }
             }
         }
