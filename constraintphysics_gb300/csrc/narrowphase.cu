@@ -2376,17 +2376,22 @@ __global__ void k_raycast(Dev d, int s, int e, const float* rays, int n, const u
     };
     if (tid == 0) n_list = 0;
     __syncthreads();
-    // bodies in the list, counted by the barrier: the counter itself may be
-    // ahead again when a late warp reads it, and the warps must agree on
-    // whether this round empties the list
-    int m = 0;
+    // The counter is read between two barriers, so that all warps see the same and
+    // agree on whether this round empties the list; rounds that cannot have filled
+    // it (`bound`: entries at most) go on without one.
+    int bound = 0;
     for (int base = s; base < e; base += nt) {
         const int g = base + tid;
-        const bool crossed =
-            g < e && rayAABB(mk(d.aabb_lo[g]), mk(d.aabb_hi[g]), o, dir) && !rayIgnored(ignore, n_ignore, (uint32_t)(g - s + 1));
-        if (crossed) list[atomicAdd(&n_list, 1)] = g;
-        m += __syncthreads_count(crossed);
-        if (m + nt <= kRayList && base + nt < e) continue;
+        if (g < e && rayAABB(mk(d.aabb_lo[g]), mk(d.aabb_hi[g]), o, dir) && !rayIgnored(ignore, n_ignore, (uint32_t)(g - s + 1)))
+            list[atomicAdd(&n_list, 1)] = g;
+        bound += nt;
+        const bool last = base + nt >= e;
+        if (!last && bound + nt <= kRayList) continue;
+        __syncthreads();
+        const int m = n_list;
+        __syncthreads();
+        bound = m;
+        if (!last && m + nt <= kRayList) continue;
         for (int q0 = 0; q0 < m; q0 += nt) {
             const bool in = q0 + tid < m;
             const int b = in ? list[q0 + tid] : 0;
@@ -2409,7 +2414,7 @@ __global__ void k_raycast(Dev d, int s, int e, const float* rays, int n, const u
         __syncthreads();
         if (tid == 0) n_list = 0;
         __syncthreads();
-        m = 0;
+        bound = 0;
     }
     if (__syncthreads_or(nan || !(mag2(o) + mag2(dir) < INFINITY))) {
         mine = RayHitD{false};
