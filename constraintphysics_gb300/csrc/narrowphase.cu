@@ -2145,7 +2145,7 @@ int mesh_scratch_warps(int n_sms) { return n_sms * kMeshBlocksPerSm * 8; }
 
 // ---- ray queries ------------------------------------------------------------------
 // PhysicsEngine::raycastFirstIntersection (PhysicsEngine.cpp:582-609) for one
-// ray per block against the bodies [s, e) of one world: every body whose
+// ray per block (many rays: per thread) against the bodies [s, e) of one world: every body whose
 // current AABB the ray crosses is tested with its primitive's ray test, the
 // nearest hit wins (strictly nearer replaces, in body order).
 namespace {
@@ -2354,6 +2354,39 @@ __device__ __forceinline__ bool rayIgnored(const uint32_t* ignore, int n, uint32
     return skip;
 }
 
+// One ray on one thread, the bodies in their order
+__device__ void raySerial(const Dev& d, int s, int e, f3 o, f3 dir, const uint32_t* ignore, int n_ignore, float* r) {
+    RayHitD best{false};
+    int best_id = 0;
+    for (int g = s; g < e; g++) {
+        if (rayIgnored(ignore, n_ignore, (uint32_t)(g - s + 1)) || !rayAABB(mk(d.aabb_lo[g]), mk(d.aabb_hi[g]), o, dir)) continue;
+        bool mesh = false;
+        RayHitD h = rayBody(d, g, o, dir, &mesh);
+        if (mesh) h = rayMeshSerial(prim_blob(d, g, 0), o, dir);
+        if (h.hit && (!best.hit || h.t < best.t)) { best = h; best_id = g - s + 1; }
+    }
+    r[0] = __int_as_float(best_id);
+    r[1] = best.hit ? best.p.x : 0.f; r[2] = best.hit ? best.p.y : 0.f; r[3] = best.hit ? best.p.z : 0.f;
+    r[4] = best.hit ? best.n.x : 0.f; r[5] = best.hit ? best.n.y : 0.f; r[6] = best.hit ? best.n.z : 0.f;
+    r[7] = best.hit ? best.t : -1.f;
+}
+// Many rays: a thread each.  The threads of a warp test the same body and the same
+// triangle, one load for 32 rays, where a block loads everything for its one ray;
+// but a thread takes the bodies one after the other whatever the number of rays.
+// Calls of 4,096 / 32,768 / 65,536 / 262,144 rays, a thread a ray against a block:
+// 217 hulls 624 / 866 / 1,212 / 4,554 against 205 / 1,089 / 2,071 / 7,824 us; a
+// terrain mesh 1,118 / 1,365 / 1,692 / 6,127 against 230 / 1,447 / 2,823 / 10,965;
+// 2,000 bodies 845 / 1,092 / 1,377 / 4,632 against 151 / 875 / 1,673 / 7,356: the
+// line (kRayMany) lies between 16,000 and 50,000 rays whatever the scene, since
+// both times grow with the bodies.
+__global__ void __launch_bounds__(128) k_raycast_many(Dev d, int s, int e, const float* rays, int n, const uint32_t* ignore, int n_ignore,
+                                                      float* out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    raySerial(d, s, e, mk(rays[6 * k], rays[6 * k + 1], rays[6 * k + 2]), mk(rays[6 * k + 3], rays[6 * k + 4], rays[6 * k + 5]), ignore,
+              n_ignore, out + 8 * (size_t)k);
+}
+
 // A block per ray: its threads test the bodies' AABBs, the few that the ray
 // crosses are listed in shared memory and then tested one per thread (a mesh
 // by the whole block).  Bound by the AABB tests' loads (L2); a thread per ray
@@ -2361,6 +2394,7 @@ __device__ __forceinline__ bool rayIgnored(const uint32_t* ignore, int n, uint32
 // A hit at distance NaN (a disk's plane holding the ray) has no place in an
 // order of distances: one thread then takes the bodies one after the other.
 constexpr int kRayList = 512;
+constexpr int kRayMany = 40960;
 __global__ void k_raycast(Dev d, int s, int e, const float* rays, int n, const uint32_t* ignore, int n_ignore, float* out) {
     __shared__ int list[kRayList];
     __shared__ int n_list;
@@ -2417,22 +2451,7 @@ __global__ void k_raycast(Dev d, int s, int e, const float* rays, int n, const u
         bound = 0;
     }
     if (__syncthreads_or(nan || !(mag2(o) + mag2(dir) < INFINITY))) {
-        mine = RayHitD{false};
-        mine_id = 0;
-        if (tid == 0)
-            for (int g = s; g < e; g++) {
-                if (rayIgnored(ignore, n_ignore, (uint32_t)(g - s + 1)) || !rayAABB(mk(d.aabb_lo[g]), mk(d.aabb_hi[g]), o, dir)) continue;
-                bool mesh = false;
-                RayHitD h = rayBody(d, g, o, dir, &mesh);
-                if (mesh) h = rayMeshSerial(prim_blob(d, g, 0), o, dir);
-                if (h.hit && (!mine.hit || h.t < mine.t)) { mine = h; mine_id = g - s + 1; }
-            }
-        if (tid > 0) return;
-        float* r = out + 8 * (size_t)k;
-        r[0] = __int_as_float(mine_id);
-        r[1] = mine.hit ? mine.p.x : 0.f; r[2] = mine.hit ? mine.p.y : 0.f; r[3] = mine.hit ? mine.p.z : 0.f;
-        r[4] = mine.hit ? mine.n.x : 0.f; r[5] = mine.hit ? mine.n.y : 0.f; r[6] = mine.hit ? mine.n.z : 0.f;
-        r[7] = mine.hit ? mine.t : -1.f;
+        if (tid == 0) raySerial(d, s, e, o, dir, ignore, n_ignore, out + 8 * (size_t)k);
         return;
     }
     const RayBest best = ray_block_best<false>(RayBest{mine.t, mine.hit ? mine_id : -1}, sh);
@@ -2451,6 +2470,10 @@ __global__ void k_raycast(Dev d, int s, int e, const float* rays, int n, const u
 void launch_raycast(const Dev& d, int s, int e, const float* rays, int n, const uint32_t* ignore, int n_ignore, float* out,
                     cudaStream_t st) {
     if (n <= 0) return;
+    if (n >= kRayMany) {
+        k_raycast_many<<<(n + 127) / 128, 128, 0, st>>>(d, s, e, rays, n, ignore, n_ignore, out);
+        return;
+    }
     // few rays: more threads a ray, so that the bodies' loads run side by side
     const int nt = e - s <= 64 ? 32 : (n <= 1024 ? 256 : 128);
     k_raycast<<<n, nt, 0, st>>>(d, s, e, rays, n, ignore, n_ignore, out);
