@@ -233,8 +233,10 @@ __global__ void k_contacts(Dev d, int write) {
 // their global index, stored as -(k + 1)).
 __device__ __forceinline__ long long islands_need(int nb, int ne_w, int nj) {
     const long long E = (long long)ne_w + nj;
-    return 4LL * (7LL * nb + 1 + 4 * E + ne_w + 2 * E + nb) + nb;   // ints, then the body flags (bytes)
+    return 4LL * (5LL * nb + 4 * E + ne_w + 2 * E + nb) + nb;   // ints, then the body flags (bytes)
 }
+// and for the search's visits and components beside it
+__device__ __forceinline__ long long islands_lists(int nb) { return 4LL * (2LL * nb + 1); }
 
 // exclusive prefix of one value per thread (whole warps, at most 32) with the
 // block's total in *total; `ws` holds an int per warp
@@ -414,7 +416,7 @@ __device__ void islands_place(const Dev& d, int w, int s, int nb, int e0, int ro
     }
 }
 
-// a world whose graph is in shared memory, by one warp
+// a world whose graph is in shared memory (ord and first may be in global memory), by one warp
 __device__ void islands_small(const Dev& d, int w, int s, int nb, int e0, int row0, int* vis, const int* a_ofs, const int* a_cur,
                               const int* adj, const int* live, int* stk, int* order, int* ord, int* first, const uint8_t* mov,
                               int* ws, int* sh_rows_end) {
@@ -763,7 +765,15 @@ __global__ void __launch_bounds__(NT) k_islands(Dev d, int smem_bytes) {
     const int sys0 = joints ? d.hs_world_start[w] : 0;
     const int nb = e - s, ne_w = e1 - e0, nj = je1 - je0, E = ne_w + nj;
     const int stack_cap = 2 * E + nb;
-    const bool fast = islands_need(nb, ne_w, nj) <= smem_bytes;
+    const bool big = d.comp != nullptr && nb > kTileWorld;
+    // The visits and components are written once and read little: a graph that
+    // fits without them keeps its place, and they take global scratch that such a
+    // world leaves unused (one world of 1,500 touching spheres, whose graph they
+    // would push out: 2,130 us with the graph in global memory, 434 so).  Such a
+    // world has edges, so a stack slice holds nb + 1 entries.
+    const long long need = islands_need(nb, ne_w, nj);
+    const bool lists = need + islands_lists(nb) <= smem_bytes;
+    const bool fast = big ? lists : need <= smem_bytes;
     int *vis, *a_ofs, *a_cur, *adj, *live, *stk, *order = nullptr, *ord = nullptr, *first = nullptr;
     const uint8_t* mov;
     uint8_t* mov_s = nullptr;
@@ -772,7 +782,7 @@ __global__ void __launch_bounds__(NT) k_islands(Dev d, int smem_bytes) {
         live = adj + 4 * E; stk = live + ne_w; order = stk + stack_cap;
         ord = order + nb;        // bodies in the order visited
         first = ord + nb;        // per component: its first place there
-        mov_s = reinterpret_cast<uint8_t*>(first + nb + 1);
+        mov_s = reinterpret_cast<uint8_t*>(lists ? first + nb + 1 : ord);
         mov = mov_s;
     } else {
         vis = d.visited + s; a_ofs = d.adj_ofs + s; a_cur = d.adj_cursor + s;
@@ -864,7 +874,7 @@ __global__ void __launch_bounds__(NT) k_islands(Dev d, int smem_bytes) {
         }
     }
     __syncthreads();
-    if (d.comp != nullptr && nb > kTileWorld) {
+    if (big) {
         IslandCtx x;
         x.w = w; x.s = s; x.e0 = e0; x.ready_steps = d.wparams[w].ready_steps;
         x.sleep_on = d.has_sleep != 0;
@@ -872,8 +882,11 @@ __global__ void __launch_bounds__(NT) k_islands(Dev d, int smem_bytes) {
         x.joints = joints;
         x.a_ofs = a_ofs; x.a_cur = a_cur; x.adj = adj; x.live = live; x.mov = mov; x.vis = vis;
         islands_big(d, x, nb, ne_w, c0 + jj0, sys0, fast ? ord : (4LL * nb <= smem_bytes ? sm_isl : nullptr), warp_sums, &sh_rows_end);
-    } else if (fast && nj == 0 && !d.has_sleep && !d.isl_serial) {
+    } else if (fast && lists && nj == 0 && !d.has_sleep && !d.isl_serial) {
         islands_small(d, w, s, nb, e0, c0 + jj0, vis, a_ofs, a_cur, adj, live, stk, order, ord, first, mov, warp_sums, &sh_rows_end);
+    } else if (fast && nj == 0 && !d.has_sleep && !d.isl_serial) {
+        islands_small(d, w, s, nb, e0, c0 + jj0, vis, a_ofs, a_cur, adj, live, stk, order, d.adj_ofs + s, d.stack + 2 * (e0 + je0) + s,
+                      mov, warp_sums, &sh_rows_end);
     } else if (tid == 0) {
         // sleeping (sleepOrSolveIslands, PhysicsEngine.cpp:1536-1613): a
         // sleeping body's edges to sleeping or fixed bodies carry no rows, and
