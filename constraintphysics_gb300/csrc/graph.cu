@@ -740,8 +740,11 @@ __device__ void islands_big(const Dev& d, const IslandCtx& x, int nb, int ne_w, 
     }
 }
 
-// NT threads a block: 256, or 1,024 for a batch of a few large worlds, whose
-// islands one block each walks through (20,000 bodies 4.3 -> 1.5 ms, 1,000
+// NT threads a block: 256; 64 for a batch of more worlds of up to 64 bodies than
+// four an SM (a block's barriers are most of such a world's time, and eight
+// blocks of 256 fill an SM: 20,000 worlds of 2 / 10 / 20 bodies 377 / 567 / 698 ->
+// 131 / 199 / 254 us, 60 worlds of 60 bodies 56 -> 66); 1,024 for a batch of a
+// few large worlds, whose islands one block each walks through (20,000 bodies 4.3 -> 1.5 ms, 1,000
 // bodies 360 -> 306 us; worlds of up to 64 bodies the same with either)
 template <int NT>
 __global__ void __launch_bounds__(NT) k_islands(Dev d, int smem_bytes) {
@@ -1087,6 +1090,7 @@ int islands_smem_bytes(int max_bodies) {
     // about four constraint edges per body, at most kIslandsSmemMax; the
     // kernel's limit (shared by every batch of the process) is that maximum
     const long long want = 4LL * (8LL * max_bodies + 7LL * 4 * max_bodies) + max_bodies + 64;
+    cudaFuncSetAttribute(k_islands<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kIslandsSmemMax);
     cudaFuncSetAttribute(k_islands<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, kIslandsSmemMax);
     cudaFuncSetAttribute(k_islands<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, kIslandsSmemMax);
     return (int)std::min<long long>(want, kIslandsSmemMax);
@@ -1094,6 +1098,7 @@ int islands_smem_bytes(int max_bodies) {
 
 void launch_islands(const Dev& d, int max_world, int smem_bytes, const Launch& L) {
     if (max_world > 256 && d.n_worlds <= L.n_sms) k_islands<1024><<<d.n_worlds, 1024, smem_bytes, L.st>>>(d, smem_bytes);
+    else if (max_world <= 64 && d.n_worlds > 4 * L.n_sms) k_islands<64><<<d.n_worlds, 64, smem_bytes, L.st>>>(d, smem_bytes);
     else k_islands<256><<<d.n_worlds, 256, smem_bytes, L.st>>>(d, smem_bytes);
     launch_scan<IslandScan>(d, nullptr, d.n_worlds, d.n_worlds, L);
     k_island_copy<<<grid_for(d.n_bodies, 128, L.n_sms), 128, 0, L.st>>>(d);
