@@ -79,7 +79,7 @@ struct GridWorld {
     __device__ __forceinline__ int operator()(int i) const { return d.world[i]; }
 };
 __device__ __forceinline__ PairGrid<int> dev_grid(const Dev& d) {
-    return PairGrid<int>{d.grid_bucket, d.grid_ids, d.grid_far, d.grid_n_far, d.grid_inv, d.grid_buckets};
+    return PairGrid<int>{d.grid_bucket, d.grid_ids, d.grid_far, d.grid_n_far, d.grid_inv, d.grid_buckets, d.n_bodies, d.n_bodies};
 }
 __device__ __forceinline__ bool in_grid_world(const Dev& d, int i) {
     const int w = d.world[i];

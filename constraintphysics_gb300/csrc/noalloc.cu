@@ -75,7 +75,7 @@ struct NaEnd {
     __device__ __forceinline__ int operator()(int) const { return n; }
 };
 __device__ __forceinline__ void na_put(uint32_t* pairs, int cap, int o, int i, int j) {
-    if (o < cap) { pairs[2 * (size_t)o] = (uint32_t)i + 1; pairs[2 * (size_t)o + 1] = (uint32_t)j + 1; }
+    if ((unsigned)o < (unsigned)cap) { pairs[2 * (size_t)o] = (uint32_t)i + 1; pairs[2 * (size_t)o + 1] = (uint32_t)j + 1; }
 }
 
 __global__ void __launch_bounds__(256) k_na_count(const float* aabbs, int n, NoAllocScratch* s) {
@@ -98,8 +98,8 @@ __global__ void __launch_bounds__(256) k_na_write(const float* aabbs, int n, con
 }
 
 // ---- the grid ------------------------------------------------------------------------
-__device__ __forceinline__ PairGrid<uint16_t> na_grid(NoAllocScratch* s) {
-    return PairGrid<uint16_t>{s->bucket, s->ids, s->far_ids, &s->n_far, &s->inv, kNoAllocBuckets};
+__device__ __forceinline__ PairGrid<uint16_t> na_grid(NoAllocScratch* s, int n) {
+    return PairGrid<uint16_t>{s->bucket, s->ids, s->far_ids, &s->n_far, &s->inv, kNoAllocBuckets, n, kNoAllocMaxBodies};
 }
 struct NaWorld {   // one world
     __device__ __forceinline__ int operator()(int) const { return 0; }
@@ -107,18 +107,18 @@ struct NaWorld {   // one world
 __global__ void __launch_bounds__(1024) k_na_begin(const float* aabbs, int n, NoAllocScratch* s) {
     if (blockIdx.x == 0 && threadIdx.x < kNoAllocMaxBodies / 1024) s->chunk[threadIdx.x] = 0;
     const int step = grid_sample_step(n);
-    grid_begin(na_grid(s), grid_sample_count(n), NaLoad(aabbs), [=](int k) { return k * step; });
+    grid_begin(na_grid(s, n), grid_sample_count(n), NaLoad(aabbs), [=](int k) { return k * step; });
 }
 __global__ void __launch_bounds__(256) k_na_put(const float* aabbs, int n, NoAllocScratch* s, int pass) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) grid_put(na_grid(s), i, 0, NaLoad(aabbs), pass);
+    if (i < n) grid_put(na_grid(s, n), i, 0, NaLoad(aabbs), pass);
 }
 __global__ void __launch_bounds__(1024) k_na_buckets(NoAllocScratch* s) { block_prefix_1024(s->bucket, kNoAllocBuckets); }
 __global__ void __launch_bounds__(256) k_na_grid_count(const float* aabbs, int n, NoAllocScratch* s) {
     const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (i >= n) return;
     const NaLoad load(aabbs);
-    int c = grid_near(na_grid(s), i, 0, load, NaWorld{}, [](int) {});
+    int c = grid_near(na_grid(s, n), i, 0, load, NaWorld{}, [](int) {});
     if (c == -2) return;   // k_na_far's
     if (c < 0) {
         int one[1];
@@ -131,9 +131,16 @@ __global__ void __launch_bounds__(256) k_na_grid_count(const float* aabbs, int n
     }
 }
 __global__ void __launch_bounds__(1024) k_na_far(const float* aabbs, int n, NoAllocScratch* s, uint32_t* pairs, int cap, int write) {
-    const int m = s->n_far;
+    // one thread reads for the block: its threads go through the same barriers
+    // whatever another call writes meanwhile
+    __shared__ int sh_m, sh_i;
+    if (threadIdx.x == 0) sh_m = min(s->n_far, kNoAllocMaxBodies);
+    __syncthreads();
+    const int m = sh_m;
     for (int k = blockIdx.x; k < m; k += gridDim.x) {
-        const int i = s->far_ids[k], o = write ? s->count[i] : 0;
+        if (threadIdx.x == 0) sh_i = min((int)s->far_ids[k], n - 1);
+        __syncthreads();
+        const int i = sh_i, o = write ? s->count[i] : 0;
         const int c = grid_far(i, n, NaLoad(aabbs), write != 0, [&](int r, int j) { na_put(pairs, cap, o + r, i, j); });
         if (!write && threadIdx.x == 0) {
             s->count[i] = c;
@@ -173,9 +180,10 @@ __global__ void __launch_bounds__(256) k_na_grid_write(const float* aabbs, int n
     __shared__ int near[8][kGridNear], n_near[8];
     const int wid = threadIdx.x >> 5, i = blockIdx.x * 8 + wid;
     if (i >= n) return;
-    const int o = s->count[i], m = (i + 1 < n ? s->count[i + 1] : s->total) - o;
+    const int o = __shfl_sync(0xffffffffu, s->count[i], 0);
+    const int m = __shfl_sync(0xffffffffu, i + 1 < n ? s->count[i + 1] : s->total, 0) - o;
     if (m == 0 || o >= cap) return;
-    grid_write(na_grid(s), i, n, m, NaLoad(aabbs), NaWorld{}, NaEnd{n}, near[wid], &n_near[wid],
+    grid_write(na_grid(s, n), i, n, m, NaLoad(aabbs), NaWorld{}, NaEnd{n}, near[wid], &n_near[wid],
                [&](int k, int j) { na_put(pairs, cap, o + k, i, j); });
 }
 

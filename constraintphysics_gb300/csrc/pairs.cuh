@@ -99,6 +99,9 @@ __device__ __forceinline__ int block_prefix_1024(int* v, int n) {
 // Cell numbers come from the
 // same rounded products everywhere, which are monotonic in the coordinate, so
 // no neighbour is missed; the result does not depend on the cells at all.
+// Nothing read from the grid's own arrays is used as an index unchecked: the
+// allocation-free call's are shared by all calls on a device, and calls that
+// overlap (which gives wrong pairs) still stay inside their buffers.
 template <class Id>
 struct PairGrid {
     int* bucket;       // [buckets]: sizes, their exclusive prefix, then (filled) each bucket's end
@@ -107,6 +110,7 @@ struct PairGrid {
     int* n_far;
     float* inv;        // 1 / cell side (0: no usable box)
     int buckets;       // a power of two
+    int n, cap;        // boxes; entries of ids and far_ids
     __device__ __forceinline__ int of(int x, int y, int z, int w) const {
         return (int)(((uint32_t)x * 73856093u ^ (uint32_t)y * 19349663u ^ (uint32_t)z * 83492791u ^ (uint32_t)w * 2654435761u) &
                      (uint32_t)(buckets - 1));
@@ -183,9 +187,10 @@ __device__ __forceinline__ void grid_put(const PairGrid<Id>& g, int i, int w, co
     if (box_cell(load(i), *g.inv, &c)) {
         const int b = g.of(c.x, c.y, c.z, w);
         const int at = atomicAdd(&g.bucket[b], 1);
-        if (pass == 1) g.ids[at] = (Id)i;
+        if (pass == 1 && (unsigned)at < (unsigned)g.cap) g.ids[at] = (Id)i;
     } else if (pass == 0) {
-        g.far_ids[atomicAdd(g.n_far, 1)] = (Id)i;
+        const int at = atomicAdd(g.n_far, 1);
+        if ((unsigned)at < (unsigned)g.cap) g.far_ids[at] = (Id)i;
     }
 }
 // Box i's overlaps j > i in its world w by one warp, in no order: lane k < 27
@@ -199,7 +204,7 @@ template <class Id, class Load, class World, class Hit>
 __device__ __forceinline__ int grid_near(const PairGrid<Id>& g, int i, int w, const Load& load, const World& world, const Hit& hit) {
     const int lane = threadIdx.x & 31;
     const PairBox a = load(i);
-    const float inv = *g.inv;
+    const float inv = __shfl_sync(0xffffffffu, *g.inv, 0);   // one value for the warp's branches
     PairCell c;
     if (!box_cell(a, inv, &c)) return -2;
     int b0 = 0, b1 = 0, x = 0, y = 0, z = 0;
@@ -208,23 +213,23 @@ __device__ __forceinline__ int grid_near(const PairGrid<Id>& g, int i, int w, co
         y = c.y + lane / 3 % 3 - 1;
         z = c.z + lane / 9 - 1;
         const int b = g.of(x, y, z, w);
-        b0 = b > 0 ? g.bucket[b - 1] : 0;
-        b1 = g.bucket[b];
+        b0 = b > 0 ? max(g.bucket[b - 1], 0) : 0;
+        b1 = min(g.bucket[b], g.cap);
     }
-    const int n_far = *g.n_far;
+    const int n_far = min(*g.n_far, g.cap);
     if (__any_sync(0xffffffffu, b1 - b0 > kGridMost) || n_far > kGridFar) return -1;
     int cnt = 0;
 #pragma unroll 4
     for (int k = b0; k < b1; k++) {
         const int j = g.ids[k];
-        if (j <= i || world(j) != w) continue;
+        if (j <= i || j >= g.n || world(j) != w) continue;
         const PairBox b = load(j);
         PairCell cj;
         if (box_meet(a, b) && box_cell(b, inv, &cj) && cj.x == x && cj.y == y && cj.z == z) { hit(j); cnt++; }
     }
     for (int k = lane; k < n_far; k += 32) {
         const int j = g.far_ids[k];
-        if (j > i && world(j) == w && box_meet(a, load(j))) { hit(j); cnt++; }
+        if (j > i && j < g.n && world(j) == w && box_meet(a, load(j))) { hit(j); cnt++; }
     }
     return __reduce_add_sync(0xffffffffu, cnt);
 }
@@ -237,10 +242,14 @@ __device__ __forceinline__ void grid_write(const PairGrid<Id>& g, int i, int n, 
                                            const End& end, int* near, int* n_near, const Put& put) {
     const int lane = threadIdx.x & 31;
     PairCell cell;
-    if (!box_cell(load(i), *g.inv, &cell)) return;
+    if (!box_cell(load(i), __shfl_sync(0xffffffffu, *g.inv, 0), &cell)) return;
     if (lane == 0) *n_near = 0;
     __syncwarp();
-    const int c = m <= kGridNear ? grid_near(g, i, world(i), load, world, [&](int j) { near[atomicAdd(n_near, 1)] = j; }) : -1;
+    const auto keep = [&](int j) {
+        const int at = atomicAdd(n_near, 1);
+        if (at < kGridNear) near[at] = j;
+    };
+    const int c = m <= kGridNear ? min(grid_near(g, i, world(i), load, world, keep), kGridNear) : -1;
     __syncwarp();
     if (c >= 0) {
         for (int k = lane; k < c; k += 32) {   // each overlap at its rank
