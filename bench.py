@@ -177,9 +177,9 @@ def measured_peaks():
 
 def measured_traffic(stage, worlds):
     """DRAM bytes per launch of the stage's dominant kernel, from the committed
-    summary of an ncu capture of the current build (profiles/pgs_traffic.txt:
-    lines `stage bytes worlds`, the bytes scaled to the workload's world count
-    from a smaller capture, as the file states), or None."""
+    summary of an ncu capture (profiles/pgs_traffic.txt states which kernels and
+    when: lines `stage bytes worlds`, the bytes scaled to the workload's world
+    count from a smaller capture), or None."""
     path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "profiles", "pgs_traffic.txt")
     try:
         with open(path) as f:
@@ -263,6 +263,27 @@ def run_serving(cg, rates, duration, seed, budget_bytes=150 << 30, epoch_steps=1
                     "device_gb": st["device_bytes"] / 1e9, "running_bodies_at_end": st["running_bodies"],
                     "budget_gb": budget_bytes / 1e9})
     return out
+
+
+def reference_missing():
+    """Why the reference engine cannot be run here (neither its library nor its
+    sources are there), or None."""
+    import oracle
+    from oracle import stage_ref
+    if oracle.ref_available() or os.path.isdir(os.path.join(stage_ref.DEST, "src")) or stage_ref.reference_root():
+        return None
+    return "the reference's library is not built and its sources are not there to build it"
+
+
+def cpu_baseline(cg, ws_scenes, warmup, steps, budget_s, threads):
+    """The reference engine's rate and the drift against it; where it is not
+    there, the line says so.  Any other failure is raised."""
+    why = reference_missing()
+    if why:
+        return {"value": None, "unit": UNIT, "kind": "reference", "unavailable": why}
+    bsps, sample, _ = run_reference_sample(ws_scenes, warmup, steps, budget_s, threads)
+    return {"value": bsps, "unit": UNIT, "cores": threads, "kind": "reference", "sample": sample,
+            "drift_300": measure_drift(cg, ws_scenes)}
 
 
 def run_reference_sample(ws_scenes, warmup, steps, budget_s, threads):
@@ -612,12 +633,7 @@ def main():
 
     cpu = None
     if not a.no_cpu and rank == 0:
-        try:
-            bsps, sample, wall = run_reference_sample(ws_scenes, a.warmup, a.steps, a.cpu_budget_s, threads)
-            cpu = {"value": bsps, "unit": UNIT, "cores": threads, "kind": "reference", "sample": sample,
-                   "drift_300": measure_drift(cg, ws_scenes)}
-        except FileNotFoundError as e:   # the reference's sources were not there to build
-            cpu = {"value": None, "unit": UNIT, "kind": "reference", "unavailable": str(e)}
+        cpu = cpu_baseline(cg, ws_scenes, a.warmup, a.steps, a.cpu_budget_s, threads)
 
     if rank == 0:
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world_size, "steps": a.steps,
