@@ -1773,10 +1773,8 @@ __device__ __forceinline__ int next_pair(int* counter, int lane) {
     return __shfl_sync(0xffffffffu, p, 0);
 }
 
-// One warp per candidate pair that involves a sphere or a cylinder (the other
-// pairs are k_narrowphase's).  Same staging as k_narrowphase.
-// Pairs with a round shape listed by kind, the costliest kinds first: the
-// kernel holds nine detectors, far more code than the instruction cache, and
+// Pairs with a round shape listed by kind, the costliest kinds first:
+// k_narrow_prim holds nine detectors, far more code than the instruction cache, and
 // warps of one SM that run different ones wait for instructions most of the
 // time (4.2 of 10 cycles an instruction); a list by kind has them on the same
 // detector together, and the longest pairs start first.  Pass 0 counts the
@@ -1815,6 +1813,9 @@ __global__ void __launch_bounds__(256) k_prim_list(Dev d, int pass) {
     }
 }
 
+// One warp per listed pair (with a sphere, cylinder or capsule, no mesh and no
+// union; the other pairs are k_narrowphase's and k_narrow_mesh's).  Same staging
+// as k_narrowphase.
 __global__ void __launch_bounds__(256, 1) k_narrow_prim(Dev d, int slot_bytes) {
     extern __shared__ __align__(16) uint8_t smem[];
     const int lane = threadIdx.x & 31;
@@ -1838,7 +1839,6 @@ __global__ void __launch_bounds__(256, 1) k_narrow_prim(Dev d, int slot_bytes) {
         const HullHeader* Ha = reinterpret_cast<const HullHeader*>(ga);
         const HullHeader* Hb = reinterpret_cast<const HullHeader*>(gb);
         const uint32_t ka = Ha->kind, kb = Hb->kind;
-        if ((ka | kb) == SHAPE_HULL || ka == SHAPE_MESH || kb == SHAPE_MESH || is_union(d, a) || is_union(d, b)) continue;
         if (failed || !(d.movement[a] == 0 || d.movement[b] == 0) || both_asleep(d, a, b) || jointed(d, a, b)) {
             if (lane == 0) no_manifold(d, p);
             continue;
@@ -2145,9 +2145,9 @@ int mesh_scratch_warps(int n_sms) { return n_sms * kMeshBlocksPerSm * 8; }
 
 // ---- ray queries ------------------------------------------------------------------
 // PhysicsEngine::raycastFirstIntersection (PhysicsEngine.cpp:582-609) for one
-// ray per block (many rays: per thread) against the bodies [s, e) of one world: every body whose
-// current AABB the ray crosses is tested with its primitive's ray test, the
-// nearest hit wins (strictly nearer replaces, in body order).
+// ray per block (many rays: per thread) against the bodies [s, e) of one world:
+// every body whose current AABB the ray crosses is tested with its primitive's
+// ray test, the nearest hit wins (strictly nearer replaces, in body order).
 namespace {
 struct RayHitD { bool hit; f3 p, n; float t; };
 
