@@ -2758,8 +2758,8 @@ int cpgpu_world_read_audit(cpgpu_world* w, double* out) {
     });
 }
 
-// PhysicsEngine::raycastFirstIntersection (PhysicsEngine.cpp:582-609), one
-// device thread per ray against the world's current geometry
+// PhysicsEngine::raycastFirstIntersection (PhysicsEngine.cpp:582-609) against the
+// world's current geometry, a block per ray (from kRayMany rays on a thread)
 int cpgpu_raycast(cpgpu_world* w, const double* origins, const double* dirs, int n_rays, const uint32_t* ignore,
                   int n_ignore, uint32_t* hit_body, double* hit_pos, double* hit_normal, double* hit_dist) {
     W_OR_FAIL(w);

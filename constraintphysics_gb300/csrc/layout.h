@@ -410,7 +410,7 @@ struct Dev {
     int* row_contact;              // row slot -> contact
     int* row_of_contact;           // contact -> row slot
     RowBlock* rows;
-    float4* dv;                    // 4 float4 per island body slot: dv lin, dv ang, dpv lin, dpv ang
+    float4* dv;                    // kDvF4 float4 per island body slot
     float4* stage;                 // 4 float4 per body: staging of external state writes
     int* big_list; int* small_list;  // island indices split by row count (PGS scheduling)
     int* sched;                    // schedule counters and tables (kSchedInts ints, layout in solver.cu)
@@ -429,7 +429,7 @@ struct Dev {
     int* joint_list;               // joint islands (PGS scheduling), count in sched[3]
     const int* hs_world_start;     // [n_worlds + 1] holonomic system ranges (island lists)
     float lin_err_threshold;       // excessive_linear_error_torque_threshold
-    float4* dv_err;                // 4 float4 per island body: linearisation-error probe
+    float4* dv_err;                // kDvF4 float4 per island body: linearisation-error probe
     SpringStore sp;                // springs (sp.n == 0: none in the batch)
     // polls of a bounded mbarrier wait before a kernel gives up and reports
     // ST_TIMEOUT (kDefaultWaitLimit; CPGPU_WAIT_LIMIT lowers it so that a test

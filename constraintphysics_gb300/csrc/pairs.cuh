@@ -96,9 +96,11 @@ __device__ __forceinline__ int block_prefix_1024(int* v, int n) {
 // A box that reaches at most one cell beyond the cell of its lower corner meets
 // only boxes of the 27 cells around it; the others (larger, NaN, inverted or
 // out of the cell numbers' range) are listed apart and tested against all.
-// Cell numbers come from the
-// same rounded products everywhere, which are monotonic in the coordinate, so
-// no neighbour is missed; the result does not depend on the cells at all.
+// Cell numbers come from the same rounded products everywhere, which are
+// monotonic in the coordinate, so no neighbour is missed; the result does not
+// depend on the cells at all.  The bucket hash takes the primes of Teschner et
+// al. ("Optimized Spatial Hashing for Collision Detection of Deformable
+// Objects", 2003) and, for the world, Knuth's multiplier.
 // Nothing read from the grid's own arrays is used as an index unchecked: the
 // allocation-free call's are shared by all calls on a device, and calls that
 // overlap (which gives wrong pairs) still stay inside their buffers.

@@ -7,11 +7,13 @@
 // values, chunk sums, their prefix, its addition and the total's check took
 // five launches of 2-3 us each.
 //
-// Chunks are taken in order from a counter.  A chunk's block publishes its sum,
-// then finds the sum of the chunks before it by looking back at theirs, 32 at
-// a time (sums, or a prefix where one is known).  A block only ever waits for
-// chunks that other blocks have already taken, so it makes progress whatever
-// else runs; the wait is bounded like every other (ST_TIMEOUT).
+// The decoupled look-back prefix of Merrill and Garland ("Single-pass Parallel
+// Prefix Scan with Decoupled Look-back", 2016).  Chunks are taken in order from
+// a counter.  A chunk's block publishes its sum, then finds the sum of the
+// chunks before it by looking back at theirs, 32 at a time (sums, or a prefix
+// where one is known).  A block only ever waits for chunks that other blocks
+// have already taken, so it makes progress whatever else runs; the wait is
+// bounded like every other (ST_TIMEOUT).
 #pragma once
 #include <algorithm>
 

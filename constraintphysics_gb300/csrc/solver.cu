@@ -8,14 +8,15 @@
 // the contact's slot in island order.  The same pass advances the contact's
 // lifetime (PhysicsEngine.cpp:1378-1399) and marks expired contacts.
 //
-// PGS (PGS_solve, ConstraintSolver.cpp:80-213): one thread per island walks
-// its rows in the reference's order: targets from the bodies' velocities,
-// warm start, n_vel velocity sweeps of block Gauss-Seidel with the projection
-// on the accumulated impulse, n_pos pseudo-velocity sweeps of the normal rows,
-// then the velocity deltas are applied to the island's bodies.  A serial chain
-// per island is the latency-optimal form of Gauss-Seidel (each row depends on
-// the previous one); throughput comes from running thousands of islands at
-// once.
+// PGS (PGS_solve, ConstraintSolver.cpp:80-213): each island's rows one after the
+// other in the reference's order: targets from the bodies' velocities, warm
+// start, n_vel velocity sweeps of block Gauss-Seidel with the projection on the
+// accumulated impulse, n_pos pseudo-velocity sweeps of the normal rows, then the
+// velocity deltas are applied to the island's bodies.  A large or middling island
+// takes two lanes of a warp (a body of the contact each), one with joints a
+// warp, a small one a thread.  A serial chain per island is the latency-optimal
+// form of Gauss-Seidel (each row depends on the previous one); throughput comes
+// from running thousands of islands at once.
 //
 // Integration (PhysicsEngine.cpp:390-419, RigidBody.cpp:207-279): one thread
 // per body.
