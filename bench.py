@@ -499,6 +499,10 @@ def main():
     if a.impl == "reference":
         if rank != 0:
             return
+        why = reference_missing()
+        if why:
+            print(json.dumps({"impl": "reference", "unavailable": why}), flush=True)
+            return
         bsps, sample, wall = run_reference_sample(ws_scenes, a.warmup, a.steps, a.cpu_budget_s, threads)
         line = {"impl": "reference", "metric": METRIC, "value": bsps, "unit": UNIT, "n_gpus": a.gpus, "steps": a.steps,
                 "warmup": a.warmup, "ms_per_step": None, "higher_is_better": True, "scaling": "weak",

@@ -1,5 +1,6 @@
 """bench.py's CPU leg: only a reference that is not there is reported as
 unavailable; a baseline that is there and fails to build or run is an error."""
+import json
 import os
 
 import pytest
@@ -37,3 +38,10 @@ def test_a_failing_baseline_is_not_an_absent_one(nothing, monkeypatch, have):
         monkeypatch.setattr(stage_ref, "reference_root", lambda: str(nothing))
     with pytest.raises(FileNotFoundError, match="g\\+\\+"):
         bench.cpu_baseline(None, [], 1, 1, 1.0, 1)
+
+
+def test_the_reference_arm_prints_its_line_without_the_reference(nothing, monkeypatch, capsys):
+    monkeypatch.setattr("sys.argv", ["bench.py", "--impl", "reference", "--worlds", "2", "--steps", "1", "--warmup", "1"])
+    bench.main()
+    line = json.loads(capsys.readouterr().out.strip().splitlines()[-1])
+    assert line["impl"] == "reference" and "sources" in line["unavailable"]
