@@ -599,7 +599,9 @@ struct Batch {
     std::vector<uint8_t> movement;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // ray queries' device buffer (rays, results, ignored ids), kept between calls
-    // and grown as needed; freed with the batch
+    // and grown as needed; freed with the batch.  ray_use: queries of several
+    // threads take it one after the other
+    std::mutex ray_use;
     uint8_t* ray_mem = nullptr;
     size_t ray_bytes = 0;
     uint8_t* ray_buffer(size_t n) {
@@ -2781,6 +2783,7 @@ int cpgpu_raycast(cpgpu_world* w, const double* origins, const double* dirs, int
                 rays[6 * k + 3 + c] = (float)dirs[i];
             }
             if (n_ignore > 0) std::memcpy(&rays[nr], ignore, sizeof(uint32_t) * (size_t)n_ignore);
+            std::lock_guard<std::mutex> lock(B.ray_use);   // until the results are here
             uint8_t* mem = B.ray_buffer(out_at + sizeof(float) * out.size());
             CK(cudaMemcpyAsync(mem, rays.data(), in_bytes, cudaMemcpyHostToDevice, B.st));
             launch_raycast(B.cur(), 0, (int)w->w.bodies.size(), reinterpret_cast<float*>(mem), n_rays,
