@@ -1273,8 +1273,8 @@ __device__ __forceinline__ void joint_passes(JointRow* joints, RowBlock* rows, i
 // of an island of up to kJointList rows) and the Δv of islands of up to kJointDv
 // bodies (`dv_cap` lowers it) are held in shared memory.  On 512 chains of 16-64
 // links: one lane and everything in global memory 568 us a substep, the rows
-// in global memory 263, in shared memory 219 (the first, with the solve, 1,880
-// -> 594).  Past the lines (and past those of the block solve: kHoloN, kHoloL and
+// in global memory 263, in shared memory 219, with each pass's own fields alone
+// 131 (the first, with the solve, 1,880 -> 594 -> 438).  Past the lines (and past those of the block solve: kHoloN, kHoloL and
 // the factor's kFactorBytes), a step of 256 hung chains of 64 / 65 / 69 / 100
 // links, FP64 systems: 1.98 / 3.17 / 4.31 / 6.61 ms (6.78 / 6.84 / 7.64 / 12.8 by
 // one lane with everything in global memory).
